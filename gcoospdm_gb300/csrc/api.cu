@@ -122,10 +122,45 @@ gcoo_status ensure_split_work(gcoo_handle *h, int64_t n)
     return GCOO_SUCCESS;
 }
 
+// Walk of a matrix whose groups share columns, by the width of B. Measured
+// at 4096^2 (us; row walk / group walk / panels):
+//   16 x 16 blocks, 25 %: n 64 199 / 366 / 139, n 128 215 / 380 / 147, n 256 331 / 397 / 106, n 1024 1030 / 561 / 230
+//   16 x 16 blocks,  5 %: n 64  36 /  91 /  59, n 128  42 /  93 /  57, n 256  60 /  97 /  46, n 1024  158 / 137 /  74
+//   4 x 4 blocks, 10 %:   n 128 59 / 154, n 256 103 / 162, n 300 - / 127, n 1024 333 / 235
+//   unstructured 30 %:    n 128 244 / 1178 / 345, n 256 375 / 1200 / 344, n 1024 1169 / 1548 / 937
+// Narrow B: one staging of a panel's or a group's entries serves few columns
+// and the row walk is faster, long rows in panels aside; the group walk is
+// slow there with 8 columns per lane (n % 8 == 0) only.
+enum SharedWalk { kWalkRows, kWalkGroups, kWalkPanels };
+
+static SharedWalk shared_walk(const gcoo_handle *h, int64_t n, uintptr_t b, uintptr_t c)
+{
+    const bool vec4 = n % 4 == 0 && !((b | c) & 15);
+    if (h->panels && h->p.vec == 0 && panel_ok(n)) {
+        const bool long_rows = h->nnz >= 1000 * h->m;
+        if (h->p.fp32_order == 2 || (vec4 ? n > 128 || long_rows : n >= 192))
+            return kWalkPanels;
+        return vec4 ? kWalkRows : kWalkGroups;
+    }
+    if (h->p.fp32_order != 2 && vec4 && n % 8 == 0 && n <= 256 && h->p.vec == 0)
+        return kWalkRows;
+    return kWalkGroups;
+}
+
 gcoo_status spdm_fp32(gcoo_handle *h, const float *dB, int64_t n, float *dC, cudaStream_t st,
                       const gcoo_params *override_params)
 {
-    if (!override_params && group_order_chosen(h)) {
+    const SharedWalk walk = !override_params && group_order_chosen(h)
+                                ? shared_walk(h, n, reinterpret_cast<uintptr_t>(dB), reinterpret_cast<uintptr_t>(dC))
+                                : kWalkRows;
+    if (walk == kWalkPanels) {
+        const cudaError_t e = launch_spdm_fp32_panel(h->packed.ptr, h->row_ptr.ptr, h->tile_cnt.ptr, h->m, h->k, dB, n,
+                                                     dC, st);
+        if (e != cudaSuccess)
+            return cuda_fail(e, "spdm_panel_kernel launch");
+        return GCOO_SUCCESS;
+    }
+    if (walk == kWalkGroups) {
         // 8 columns per lane (two 16-byte loads: more FMAs per shuffled entry) where n allows
         int v = n % 8 == 0 ? 8 : 4;
         const uintptr_t b = reinterpret_cast<uintptr_t>(dB), c = reinterpret_cast<uintptr_t>(dC);
@@ -282,6 +317,35 @@ gcoo_status gcoo_create(gcoo_handle **out, const float *dA, int64_t m, int64_t k
 
 namespace {
 
+// Whether the FP32 multiply of a matrix whose groups share columns takes 16
+// rows per B load. Groups of four rows that share only part of their columns
+// (fewer than 3 of the 4 rows on average) share with their neighbours much
+// as among themselves: yes. Groups that share nearly all of them are blocks
+// of 4 rows or higher: only where the blocks reach across the 16 rows, which
+// a sample of panels tells (one more readback, for such matrices only). A
+// panel's staging costs about the same whatever its window holds: at 2 %
+// density (16 x 16 blocks, 4096^2) panels take 36 against the group walk's 53 us
+// at n = 256 and 54 against 60 at n = 1024, so below 1/64 the group walk stays.
+gcoo_status choose_panels(gcoo_handle *h, cudaStream_t st)
+{
+    h->panels = false;
+    if (!h->seg_prefix || !group_order_chosen(h) || 64.0 * static_cast<double>(h->nnz) < static_cast<double>(h->m) * h->k)
+        return GCOO_SUCCESS;
+    if (h->nnz < 3 * h->distinct_cols) {
+        h->panels = true;
+        return GCOO_SUCCESS;
+    }
+    if (!h->long_count.ensure(2))
+        return fail(GCOO_ERROR_ALLOC, "device allocation of the sharing counts failed");
+    unsigned long long share[2] = {0, 0};
+    GCOO_CUDA(cudaMemsetAsync(h->long_count.ptr, 0, sizeof(share), st));
+    GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m, h->long_count.ptr, st));
+    GCOO_CUDA(cudaMemcpyAsync(share, h->long_count.ptr, sizeof(share), cudaMemcpyDeviceToHost, st));
+    GCOO_CUDA(cudaStreamSynchronize(st));
+    h->panels = share[0] >= 12 * share[1];
+    return GCOO_SUCCESS;
+}
+
 // The end of every successful build: plans derived from the old arrays go,
 // and for a skewed matrix the list of its long rows (multiplied by their own
 // kernel) is collected, one readback of its length.
@@ -292,6 +356,9 @@ gcoo_status finish_build(gcoo_handle *h, cudaStream_t st)
     h->tc = nullptr;
     destroy_left_plan(h->left);
     h->left = nullptr;
+    const gcoo_status ps = choose_panels(h, st);
+    if (ps != GCOO_SUCCESS)
+        return ps;
     h->n_long = 0;
     h->long_entries = 0;
     h->pieces_bound = 0;
@@ -353,6 +420,7 @@ gcoo_status gcoo_build(gcoo_handle *h, void *stream)
         return fail(GCOO_ERROR_INVALID_VALUE, "handle is NULL");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     h->built = false;
+    h->seg_prefix = false;
     if (h->coo) {
         gcoo_status s = coo_build(h, st);
         if (s != GCOO_SUCCESS)
@@ -406,6 +474,7 @@ gcoo_status gcoo_build(gcoo_handle *h, void *stream)
             h->max_row_nnz = t3[1];
             h->distinct_cols = t3[2];
             h->nnz = total;
+            h->seg_prefix = true;
             return finish_build(h, st);
         }
         GCOO_CUDA(cudaMemsetAsync(d_total + 1, 0, 7 * sizeof(int64_t), st));
@@ -444,6 +513,7 @@ gcoo_status gcoo_build(gcoo_handle *h, void *stream)
         GCOO_CUDA(launch_scatter(h->dA, h->m, h->k, cpg, h->group_index(), h->row_ptr.ptr, h->vals.ptr, rows,
                                  cols, h->packed.ptr, st));
     h->nnz = total;
+    h->seg_prefix = tiled;
     return finish_build(h, st);
 }
 

@@ -39,7 +39,9 @@ struct gcoo_handle {
     gcoo::DevBuf<float> vals;        // reference GCOO order
     gcoo::DevBuf<int32_t> rc;        // rows[nnz] | cols[nnz]
     gcoo::DevBuf<gcoo::Entry> packed; // row order, nnz + 2 (16-byte padded)
-    gcoo::DevBuf<int32_t> tile_cnt;  // per-(row, column segment) counts of the tiled conversion
+    gcoo::DevBuf<int32_t> tile_cnt;  // per-(row, column segment) counts of the tiled conversion, then their prefix
+    bool panels = false;             // the FP32 multiply takes 16 rows per B load (api.cu: choose_panels)
+    bool seg_prefix = false;         // tile_cnt holds the built arrays' prefixes (built by the tiled conversion)
     gcoo::DevBuf<uint2> stage;       // staged rebuild: each tile's entries in a fixed slot
     gcoo::DevBuf<int32_t> tile_tot;  // staged rebuild: entries per tile, -1 when it overflowed
     gcoo::DevBuf<int32_t> over_list; // staged rebuild: the overflowed tiles

@@ -209,6 +209,16 @@ bool group_order_ok(int32_t rows_per_group);
 cudaError_t launch_spdm_fp32_group(const float *vals, const int32_t *rows, const int32_t *cols,
                                    const int32_t *group_index, int64_t m, int64_t ng, const float *B,
                                    int64_t n, float *C, int vec, cudaStream_t st);
+// Sixteen rows per CTA sharing every B load (spdm_fp32_panel.cu), from the
+// row-ordered entries and the tiled conversion's segment prefixes
+// (pref[r * conv_segments(k) + s]).
+bool panel_ok(int64_t n);
+// Sampled sharing inside 16-row panels: out[0] += entries, out[1] += distinct
+// (panel, column) pairs (zeroed by the caller).
+cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, unsigned long long *out,
+                               cudaStream_t st);
+cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, const int32_t *pref, int64_t m,
+                                   int64_t k, const float *B, int64_t n, float *C, cudaStream_t st);
 // The same walk for the BF16 / FP8-B forms on the FMA engine, from B already
 // converted to bf16 or E4M3 (+ per-column scales); n % 8 == 0.
 cudaError_t launch_spdm_lowp_group(const float *vals, const int32_t *rows, const int32_t *cols,
