@@ -23,39 +23,74 @@ namespace {
 
 constexpr int kChunk = 2048; // most entries staged per pass (16 KB)
 
-template <int V>
-struct Vec;
+// V output columns of a lane, in V / W loads of W consecutive columns at
+// strides of 32 W: W = V where B's and C's rows are aligned for it, else the
+// widest that they are. Each load is contiguous across the warp whatever W is.
+template <int W>
+struct Piece;
 template <>
-struct Vec<4> {
-    static __device__ __forceinline__ void load(const float *p, float (&o)[4])
+struct Piece<4> {
+    static __device__ __forceinline__ void load(const float *p, float *o)
     {
         const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
         o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
     }
-    static __device__ __forceinline__ void store(float *p, const float (&o)[4])
+    static __device__ __forceinline__ void store(float *p, const float *o)
     {
         *reinterpret_cast<float4 *>(p) = make_float4(o[0], o[1], o[2], o[3]);
     }
 };
 template <>
-struct Vec<2> {
-    static __device__ __forceinline__ void load(const float *p, float (&o)[2])
+struct Piece<2> {
+    static __device__ __forceinline__ void load(const float *p, float *o)
     {
         const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
         o[0] = t.x; o[1] = t.y;
     }
-    static __device__ __forceinline__ void store(float *p, const float (&o)[2])
+    static __device__ __forceinline__ void store(float *p, const float *o)
     {
         *reinterpret_cast<float2 *>(p) = make_float2(o[0], o[1]);
     }
 };
 template <>
-struct Vec<1> {
-    static __device__ __forceinline__ void load(const float *p, float (&o)[1]) { o[0] = __ldg(p); }
-    static __device__ __forceinline__ void store(float *p, const float (&o)[1]) { *p = o[0]; }
+struct Piece<1> {
+    static __device__ __forceinline__ void load(const float *p, float *o) { o[0] = __ldg(p); }
+    static __device__ __forceinline__ void store(float *p, const float *o) { *p = o[0]; }
 };
 
-template <int V, int U, bool PIPE>
+template <int V, int W>
+struct Vec {
+    static __device__ __forceinline__ void load(const float *p, float (&o)[V])
+    {
+#pragma unroll
+        for (int h = 0; h < V / W; ++h)
+            Piece<W>::load(p + h * 32 * W, o + h * W);
+    }
+    // the pieces whose first column, j + h * 32 W, is at least `from`
+    static __device__ __forceinline__ void store(float *p, const float (&o)[V], int64_t j, int64_t from)
+    {
+#pragma unroll
+        for (int h = 0; h < V / W; ++h)
+            if (W == V || j + h * 32 * W >= from)
+                Piece<W>::store(p + h * 32 * W, o + h * W);
+    }
+};
+
+// A lane's columns in a 32 V-column tile. W == V: jt is the lane's first
+// column. W < V: jt is the tile's, and the last tile of a ragged row starts
+// early enough to be whole (n >= 32 V) and stores only its own columns.
+template <int V, int W>
+struct LaneCols {
+    int64_t j, from;
+    bool on;
+    __device__ __forceinline__ LaneCols(int64_t jt, int lane, int64_t n) : j(jt), from(jt), on(jt < n)
+    {
+        if constexpr (W < V)
+            j = (jt + 32 * V <= n ? jt : n - 32 * V) + lane * W;
+    }
+};
+
+template <int V, int W, int U, bool PIPE>
 __device__ __forceinline__ void row_chain(const Entry *__restrict__ s, int cnt, const float *__restrict__ Bj,
                                           int64_t n, float (&acc)[V])
 {
@@ -68,7 +103,7 @@ __device__ __forceinline__ void row_chain(const Entry *__restrict__ s, int cnt, 
         for (int u = 0; u < U; ++u) {
             const Entry e = s[u];
             a[u] = e.val;
-            Vec<V>::load(Bj + static_cast<int64_t>(e.col) * n, b[u]);
+            Vec<V, W>::load(Bj + static_cast<int64_t>(e.col) * n, b[u]);
         }
 #pragma unroll 1
         for (i = U; i + U <= cnt; i += U) {
@@ -76,7 +111,7 @@ __device__ __forceinline__ void row_chain(const Entry *__restrict__ s, int cnt, 
             for (int u = 0; u < U; ++u) {
                 const Entry e = s[i + u];
                 a2[u] = e.val;
-                Vec<V>::load(Bj + static_cast<int64_t>(e.col) * n, b2[u]);
+                Vec<V, W>::load(Bj + static_cast<int64_t>(e.col) * n, b2[u]);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -106,7 +141,7 @@ __device__ __forceinline__ void row_chain(const Entry *__restrict__ s, int cnt, 
             e[u] = s[i + u];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            Vec<V>::load(Bj + static_cast<int64_t>(e[u].col) * n, b[u]);
+            Vec<V, W>::load(Bj + static_cast<int64_t>(e[u].col) * n, b[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -117,7 +152,7 @@ __device__ __forceinline__ void row_chain(const Entry *__restrict__ s, int cnt, 
     for (; i < cnt; ++i) {
         const Entry e = s[i];
         float b[V];
-        Vec<V>::load(Bj + static_cast<int64_t>(e.col) * n, b);
+        Vec<V, W>::load(Bj + static_cast<int64_t>(e.col) * n, b);
 #pragma unroll
         for (int v = 0; v < V; ++v)
             acc[v] = fmaf(e.val, b[v], acc[v]);
@@ -126,7 +161,7 @@ __device__ __forceinline__ void row_chain(const Entry *__restrict__ s, int cnt, 
 
 // One row's chain over two column tiles at once (same entries, same fmaf
 // order per element as row_chain): U entries per batch, 2U B loads in flight.
-template <int V, int U>
+template <int V, int W, int U>
 __device__ __forceinline__ void row_chain_pair(const Entry *__restrict__ s, int cnt, const float *__restrict__ Ba,
                                                const float *__restrict__ Bb, int64_t n, float (&acc_a)[V],
                                                float (&acc_b)[V])
@@ -141,8 +176,8 @@ __device__ __forceinline__ void row_chain_pair(const Entry *__restrict__ s, int 
             e[u] = s[i + u];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            Vec<V>::load(Ba + static_cast<int64_t>(e[u].col) * n, ba[u]);
-            Vec<V>::load(Bb + static_cast<int64_t>(e[u].col) * n, bb[u]);
+            Vec<V, W>::load(Ba + static_cast<int64_t>(e[u].col) * n, ba[u]);
+            Vec<V, W>::load(Bb + static_cast<int64_t>(e[u].col) * n, bb[u]);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -156,8 +191,8 @@ __device__ __forceinline__ void row_chain_pair(const Entry *__restrict__ s, int 
     for (; i < cnt; ++i) {
         const Entry e = s[i];
         float ba[V], bb[V];
-        Vec<V>::load(Ba + static_cast<int64_t>(e.col) * n, ba);
-        Vec<V>::load(Bb + static_cast<int64_t>(e.col) * n, bb);
+        Vec<V, W>::load(Ba + static_cast<int64_t>(e.col) * n, ba);
+        Vec<V, W>::load(Bb + static_cast<int64_t>(e.col) * n, bb);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             acc_a[v] = fmaf(e.val, ba[v], acc_a[v]);
@@ -171,7 +206,7 @@ __device__ __forceinline__ void row_chain_pair(const Entry *__restrict__ s, int 
 // col_iters > 1 (only when every group's entries fit one staging chunk): each
 // warp walks col_iters column tiles, col_warps tiles apart, reusing the
 // staged entries, so short rows do not pay one staging per tile.
-template <int V, int MAXT, bool PIPE, bool MULTI>
+template <int V, int W, int MAXT, bool PIPE, bool MULTI>
 __global__ void __launch_bounds__(MAXT)
 spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m,
                  int32_t cpg, const float *__restrict__ B, int64_t n, float *__restrict__ C,
@@ -191,7 +226,7 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
     const bool has_row = slot < cpg && row < r_end;
     const int64_t tile_stride = static_cast<int64_t>(col_warps) * (32 * V);
     const int64_t j = (static_cast<int64_t>(blockIdx.y) * col_iters * col_warps + sub) * (32 * V) +
-                      static_cast<int64_t>(lane) * V;
+                      (W == V ? static_cast<int64_t>(lane) * V : 0);
 
     const int64_t gs = row_ptr[r0];
     const int64_t ge = row_ptr[r_end];
@@ -220,8 +255,8 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
     bool ok = true;
     uint32_t phase = 0;
     for (int it = 0; it < tiles_staged && ok; ++it) {
-        const int64_t jt = j + it * tile_stride;
-        const float *Bj = B + jt;
+        const LaneCols<V, W> at(j + it * tile_stride, lane, n);
+        const float *Bj = B + at.j;
 #pragma unroll
         for (int v = 0; v < V; ++v)
             acc[v] = 0.0f;
@@ -246,12 +281,12 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
             }
             const int64_t lo = rs > cs ? rs : cs;
             const int64_t hi = re < ce ? re : ce;
-            if (!multi_all && jt < n && lo < hi)
-                row_chain<V, (MAXT > 512 ? 4 : 8), PIPE>(s_nz + (lo - a0), static_cast<int>(hi - lo), Bj, n, acc);
+            if (!multi_all && at.on && lo < hi)
+                row_chain<V, W, (MAXT > 512 ? 4 : 8), PIPE>(s_nz + (lo - a0), static_cast<int>(hi - lo), Bj, n, acc);
             __syncthreads(); // buffer free before the next copy
         }
-        if (!multi_all && has_row && jt < n && ok)
-            Vec<V>::store(C + row * n + jt, acc);
+        if (!multi_all && has_row && at.on && ok)
+            Vec<V, W>::store(C + row * n + at.j, acc, at.j, at.from);
     }
     // all column tiles of the warp's row from the (single) staged chunk
     if (multi_all && ok && has_row) {
@@ -262,31 +297,31 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
         // very short rows: two tiles at a time, twice the B loads in flight
         // (longer rows already keep a batch of 8 loads in flight per tile)
         for (; cnt < 16 && it + 1 < col_iters; it += 2) {
-            const int64_t ja = j + it * tile_stride, jb = ja + tile_stride;
-            if (ja >= n)
+            const LaneCols<V, W> aa(j + it * tile_stride, lane, n), ab(j + it * tile_stride + tile_stride, lane, n);
+            if (!aa.on)
                 break;
             float a2[V], b2[V];
 #pragma unroll
             for (int v = 0; v < V; ++v)
                 a2[v] = b2[v] = 0.0f;
-            if (jb < n)
-                row_chain_pair<V, 4>(s_row, cnt, B + ja, B + jb, n, a2, b2);
+            if (ab.on)
+                row_chain_pair<V, W, 4>(s_row, cnt, B + aa.j, B + ab.j, n, a2, b2);
             else if (cnt > 0)
-                row_chain<V, 4, false>(s_row, cnt, B + ja, n, a2);
-            Vec<V>::store(C + row * n + ja, a2);
-            if (jb < n)
-                Vec<V>::store(C + row * n + jb, b2);
+                row_chain<V, W, 4, false>(s_row, cnt, B + aa.j, n, a2);
+            Vec<V, W>::store(C + row * n + aa.j, a2, aa.j, aa.from);
+            if (ab.on)
+                Vec<V, W>::store(C + row * n + ab.j, b2, ab.j, ab.from);
         }
         for (; it < col_iters; ++it) {
-            const int64_t jt = j + it * tile_stride;
-            if (jt >= n)
+            const LaneCols<V, W> at(j + it * tile_stride, lane, n);
+            if (!at.on)
                 break;
 #pragma unroll
             for (int v = 0; v < V; ++v)
                 acc[v] = 0.0f;
             if (cnt > 0)
-                row_chain<V, (MAXT > 512 ? 4 : 8), false>(s_row, cnt, B + jt, n, acc);
-            Vec<V>::store(C + row * n + jt, acc);
+                row_chain<V, W, (MAXT > 512 ? 4 : 8), false>(s_row, cnt, B + at.j, n, acc);
+            Vec<V, W>::store(C + row * n + at.j, acc, at.j, at.from);
         }
     }
 }
@@ -323,7 +358,7 @@ __device__ __forceinline__ void short_window(const Entry &my, int nw, bool all_c
             for (int u = 0; u < 8; ++u) {
                 const int col = __shfl_sync(0xffffffffu, my.col, u0 + u);
                 a[u] = __shfl_sync(0xffffffffu, my.val, u0 + u);
-                Vec<V>::load(Bj + static_cast<int64_t>(col) * n, b[u]);
+                Piece<V>::load(Bj + static_cast<int64_t>(col) * n, b[u]);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u)
@@ -340,7 +375,7 @@ __device__ __forceinline__ void short_window(const Entry &my, int nw, bool all_c
             const int col = __shfl_sync(0xffffffffu, my.col, (u0 + u) & 31);
             a[u] = __shfl_sync(0xffffffffu, my.val, (u0 + u) & 31);
             if (u0 + u < nw && has_col) {
-                Vec<V>::load(Bj + static_cast<int64_t>(col) * n, b[u]);
+                Piece<V>::load(Bj + static_cast<int64_t>(col) * n, b[u]);
             } else {
 #pragma unroll
                 for (int v = 0; v < V; ++v)
@@ -403,7 +438,7 @@ spdm_short_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
         short_window<V>(my, nw, all_cols, has_col, Bj, n, acc);
     }
     if (has_col)
-        Vec<V>::store(C + row * n + j, acc);
+        Piece<V>::store(C + row * n + j, acc);
 }
 
 // Multiply straight from reference-layout arrays (entries of a group in
@@ -459,6 +494,8 @@ bool row_lengths_skewed(int64_t m, int64_t nnz, int64_t max_row)
     return max_row >= 256 && static_cast<double>(max_row) > 8.0 * (mean > 1.0 ? mean : 1.0);
 }
 
+constexpr int64_t kWideCols = 1 << 20;
+
 LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, int64_t max_row,
                        uintptr_t b_addr, uintptr_t c_addr)
 {
@@ -470,16 +507,23 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
     const double mean = m > 0 ? static_cast<double>(nnz) / static_cast<double>(m) : 0.0;
     const bool skewed = row_lengths_skewed(m, nnz, max_row);
     s.rows = skewed ? 1 : p.rows_per_group;
-    int vmax = 4;
+    int w = 4; // the widest aligned load
     if (n % 4 != 0 || (b_addr & 15) || (c_addr & 15))
-        vmax = 2;
-    if (vmax == 2 && (n % 2 != 0 || (b_addr & 7) || (c_addr & 7)))
-        vmax = 1;
+        w = 2;
+    if (w == 2 && (n % 2 != 0 || (b_addr & 7) || (c_addr & 7)))
+        w = 1;
     int v = p.vec > 0 ? p.vec : (n >= 128 ? 4 : (n >= 64 ? 2 : 1));
-    if (v > vmax)
-        v = vmax;
     if (v != 1 && v != 2 && v != 4)
         v = 1;
+    // as many columns per lane from narrower loads: an entry read then serves
+    // as many FMAs as in an aligned B (4001 x 3999 at 2 %: n = 2047 157 us
+    // against 339 at one column per lane, n = 2046 149 against 185 at two,
+    // n = 2048 135). Whole tiles only, two of them in pairs of columns (n =
+    // 130 28 us against 26 at two columns per lane); and not where the number
+    // of narrow tiles decides whether the launch is possible.
+    while (v > w && (n < (w == 2 ? 64 : 32) * v || n > kWideCols))
+        v /= 2;
+    s.width = w < v ? w : v;
     s.vec = v;
     // Every group fits one staging chunk: one staging of a group's entries
     // can serve several column tiles per warp. With the launch shape left to
@@ -555,20 +599,23 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
     // kernel stages any larger group in several passes)
     const int chunk = s.chunk > 0 && s.chunk < kChunk ? s.chunk : kChunk;
     const int smem = 128 + (chunk + 2) * static_cast<int>(sizeof(Entry));
-#define GCOO_FP32_LAUNCH(V, T, P)                                                                       \
+#define GCOO_FP32_LAUNCH(V, W, T, P)                                                                       \
     do {                                                                                                \
         if (s.col_iters > 1)                                                                            \
-            spdm_fp32_kernel<V, T, P, true><<<grid, threads, smem, st>>>(                               \
+            spdm_fp32_kernel<V, W, T, P, true><<<grid, threads, smem, st>>>(                               \
                 packed, row_ptr, m, cpg, B, n, C, s.col_warps, s.col_iters, chunk, status);             \
         else                                                                                            \
-            spdm_fp32_kernel<V, T, P, false><<<grid, threads, smem, st>>>(                              \
+            spdm_fp32_kernel<V, W, T, P, false><<<grid, threads, smem, st>>>(                              \
                 packed, row_ptr, m, cpg, B, n, C, s.col_warps, 1, chunk, status);                       \
     } while (0)
 #define GCOO_FP32_VEC(T, P)                                                                             \
     do {                                                                                                \
-        if (s.vec == 4) GCOO_FP32_LAUNCH(4, T, P);                                                      \
-        else if (s.vec == 2) GCOO_FP32_LAUNCH(2, T, P);                                                 \
-        else GCOO_FP32_LAUNCH(1, T, P);                                                                 \
+        if (s.vec == 4 && s.width == 4) GCOO_FP32_LAUNCH(4, 4, T, P);                                   \
+        else if (s.vec == 4 && s.width == 2) GCOO_FP32_LAUNCH(4, 2, T, P);                              \
+        else if (s.vec == 4) GCOO_FP32_LAUNCH(4, 1, T, P);                                              \
+        else if (s.vec == 2 && s.width == 2) GCOO_FP32_LAUNCH(2, 2, T, P);                              \
+        else if (s.vec == 2) GCOO_FP32_LAUNCH(2, 1, T, P);                                              \
+        else GCOO_FP32_LAUNCH(1, 1, T, P);                                                              \
     } while (0)
     const bool pipe = s.depth >= 2;
     if (threads <= 512) {

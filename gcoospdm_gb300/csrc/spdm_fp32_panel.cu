@@ -426,8 +426,8 @@ cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int6
     return cudaGetLastError();
 }
 
-// Column strips along the grid's y dimension
-bool panel_ok(int64_t n) { return (n + kMaxWarps * kCols - 1) / (kMaxWarps * kCols) <= 65535; }
+// Wider B stays with the group walk, whose tile count decides what is possible
+bool panel_ok(int64_t n) { return n <= 1 << 20; }
 
 cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, const int32_t *pref, int64_t m,
                                    int64_t k, const float *B, int64_t n, float *C, cudaStream_t st)

@@ -1,5 +1,6 @@
-"""GPU: the sixteen-row FP32 walk (rows of a matrix sharing columns), bit for
-bit against the oracle at the edges of its panels, windows, ring and strips."""
+"""GPU: the sixteen-row FP32 walk (rows of a matrix sharing columns) and the row
+walk at ragged widths, bit for bit against the oracle at the edges of their
+panels, windows, rings, strips and tiles."""
 from __future__ import annotations
 
 import numpy as np
@@ -55,3 +56,19 @@ def test_walks_by_width_agree(native, oracle_mod, n):
         h = native.GcooHandle(torch.from_numpy(A).cuda()).build()
         ref = oracle_mod.spdm(oracle_mod.convert(A), B)
         assert same_bits(h.spdm(torch.from_numpy(B).cuda()).cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("n", [63, 65, 127, 128, 129, 191, 254, 255, 257, 258, 383, 769, 1001])
+def test_ragged_widths_bit_identical(native, oracle_mod, n):
+    """Widths that 16-byte (or 8-byte) loads do not fit: several narrow loads
+    per lane, the last tile of a row overlapping the one before it; short
+    rows (two tiles at a time), long ones, and rows beyond one staging."""
+    import torch
+    from gcoospdm_gb300 import datagen as dg
+    for m, k, p, rows_per_group in ((37, 200, 0.02, 4), (9, 700, 0.5, 4), (5, 2600, 0.9, 8), (64, 300, 0.1, 32)):
+        A, B = dg.bernoulli_dense(n, m, k, p), dg.dense_pm1(n, 6, k, n)
+        C = torch.full((m + 1, n), 7.0, device="cuda")  # the row after C must stay
+        h = native.GcooHandle(torch.from_numpy(A).cuda(), rows_per_group=rows_per_group, fp32_order="rows").build()
+        h.spdm(torch.from_numpy(B).cuda(), C[:m])
+        assert same_bits(C[:m].cpu().numpy(), oracle_mod.spdm(oracle_mod.convert(A, rows_per_group), B)), (m, k)
+        assert bool((C[m] == 7.0).all())
