@@ -15,6 +15,10 @@
 //                                   + rank in the segment (column, then row)
 //                           packed: row_ptr[r] + prefix[r][s]
 //                                   + rank of the entry in row r's segment part.
+// Rows that do not start on 16 bytes (odd k, a shifted A) take the same path:
+// whole 16-byte granules are loaded and the lanes shift them against the row
+// (a rebuild of 4001 x 3999 at 2 %: 56 us against 114 us of a CTA per group
+// with 4-byte loads, A read twice; 4000 x 4000: 52 us).
 // Once the counts are scanned every warp is independent: a conversion of a
 // few hundred rows takes about one memory round trip, a large one streams A.
 #include "internal.cuh"
@@ -33,6 +37,57 @@ __device__ __forceinline__ uint32_t nzb(float v) { return v != 0.0f ? 1u : 0u; }
 __device__ __forceinline__ uint32_t nz_bits(const float4 &v)
 {
     return nzb(v.x) | (nzb(v.y) << 1) | (nzb(v.z) << 2) | (nzb(v.w) << 3);
+}
+
+// The segment's 4 columns of lane `lane` (zeros past the row's `valid`
+// columns), by a whole warp. seg: the row's first element of the segment.
+// AL: every row starts on 16 bytes (k % 4 == 0, A aligned). Otherwise the row
+// is shifted against the 16-byte granules by a warp-uniform 0..3 floats: each
+// lane loads one granule and takes the rest of its four columns from the next
+// lane's (lane 31 loads a 33rd); granules that reach outside A are read float
+// by float. LAST: A's last reader (a streaming load).
+template <bool AL, bool LAST>
+__device__ __forceinline__ float4 seg_load(const float *seg, int lane, int64_t valid, const float *A, const float *A_end)
+{
+    const auto load = [](const float *p) {
+        const float4 *q = reinterpret_cast<const float4 *>(p);
+        return LAST ? __ldcs(q) : __ldg(q);
+    };
+    if constexpr (AL)
+        return lane * 4 < valid ? load(seg + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int shift = static_cast<int>((reinterpret_cast<uintptr_t>(seg) >> 2) & 3u);
+    const float *base = seg - shift;
+    const auto granule = [&](int i) {
+        const float *p = base + 4 * i;
+        if (4 * i - shift >= valid)
+            return make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p >= A && p + 4 <= A_end)
+            return load(p);
+        const auto one = [&](const float *q) { return q >= A && q < A_end ? __ldg(q) : 0.0f; };
+        return make_float4(one(p), one(p + 1), one(p + 2), one(p + 3));
+    };
+    const float4 t = granule(lane);
+    float x[8] = {t.x, t.y, t.z, t.w, 0.f, 0.f, 0.f, 0.f};
+    if (shift) { // warp-uniform
+        const float4 last = lane == 31 ? granule(32) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float y0 = __shfl_down_sync(0xffffffffu, t.x, 1), y1 = __shfl_down_sync(0xffffffffu, t.y, 1),
+                    y2 = __shfl_down_sync(0xffffffffu, t.z, 1);
+        x[4] = lane == 31 ? last.x : y0;
+        x[5] = lane == 31 ? last.y : y1;
+        x[6] = lane == 31 ? last.z : y2;
+    }
+    if (shift & 1) {
+#pragma unroll
+        for (int i = 0; i < 7; ++i)
+            x[i] = x[i + 1];
+    }
+    if (shift & 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            x[i] = x[i + 2];
+    }
+    const int64_t left = valid - 4 * lane;
+    return make_float4(left > 0 ? x[0] : 0.f, left > 1 ? x[1] : 0.f, left > 2 ? x[2] : 0.f, left > 3 ? x[3] : 0.f);
 }
 
 // Unit of a warp: group g, segment s (CTA = 8 segments of a group).
@@ -61,7 +116,7 @@ __device__ __forceinline__ SegUnit seg_unit(int64_t m, int64_t k, int64_t tiles,
 // distinct (when not null) accumulates the number of distinct (group,
 // column) pairs, i.e. columns with a nonzero in at least one row of the
 // group; nnz / distinct tells how many rows of a group share a B row.
-template <int CPG>
+template <int CPG, bool AL>
 __global__ void __launch_bounds__(kTileThreads)
 seg_count_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, int64_t S,
                  int32_t *__restrict__ cnt, unsigned long long *__restrict__ distinct)
@@ -72,8 +127,8 @@ seg_count_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tile
     float4 v[CPG];
 #pragma unroll
     for (int r = 0; r < CPG; ++r)
-        v[r] = (u.live && r < u.nrows && u.c < k)
-                   ? __ldg(reinterpret_cast<const float4 *>(A + (u.r0 + r) * k + u.c))
+        v[r] = (u.live && r < u.nrows) // warp-uniform
+                   ? seg_load<AL, false>(A + (u.r0 + r) * k + u.s * kSegCols, lane, k - u.s * kSegCols, A, A + m * k)
                    : make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t any = 0;
 #pragma unroll
@@ -131,8 +186,8 @@ __global__ void seg_prefix_kernel(int32_t *__restrict__ cnt, int64_t m, int64_t 
 // Ranks inside one warp's segment: per row, the nonzeros of the lanes before
 // this one. Per-lane counts (0..4) are packed four rows to a word in 8-bit
 // fields so one warp scan per word serves four rows at once.
-template <int CPG>
-__device__ __forceinline__ void scatter_segment(const float *__restrict__ A, int64_t k, int64_t S, const SegUnit &u,
+template <int CPG, bool AL>
+__device__ __forceinline__ void scatter_segment(const float *__restrict__ A, int64_t m, int64_t k, int64_t S, const SegUnit &u,
                                                 const int32_t *__restrict__ pref,
                                                 const int32_t *__restrict__ group_index,
                                                 const int32_t *__restrict__ row_ptr, float *__restrict__ vals,
@@ -150,8 +205,9 @@ __device__ __forceinline__ void scatter_segment(const float *__restrict__ A, int
     float4 v[CPG];
 #pragma unroll
     for (int r = 0; r < CPG; ++r)
-        v[r] = (r < u.nrows && u.c < k) ? __ldcs(reinterpret_cast<const float4 *>(A + (u.r0 + r) * k + u.c))
-                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[r] = r < u.nrows // warp-uniform
+                   ? seg_load<AL, true>(A + (u.r0 + r) * k + u.s * kSegCols, lane, k - u.s * kSegCols, A, A + m * k)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t bits[CPG];
     uint32_t word[NP];
     uint32_t any = 0;
@@ -228,7 +284,7 @@ __device__ __forceinline__ void scatter_segment(const float *__restrict__ A, int
     }
 }
 
-template <int CPG>
+template <int CPG, bool AL>
 // 6 CTAs per SM for up to 4 rows per group: more loads of A in flight
 __global__ void __launch_bounds__(kTileThreads, CPG <= 4 ? 6 : 4)
 seg_scatter_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, int64_t S,
@@ -236,7 +292,7 @@ seg_scatter_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t ti
                    const int32_t *__restrict__ row_ptr, float *__restrict__ vals, int32_t *__restrict__ rows,
                    int32_t *__restrict__ cols, Entry *__restrict__ packed)
 {
-    scatter_segment<CPG>(A, k, S, seg_unit<CPG>(m, k, tiles, blockIdx.x), pref, group_index, row_ptr, vals, rows,
+    scatter_segment<CPG, AL>(A, m, k, S, seg_unit<CPG>(m, k, tiles, blockIdx.x), pref, group_index, row_ptr, vals, rows,
                          cols, packed);
 }
 
@@ -258,7 +314,33 @@ seg_scatter_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t ti
 // 1024 / (32 L) warps: with L = 8 each warp's fixed costs (barriers, ranks,
 // the tile's bookkeeping) serve twice the columns and 4-warp CTAs fit 12 per
 // SM (192 KB of A in flight per SM against 128 KB with 8-warp CTAs).
-template <int CPG, int L>
+// The whole 16-byte granules of a row piece of w floats at p: floats [from,
+// to), the piece shifted by `shift` floats against 16 bytes. Without a whole
+// granule to == from, and the floats before `from` (at most w) and from `to`
+// on are the piece.
+struct RowPiece {
+    int shift, from, to;
+    __device__ __forceinline__ uint32_t bytes() const { return static_cast<uint32_t>(to - from) * 4u; }
+};
+
+__device__ __forceinline__ RowPiece row_piece(const float *p, int w)
+{
+    RowPiece x;
+    x.shift = static_cast<int>((reinterpret_cast<uintptr_t>(p) >> 2) & 3u);
+    x.from = (4 - x.shift) & 3;
+    if (x.from > w)
+        x.from = w;
+    x.to = w - ((x.shift + w) & 3);
+    if (x.to < x.from)
+        x.to = x.from;
+    return x;
+}
+
+// AL: as in seg_load. Otherwise a row piece sits in shared memory shifted by
+// its 0..3 floats against 16 bytes: its whole granules arrive by bulk copy,
+// the up to three floats on either side by plain loads, and each lane reads
+// one float4 more and shifts.
+template <int CPG, int L, bool AL>
 __global__ void __launch_bounds__(1024 / L, L == 8 ? 12 : (CPG <= 4 ? 8 : 6))
 stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, int64_t S, int32_t *__restrict__ cnt,
              unsigned long long *__restrict__ distinct, int32_t slot, uint2 *__restrict__ stage,
@@ -271,7 +353,7 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
     static_assert(kWarps == 4 || kWarps == 8, "two int4 loads at most read the warp totals");
     // the tile's rows arrive by bulk copies: no registers held while they are in
     // flight, so a full complement of CTAs per SM keeps A streaming
-    __shared__ __align__(128) float s_a[CPG][kTileCols];
+    __shared__ __align__(128) float s_a[CPG][kTileCols + (AL ? 0 : 4)];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ __align__(16) int s_wtot[8];
     __shared__ int s_dist[8];
@@ -283,13 +365,26 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
         fence_mbar_init();
         const SegUnit u0 = seg_unit<CPG>(m, k, tiles, b);
         s_g = u0.g;
-        // k % 4 == 0 and a 16-byte aligned A: every row piece starts on 16 bytes and is a multiple of 16 long
         const int64_t c0 = (b - u0.g * tiles) * kTileCols;
         const int64_t w = k - c0 < kTileCols ? k - c0 : kTileCols;
-        const uint32_t bytes = static_cast<uint32_t>(w * static_cast<int64_t>(sizeof(float)));
-        mbar_arrive_expect_tx(&s_bar, bytes * static_cast<uint32_t>(u0.nrows));
-        for (int r = 0; r < u0.nrows; ++r)
-            bulk_g2s(s_a[r], A + (u0.r0 + r) * k + c0, bytes, &s_bar);
+        if constexpr (AL) {
+            // every row piece starts on 16 bytes and is a multiple of 16 long
+            const uint32_t bytes = static_cast<uint32_t>(w * static_cast<int64_t>(sizeof(float)));
+            mbar_arrive_expect_tx(&s_bar, bytes * static_cast<uint32_t>(u0.nrows));
+            for (int r = 0; r < u0.nrows; ++r)
+                bulk_g2s(s_a[r], A + (u0.r0 + r) * k + c0, bytes, &s_bar);
+        } else {
+            uint32_t bytes = 0;
+            for (int r = 0; r < u0.nrows; ++r)
+                bytes += row_piece(A + (u0.r0 + r) * k + c0, static_cast<int>(w)).bytes();
+            mbar_arrive_expect_tx(&s_bar, bytes);
+            for (int r = 0; r < u0.nrows; ++r) {
+                const float *p = A + (u0.r0 + r) * k + c0;
+                const RowPiece x = row_piece(p, static_cast<int>(w));
+                if (x.bytes())
+                    bulk_g2s(&s_a[r][x.shift + x.from], p + x.from, x.bytes(), &s_bar);
+            }
+        }
     }
     __syncthreads();
     const int64_t g = s_g;
@@ -299,6 +394,20 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
     const int sc = warp * (32 * L) + lane * L;                        // the lane's first column inside the tile
     const int64_t c = t * kTileCols + sc;                              // ... in A
     const int64_t s0 = t * (kTileCols / kSegCols) + warp * kSegPerWarp; // the warp's first segment
+    // 4-byte shift of row r's piece against 16 bytes: (sh0 + r * k) & 3
+    const unsigned sh0 = AL ? 0u : static_cast<unsigned>((reinterpret_cast<uintptr_t>(A) >> 2) + r0 * k + t * kTileCols);
+    const unsigned k3 = static_cast<unsigned>(k);
+    if (!AL && threadIdx.x < 8 * CPG) { // the floats outside whole granules: 4 threads per row and side
+        const int r = threadIdx.x >> 3, i = threadIdx.x & 7;
+        const int w = static_cast<int>(k - t * kTileCols < kTileCols ? k - t * kTileCols : kTileCols);
+        if (r < nrows) {
+            const float *p = A + (r0 + r) * k + t * kTileCols;
+            const RowPiece x = row_piece(p, w);
+            const int j = i < 4 ? i : x.to + i - 4;
+            if (i < 4 ? j < x.from : j < w)
+                s_a[r][x.shift + j] = __ldg(p + j);
+        }
+    }
     // one warp polls the barrier, the others wait at the CTA barrier (no issue
     // slots spent); a wait that gives up (it never should) flags the build,
     // which the host then redoes on the two-pass path, once the copies landed
@@ -316,7 +425,29 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
     uint32_t msk = 0;
 #pragma unroll
     for (int r = 0; r < CPG; ++r) {
-        if (r < nrows) {
+        if (!AL && r < nrows) {
+            const unsigned shift = (sh0 + static_cast<unsigned>(r) * k3) & 3u;
+            float x[L + 4];
+#pragma unroll
+            for (int h = 0; h < L / 4 + 1; ++h) {
+                const float4 y = *reinterpret_cast<const float4 *>(&s_a[r][sc + 4 * h]);
+                x[4 * h] = y.x; x[4 * h + 1] = y.y; x[4 * h + 2] = y.z; x[4 * h + 3] = y.w;
+            }
+            if (shift & 1u) {
+#pragma unroll
+                for (int i = 0; i < L + 3; ++i)
+                    x[i] = x[i + 1];
+            }
+            if (shift & 2u) {
+#pragma unroll
+                for (int i = 0; i < L + 1; ++i)
+                    x[i] = x[i + 2];
+            }
+#pragma unroll
+            for (int q = 0; q < L; ++q)
+                msk |= (c + q < k ? nzb(x[q]) : 0u) << (q * CPG + r);
+        }
+        if (AL && r < nrows) {
 #pragma unroll
             for (int h = 0; h < L / 4; ++h) {
                 if (c + 4 * h < k) { // k % 4 == 0: a float4 is wholly inside or wholly past the row
@@ -406,11 +537,11 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
         msk &= msk - 1u;
         const int q = i / CPG, r = i % CPG;
         stage[pos++] = make_uint2((static_cast<uint32_t>(c + q) << 3) | static_cast<uint32_t>(r),
-                                  __float_as_uint(s_a[r][sc + q]));
+                                  __float_as_uint(s_a[r][(AL ? 0u : ((sh0 + static_cast<unsigned>(r) * k3) & 3u)) + sc + q]));
     }
 }
 
-template <int CPG>
+template <int CPG, bool AL>
 __global__ void __launch_bounds__(kTileThreads, CPG <= 4 ? 6 : 4)
 place_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, int64_t S, int64_t units,
              int32_t slot, const uint2 *__restrict__ stage, const int32_t *__restrict__ tile_tot,
@@ -492,7 +623,7 @@ place_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
     const int64_t n_over = static_cast<int64_t>(*over_count);
     const int64_t stride = static_cast<int64_t>(gridDim.x) - staged_blocks;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) - staged_blocks; i < n_over; i += stride)
-        scatter_segment<CPG>(A, k, S, seg_unit<CPG>(m, k, tiles, over_list[i]), pref, group_index, row_ptr, vals,
+        scatter_segment<CPG, AL>(A, m, k, S, seg_unit<CPG>(m, k, tiles, over_list[i]), pref, group_index, row_ptr, vals,
                              rows, cols, packed);
 }
 
@@ -500,13 +631,15 @@ place_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
 
 int64_t conv_segments(int64_t k) { return (k + kSegCols - 1) / kSegCols; }
 
+// Every row of A starts on 16 bytes
+static bool rows_aligned(const float *A, int64_t k) { return k % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0; }
+
 static int64_t conv_tiles(int64_t k) { return (k + kTileCols - 1) / kTileCols; }
 
 bool tiled_convert_ok(const float *A, int64_t m, int64_t k, int32_t cpg)
 {
     const int64_t units = ((m + cpg - 1) / cpg) * conv_tiles(k);
-    return k % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && cpg <= 8 && units > 0 &&
-           units < 0x7fffffffLL;
+    return (reinterpret_cast<uintptr_t>(A) & 3) == 0 && cpg <= 8 && units > 0 && units < 0x7fffffffLL;
 }
 
 cudaError_t launch_tile_count(const float *A, int64_t m, int64_t k, int32_t cpg, int32_t *cnt,
@@ -517,13 +650,18 @@ cudaError_t launch_tile_count(const float *A, int64_t m, int64_t k, int32_t cpg,
     if (units <= 0)
         return cudaSuccess;
     const unsigned grid = static_cast<unsigned>(units);
+    const bool al = rows_aligned(A, k);
+#define GCOO_SEG_COUNT(C)                                                                             \
+    (al ? seg_count_kernel<C, true> : seg_count_kernel<C, false>)<<<grid, kTileThreads, 0, st>>>(     \
+        A, m, k, tiles, S, cnt, distinct)
     switch (cpg) {
-    case 1: seg_count_kernel<1><<<grid, kTileThreads, 0, st>>>(A, m, k, tiles, S, cnt, distinct); break;
-    case 2: seg_count_kernel<2><<<grid, kTileThreads, 0, st>>>(A, m, k, tiles, S, cnt, distinct); break;
-    case 4: seg_count_kernel<4><<<grid, kTileThreads, 0, st>>>(A, m, k, tiles, S, cnt, distinct); break;
-    case 8: seg_count_kernel<8><<<grid, kTileThreads, 0, st>>>(A, m, k, tiles, S, cnt, distinct); break;
+    case 1: GCOO_SEG_COUNT(1); break;
+    case 2: GCOO_SEG_COUNT(2); break;
+    case 4: GCOO_SEG_COUNT(4); break;
+    case 8: GCOO_SEG_COUNT(8); break;
     default: return cudaErrorInvalidValue;
     }
+#undef GCOO_SEG_COUNT
     count_launches(1);
     return cudaGetLastError();
 }
@@ -549,9 +687,10 @@ cudaError_t launch_tile_scatter(const float *A, int64_t m, int64_t k, int32_t cp
     if (units <= 0)
         return cudaSuccess;
     const unsigned grid = static_cast<unsigned>(units);
-#define GCOO_SEG_SCATTER(C)                                                                                    \
-    seg_scatter_kernel<C><<<grid, kTileThreads, 0, st>>>(A, m, k, tiles, S, pref, group_index, row_ptr, vals, \
-                                                         rows, cols, packed)
+    const bool al = rows_aligned(A, k);
+#define GCOO_SEG_SCATTER(C)                                                                                     \
+    (al ? seg_scatter_kernel<C, true> : seg_scatter_kernel<C, false>)<<<grid, kTileThreads, 0, st>>>(           \
+        A, m, k, tiles, S, pref, group_index, row_ptr, vals, rows, cols, packed)
     switch (cpg) {
     case 1: GCOO_SEG_SCATTER(1); break;
     case 2: GCOO_SEG_SCATTER(2); break;
@@ -591,9 +730,10 @@ cudaError_t launch_stage(const float *A, int64_t m, int64_t k, int32_t cpg, int3
     if (units <= 0)
         return cudaSuccess;
     const unsigned grid = static_cast<unsigned>(units);
-#define GCOO_STAGE(C, L)                                                                                        \
-    stage_kernel<C, L><<<grid, 1024 / (L), 0, st>>>(A, m, k, tiles, S, cnt, distinct, slot, stage, tile_tot,   \
-                                                    over_list, over_count, status)
+    const bool al = rows_aligned(A, k);
+#define GCOO_STAGE(C, L)                                                                          \
+    (al ? stage_kernel<C, L, true> : stage_kernel<C, L, false>)<<<grid, 1024 / (L), 0, st>>>(     \
+        A, m, k, tiles, S, cnt, distinct, slot, stage, tile_tot, over_list, over_count, status)
     switch (cpg) {
     case 1: GCOO_STAGE(1, 8); break;
     case 2: GCOO_STAGE(2, 8); break;
@@ -622,10 +762,11 @@ cudaError_t launch_place(const float *A, int64_t m, int64_t k, int32_t cpg, int3
     if (rescan_blocks > units)
         rescan_blocks = units;
     const unsigned grid = static_cast<unsigned>(staged_blocks + rescan_blocks);
-#define GCOO_PLACE(C)                                                                                            \
-    place_kernel<C><<<grid, kTileThreads, 0, st>>>(A, m, k, tiles, S, units, slot, stage, tile_tot, over_list,  \
-                                                   over_count, pref, group_index, row_ptr, vals, rc, packed,   \
-                                                   d_total, cap, packed_cap, staged_blocks)
+    const bool al = rows_aligned(A, k);
+#define GCOO_PLACE(C)                                                                                 \
+    (al ? place_kernel<C, true> : place_kernel<C, false>)<<<grid, kTileThreads, 0, st>>>(             \
+        A, m, k, tiles, S, units, slot, stage, tile_tot, over_list, over_count, pref, group_index,    \
+        row_ptr, vals, rc, packed, d_total, cap, packed_cap, staged_blocks)
     switch (cpg) {
     case 1: GCOO_PLACE(1); break;
     case 2: GCOO_PLACE(2); break;

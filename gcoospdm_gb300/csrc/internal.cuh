@@ -114,7 +114,7 @@ cudaError_t launch_scatter(const float *A, int64_t m, int64_t k, int32_t rows_pe
 
 // ---- tiled conversion (convert_tiled.cu): a warp per (group, 128-column segment)
 int64_t conv_segments(int64_t k); // segments per row: the count array is m x conv_segments(k)
-// The tiled kernels need k % 4 == 0, a 16-byte aligned A and rows_per_group <= 8.
+// The tiled kernels need a 4-byte aligned A and rows_per_group <= 8 (rows that all start on 16 bytes: fewer instructions).
 bool tiled_convert_ok(const float *A, int64_t m, int64_t k, int32_t cpg);
 // cnt[r * S + s] = nonzeros of row r in column segment s (S = conv_segments(k)).
 // distinct (may be null; zeroed by the caller) += columns with a nonzero in
