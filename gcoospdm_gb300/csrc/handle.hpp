@@ -46,6 +46,7 @@ struct gcoo_handle {
     gcoo::DevBuf<int32_t> tile_tot;  // staged rebuild: entries per tile, -1 when it overflowed
     gcoo::DevBuf<int32_t> over_list; // staged rebuild: the overflowed tiles
     int64_t *readback = nullptr;     // page-locked: the staged build's readback
+    cudaEvent_t ev_totals = nullptr; // ... and the point in the stream where it is written
     gcoo::DevBuf<int32_t> long_rows; // skewed matrices: rows multiplied by the long-row kernel
     gcoo::DevBuf<unsigned long long> long_count; // [0] long rows, [1] their entries
     int64_t n_long = 0;
@@ -74,6 +75,8 @@ struct gcoo_handle {
     {
         if (readback)
             cudaFreeHost(readback);
+        if (ev_totals)
+            cudaEventDestroy(ev_totals);
         if (ev_fork)
             cudaEventDestroy(ev_fork);
         if (ev_join)

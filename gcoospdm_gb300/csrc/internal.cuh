@@ -123,6 +123,13 @@ cudaError_t launch_tile_count(const float *A, int64_t m, int64_t k, int32_t cpg,
                               unsigned long long *distinct, cudaStream_t st);
 // cnt rows -> exclusive prefix over segments (in place); row totals -> row_cnt[0..m).
 cudaError_t launch_tile_prefix(int32_t *cnt, int64_t m, int64_t k, int32_t *row_cnt, cudaStream_t st);
+// launch_tile_prefix and launch_row_scan_max in one launch (prefix_scan_ok: up
+// to 16384 rows); d_total[1] needs no zeroing, *ticket does. host_words (may
+// be null): page-locked memory that receives d_total[0..3].
+bool prefix_scan_ok(int64_t m);
+cudaError_t launch_prefix_scan(int32_t *cnt, int64_t segments, int32_t *row_ptr, int64_t m, int32_t cpg,
+                               int32_t *group_index, int32_t *nnz_per_group, int64_t *d_total, unsigned int *ticket,
+                               int64_t *host_words, uint32_t *status, cudaStream_t st);
 // Same outputs as launch_scatter, from the segment prefixes.
 cudaError_t launch_tile_scatter(const float *A, int64_t m, int64_t k, int32_t cpg, const int32_t *pref,
                                 const int32_t *group_index, const int32_t *row_ptr, float *vals,
@@ -143,12 +150,13 @@ cudaError_t launch_stage(const float *A, int64_t m, int64_t k, int32_t cpg, int3
 // After launch_tile_prefix and launch_row_scan: the GCOO arrays (vals, rc =
 // rows | cols at rc + total) and the packed row order, total = d_total[0] read
 // on the device; writes nothing unless the stage status (d_total[3]) is 0,
-// total <= cap and total + 2 <= packed_cap.
+// total <= cap and total + 2 <= packed_cap; then, with clear_rows (m + 1 row
+// pointers, may be null), those are zeroed: no row has entries to read.
 cudaError_t launch_place(const float *A, int64_t m, int64_t k, int32_t cpg, int32_t slot, const uint2 *stage,
                          const int32_t *tile_tot, const int32_t *over_list, const unsigned long long *over_count,
                          const int32_t *pref, const int32_t *group_index, const int32_t *row_ptr, float *vals,
                          int32_t *rc, Entry *packed, const int64_t *d_total, int64_t cap, int64_t packed_cap,
-                         cudaStream_t st);
+                         int32_t *clear_rows, cudaStream_t st);
 
 // ---- FP32 multiply (spdm_fp32.cu) ------------------------------------------------------
 int device_sms(); // SMs of the current device (152 on a GB300)

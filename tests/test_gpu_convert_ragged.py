@@ -44,3 +44,26 @@ def test_ragged_rows_convert(native, oracle_mod, k, cpg):
         A2[m // 2] = 0.0
         h.build()
         check(h, oracle_mod.convert(A2, cpg))
+
+
+@pytest.mark.parametrize("cpg", [4, 8])
+@pytest.mark.parametrize("m", [1, 31, 33, 8192, 8193, 16384, 16385])
+def test_row_scan_edges(native, oracle_mod, m, cpg):
+    """The one-launch prefix and scan (up to 16384 rows, 32 rows per CTA, 8192
+    per scan chunk) and the launches beyond it; first build, rebuild, and a
+    multiply that goes ahead of the rebuild's readback, also where the arrays
+    turn out too small for it."""
+    import torch
+    rng = np.random.default_rng(m + cpg)
+    A = np.where(rng.random((m, 130)) < 0.1, rng.standard_normal((m, 130)), 0.0).astype(np.float32)
+    B = rng.standard_normal((130, 36)).astype(np.float32)
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    h = native.GcooHandle(dA, rows_per_group=cpg).build()
+    check(h, oracle_mod.convert(A, cpg))
+    for density in (0.1, 0.02, 0.9, 0.9):
+        A = np.where(rng.random((m, 130)) < density, rng.standard_normal((m, 130)), 0.0).astype(np.float32)
+        dA.copy_(torch.from_numpy(A))
+        C = h.multiply_by(dB)
+        ref = oracle_mod.convert(A, cpg)
+        check(h, ref)
+        assert np.array_equal(C.cpu().numpy().view(np.uint32), oracle_mod.spdm(ref, B).view(np.uint32))
