@@ -446,17 +446,17 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
             return s;
         return finish_build(h, st);
     }
-    const size_t sc = scan_scratch_elems(h->m);
+    const int32_t cpg = h->p.rows_per_group;
+    const bool tiled = tiled_convert_ok(h->dA, h->m, h->k, cpg);
+    const bool one_scan = tiled && prefix_scan_ok(h->m); // needs no scan scratch
     if (!h->row_ptr.ensure(static_cast<size_t>(h->m) + 1) || !h->groups.ensure(2 * static_cast<size_t>(h->ng + 1)) ||
-        !h->scratch.ensure(sc) || !h->status.ensure(2 + 8 * 2))
+        (!one_scan && !h->scratch.ensure(scan_scratch_elems(h->m))) || !h->status.ensure(2 + 8 * 2))
         return fail(GCOO_ERROR_ALLOC, "device allocation of the GCOO index arrays failed");
     // [0] total nnz, [1] longest row, [2] distinct group columns, [3] staging status, [4] overflowed tiles,
     // [5] ticket of the prefix-and-scan kernel; behind the status word: one memset clears all
     int64_t *d_total = reinterpret_cast<int64_t *>(h->status.ptr + 2);
     GCOO_CUDA(cudaMemsetAsync(h->status.ptr, 0, 8 + 8 * sizeof(int64_t), st));
     unsigned int *ticket = reinterpret_cast<unsigned int *>(d_total + 5);
-    const int32_t cpg = h->p.rows_per_group;
-    const bool tiled = tiled_convert_ok(h->dA, h->m, h->k, cpg);
     // One read of A when the entry arrays of an earlier build have room (a
     // steady loop of mutiplyBy / build); otherwise, or if they turn out too
     // small, the two-pass path below converts and sizes them exactly.
@@ -478,11 +478,10 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
             h->ev_totals = made;
         }
         unsigned long long *over_count = reinterpret_cast<unsigned long long *>(d_total + 4);
-        const bool one_scan = prefix_scan_ok(h->m); // which also writes the readback words
         GCOO_CUDA(launch_stage(h->dA, h->m, h->k, cpg, slot, h->tile_cnt.ptr,
                                reinterpret_cast<unsigned long long *>(d_total + 2), h->stage.ptr, h->tile_tot.ptr,
                                h->over_list.ptr, over_count, reinterpret_cast<uint32_t *>(d_total + 3), st));
-        if (one_scan) {
+        if (one_scan) { // which also writes the readback words
             GCOO_CUDA(launch_prefix_scan(h->tile_cnt.ptr, conv_segments(h->k), h->row_ptr.ptr, h->m, cpg,
                                          h->group_index(), h->nnz_per_group(), d_total, ticket, h->readback,
                                          h->status.ptr, st));
@@ -530,7 +529,7 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
     } else {
         GCOO_CUDA(launch_row_count(h->dA, h->m, h->k, h->row_ptr.ptr, st));
     }
-    if (tiled && prefix_scan_ok(h->m)) {
+    if (one_scan) {
         GCOO_CUDA(launch_prefix_scan(h->tile_cnt.ptr, conv_segments(h->k), h->row_ptr.ptr, h->m, cpg, h->group_index(),
                                      h->nnz_per_group(), d_total, ticket, nullptr, h->status.ptr, st));
     } else {

@@ -22,6 +22,16 @@ namespace gcoo {
 namespace {
 
 constexpr int kChunk = 2048; // most entries staged per pass (16 KB)
+// 4-warp CTAs of the row walk per SM: 48 registers a thread. Measured (us;
+// 16384^2 at 0.1 %, 8192^2 at 1 % with its conversion, B 8192 x 1024 from the
+// left): 8 CTAs 1067 / 1106 / 182, 9 1032 / 1096 / 179, 10 1011 / 1088 / 178,
+// 12 1024 / 1092 / 194, against 1085 / 1104 / 183 with neither this bound nor
+// batched row tails (44 registers).
+constexpr int kRowCtas = 10;
+// rows shorter than this walk two column tiles at once: twice the loads in
+// flight (16384^2 at 0.1 %, rows of ~16: 1011 us below 16 entries, 959 below
+// 24, 955 below 32 or 64; 8192^2 at 1 % is slower from 1000 on)
+constexpr int kPairRows = 32;
 
 // V output columns of a lane, in V / W loads of W consecutive columns at
 // strides of 32 W: W = V where B's and C's rows are aligned for it, else the
@@ -148,6 +158,39 @@ __device__ __forceinline__ void row_chain(const Entry *__restrict__ s, int cnt, 
             for (int v = 0; v < V; ++v)
                 acc[v] = fmaf(e[u].val, b[u][v], acc[v]);
     }
+    // the tail in batches too: a row of 20 entries takes 4 round trips, not 6
+    if (U == 8 && i + 4 <= cnt) {
+        Entry e[4];
+        float b[4][V];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            e[u] = s[i + u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            Vec<V, W>::load(Bj + static_cast<int64_t>(e[u].col) * n, b[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                acc[v] = fmaf(e[u].val, b[u][v], acc[v]);
+        i += 4;
+    }
+    if (i + 2 <= cnt) {
+        Entry e[2];
+        float b[2][V];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            e[u] = s[i + u];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            Vec<V, W>::load(Bj + static_cast<int64_t>(e[u].col) * n, b[u]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                acc[v] = fmaf(e[u].val, b[u][v], acc[v]);
+        i += 2;
+    }
 #pragma unroll 1
     for (; i < cnt; ++i) {
         const Entry e = s[i];
@@ -187,6 +230,26 @@ __device__ __forceinline__ void row_chain_pair(const Entry *__restrict__ s, int 
                 acc_b[v] = fmaf(e[u].val, bb[u][v], acc_b[v]);
             }
     }
+    if (i + 2 <= cnt) {
+        Entry e[2];
+        float ba[2][V], bb[2][V];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            e[u] = s[i + u];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            Vec<V, W>::load(Ba + static_cast<int64_t>(e[u].col) * n, ba[u]);
+            Vec<V, W>::load(Bb + static_cast<int64_t>(e[u].col) * n, bb[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                acc_a[v] = fmaf(e[u].val, ba[u][v], acc_a[v]);
+                acc_b[v] = fmaf(e[u].val, bb[u][v], acc_b[v]);
+            }
+        i += 2;
+    }
 #pragma unroll 1
     for (; i < cnt; ++i) {
         const Entry e = s[i];
@@ -207,7 +270,7 @@ __device__ __forceinline__ void row_chain_pair(const Entry *__restrict__ s, int 
 // warp walks col_iters column tiles, col_warps tiles apart, reusing the
 // staged entries, so short rows do not pay one staging per tile.
 template <int V, int W, int MAXT, bool PIPE, bool MULTI>
-__global__ void __launch_bounds__(MAXT)
+__global__ void __launch_bounds__(MAXT, MAXT == 128 ? kRowCtas : 1)
 spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m,
                  int32_t cpg, const float *__restrict__ B, int64_t n, float *__restrict__ C,
                  int32_t col_warps, int32_t col_iters, int32_t chunk_cap, uint32_t *__restrict__ status)
@@ -296,7 +359,7 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
         int it = 0;
         // very short rows: two tiles at a time, twice the B loads in flight
         // (longer rows already keep a batch of 8 loads in flight per tile)
-        for (; cnt < 16 && it + 1 < col_iters; it += 2) {
+        for (; cnt < kPairRows && it + 1 < col_iters; it += 2) {
             const LaneCols<V, W> aa(j + it * tile_stride, lane, n), ab(j + it * tile_stride + tile_stride, lane, n);
             if (!aa.on)
                 break;
@@ -565,12 +628,13 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
         const int64_t tile = static_cast<int64_t>(s.col_warps) * 32 * s.vec;
         const int64_t ny = (n + tile - 1) / tile;
         // about 768 columns per CTA (0.5-0.9 K columns measured best from
-        // 2048^2 to 16384^2 at 1 % to 0.1 % density), but at least two waves
-        // of CTAs (12 four-warp CTAs resident per SM) on small matrices
+        // 2048^2 to 16384^2 at 1 % to 0.1 % density), but at least four waves
+        // of CTAs on small matrices: the last wave's share of the time (4096^2
+        // at 5 % 623 us with two, 604 with four; 2048^2 at 10 % 148 and 141)
         int64_t ci = 768 / tile;
         const int64_t groups = (m + s.rows - 1) / s.rows;
-        const int64_t resident = static_cast<int64_t>(device_sms()) * (s.warps <= 4 ? 12 : 6);
-        const int64_t by_grid = groups * ny / (2 * resident);
+        const int64_t resident = static_cast<int64_t>(device_sms()) * (s.warps <= 4 ? kRowCtas : 6);
+        const int64_t by_grid = groups * ny / (4 * resident);
         ci = ci > by_grid ? by_grid : ci;
         ci = ci < 1 ? 1 : (ci > ny ? ny : ci);
         s.col_iters = static_cast<int>(ci > 64 ? 64 : ci);
@@ -618,7 +682,9 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
         else GCOO_FP32_LAUNCH(1, 1, T, P);                                                              \
     } while (0)
     const bool pipe = s.depth >= 2;
-    if (threads <= 512) {
+    if (threads <= 128 && !pipe) {
+        GCOO_FP32_VEC(128, false);
+    } else if (threads <= 512) {
         if (pipe) GCOO_FP32_VEC(512, true);
         else GCOO_FP32_VEC(512, false);
     } else {
