@@ -737,6 +737,15 @@ gcoo_status gcoo_convert_count(const float *dA, int64_t m, int64_t k, int32_t ro
     if (!valid_cpg(rows_per_group))
         return fail(GCOO_ERROR_INVALID_VALUE, "rows_per_group must be a power of two in [1, 32]");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t ng = (m + rows_per_group - 1) / rows_per_group;
+    if (group_counts_ok(dA, m, k, ng)) {
+        GCOO_CUDA(launch_group_counts(dA, m, k, rows_per_group, d_group_index, d_nnz_per_group, st));
+        int32_t total = 0;
+        GCOO_CUDA(cudaMemcpyAsync(&total, d_group_index + ng, sizeof(total), cudaMemcpyDeviceToHost, st));
+        GCOO_CUDA(cudaStreamSynchronize(st));
+        *nnz = total;
+        return GCOO_SUCCESS;
+    }
     DevBuf<int32_t> counts;
     DevBuf<int64_t> scratch;
     const size_t sc = scan_scratch_elems(m);

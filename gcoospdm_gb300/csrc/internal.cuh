@@ -102,6 +102,11 @@ size_t scan_scratch_elems(int64_t m);
 cudaError_t launch_row_scan(int32_t *row_counts_then_ptr, int64_t m, int32_t rows_per_group,
                             int32_t *group_index, int32_t *nnz_per_group, int64_t *d_total,
                             int64_t *scratch, uint32_t *status, cudaStream_t st);
+// group_index and nnz_per_group from A alone, without scratch (the total is
+// group_index[ng]): up to 16384 groups of a matrix of fewer than 2^31 elements.
+bool group_counts_ok(const float *A, int64_t m, int64_t k, int64_t ng);
+cudaError_t launch_group_counts(const float *A, int64_t m, int64_t k, int32_t cpg, int32_t *group_index,
+                                int32_t *nnz_per_group, cudaStream_t st);
 // launch_row_scan followed by the longest row into d_total[1] (zeroed by the
 // caller): one single-CTA kernel for up to 16384 rows, else the two launches.
 cudaError_t launch_row_scan_max(int32_t *row_counts_then_ptr, int64_t m, int32_t rows_per_group,

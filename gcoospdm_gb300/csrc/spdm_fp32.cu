@@ -504,36 +504,151 @@ spdm_short_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
         Piece<V>::store(C + row * n + j, acc);
 }
 
+// A row tile's sums so far, from C (its own columns only, see LaneCols)
+template <int V, int W>
+__device__ __forceinline__ void view_resume(const float *c, const LaneCols<V, W> &at, bool resume, float (&acc)[V])
+{
+#pragma unroll
+    for (int h = 0; h < V / W; ++h)
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+            acc[h * W + w] = resume && at.j + h * 32 * W >= at.from ? c[h * 32 * W + w] : 0.0f;
+}
+
 // Multiply straight from reference-layout arrays (entries of a group in
-// column-then-row order, separate vals/rows/cols): one thread per output
-// column, one shared-memory accumulator per (group row, column) so any
-// rows_per_group works; each accumulator still sees its row's entries in
-// column order, hence the same fmaf chain.
-constexpr int kViewThreads = 128;
-__global__ void __launch_bounds__(kViewThreads)
+// column-then-row order, separate vals/rows/cols, any rows_per_group up to
+// 32). One CTA per (group, strip of column tiles): the group's entries are
+// staged in chunks and sorted by row in shared memory (each warp ranks its
+// rows' entries with one ballot per 32, which keeps their column order), then
+// each warp walks its rows over the strip's tiles as spdm_fp32_kernel does:
+// the same fmaf chains. An entry whose row is not in its group is skipped.
+// Bound like the row walk by the gather of B rows (nnz * n * 4 bytes from
+// L2): 4096^2 at 1 %, n = 2048 76 us, against 306 us of a thread per column
+// with one 4-byte load in flight and its sums in shared memory.
+constexpr int kViewMaxWarps = 8;
+
+template <int V, int W>
+__global__ void __launch_bounds__(kViewMaxWarps * 32, 5)
 spdm_view_kernel(const float *__restrict__ vals, const int32_t *__restrict__ rows,
                  const int32_t *__restrict__ cols, const int32_t *__restrict__ group_index,
-                 const int32_t *__restrict__ nnz_per_group, int64_t m, int32_t cpg,
+                 const int32_t *__restrict__ nnz_per_group, int64_t m, int32_t cpg, int32_t chunk, int32_t col_iters,
                  const float *__restrict__ B, int64_t n, float *__restrict__ C)
 {
-    extern __shared__ float s_acc[]; // [cpg][kViewThreads]
-    const int64_t g = blockIdx.x;
-    const int64_t r0 = g * cpg;
-    const int64_t j = static_cast<int64_t>(blockIdx.y) * kViewThreads + threadIdx.x;
-    for (int r = 0; r < cpg; ++r)
-        s_acc[r * kViewThreads + threadIdx.x] = 0.0f;
-    const int64_t e0 = group_index[g];
-    const int64_t e1 = e0 + nnz_per_group[g];
-    if (j < n) {
-        for (int64_t e = e0; e < e1; ++e) {
-            const int32_t lr = rows[e] - static_cast<int32_t>(r0);
-            if (lr < 0 || lr >= cpg)
-                continue; // not this group's row: malformed input, skipped
-            float *a = s_acc + lr * kViewThreads + threadIdx.x;
-            *a = fmaf(vals[e], __ldg(B + static_cast<int64_t>(cols[e]) * n + j), *a);
+    extern __shared__ __align__(128) unsigned char smem[];
+    Entry *s_sorted = reinterpret_cast<Entry *>(smem); // by row
+    Entry *s_raw = s_sorted + chunk;                   // as stored
+    uint8_t *s_lr = reinterpret_cast<uint8_t *>(s_raw + chunk); // row in group, 255: none
+    __shared__ int s_start[33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * cpg;
+    const int nrows = static_cast<int>(r0 + cpg <= m ? cpg : m - r0);
+    const int64_t e0 = group_index[blockIdx.x];
+    const int64_t total = nnz_per_group[blockIdx.x];
+    const int64_t j0 = static_cast<int64_t>(blockIdx.y) * col_iters * (32 * V) + (W == V ? lane * V : 0);
+    const unsigned lt = (1u << lane) - 1u;
+
+    // entries [first, first + cnt) of the group into s_sorted, row r's at s_start[r]
+    const auto stage = [&](int64_t first, int cnt) {
+        __syncthreads(); // the previous chunk has been consumed
+        for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+            const int64_t e = e0 + first + i;
+            const int64_t lr = rows[e] - r0;
+            Entry t;
+            t.col = cols[e];
+            t.val = vals[e];
+            s_raw[i] = t;
+            s_lr[i] = lr >= 0 && lr < nrows ? static_cast<uint8_t>(lr) : 255;
         }
-        for (int r = 0; r < cpg && r0 + r < m; ++r)
-            C[(r0 + r) * n + j] = s_acc[r * kViewThreads + threadIdx.x];
+        __syncthreads();
+        for (int r = warp; r < nrows; r += nwarps) {
+            int c = 0;
+            for (int i = 0; i < cnt; i += 32)
+                c += __popc(__ballot_sync(0xffffffffu, i + lane < cnt && s_lr[i + lane] == r));
+            if (lane == 0)
+                s_start[r + 1] = c;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            int x = lane < nrows ? s_start[lane + 1] : 0;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d)
+                    x += y;
+            }
+            __syncwarp();
+            if (lane < nrows)
+                s_start[lane + 1] = x;
+            if (lane == 0)
+                s_start[0] = 0;
+        }
+        __syncthreads();
+        for (int r = warp; r < nrows; r += nwarps) {
+            int at = s_start[r];
+            for (int i = 0; i < cnt; i += 32) {
+                const bool mine = i + lane < cnt && s_lr[i + lane] == r;
+                const unsigned bal = __ballot_sync(0xffffffffu, mine);
+                if (mine)
+                    s_sorted[at + __popc(bal & lt)] = s_raw[i + lane];
+                at += __popc(bal);
+            }
+        }
+        __syncwarp(); // a warp reads only the rows that it sorted
+    };
+
+    if (total <= chunk) {
+        stage(0, static_cast<int>(total));
+        for (int r = warp; r < nrows; r += nwarps) {
+            const Entry *s_row = s_sorted + s_start[r];
+            const int cnt = s_start[r + 1] - s_start[r];
+            float *c_row = C + (r0 + r) * n;
+            int it = 0;
+            for (; cnt < kPairRows && it + 1 < col_iters; it += 2) {
+                const LaneCols<V, W> aa(j0 + it * (32 * V), lane, n), ab(j0 + (it + 1) * (32 * V), lane, n);
+                if (!aa.on)
+                    break;
+                float a2[V], b2[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+                    a2[v] = b2[v] = 0.0f;
+                if (ab.on)
+                    row_chain_pair<V, W, 4>(s_row, cnt, B + aa.j, B + ab.j, n, a2, b2);
+                else
+                    row_chain<V, W, 4, false>(s_row, cnt, B + aa.j, n, a2);
+                Vec<V, W>::store(c_row + aa.j, a2, aa.j, aa.from);
+                if (ab.on)
+                    Vec<V, W>::store(c_row + ab.j, b2, ab.j, ab.from);
+            }
+            for (; it < col_iters; ++it) {
+                const LaneCols<V, W> at(j0 + it * (32 * V), lane, n);
+                if (!at.on)
+                    break;
+                float acc[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+                    acc[v] = 0.0f;
+                row_chain<V, W, 8, false>(s_row, cnt, B + at.j, n, acc);
+                Vec<V, W>::store(c_row + at.j, acc, at.j, at.from);
+            }
+        }
+        return;
+    }
+    // more entries than one chunk: a tile's sums live in C between chunks
+    for (int64_t first = 0; first < total; first += chunk) {
+        stage(first, static_cast<int>(total - first < chunk ? total - first : chunk));
+        for (int r = warp; r < nrows; r += nwarps) {
+            const Entry *s_row = s_sorted + s_start[r];
+            const int cnt = s_start[r + 1] - s_start[r];
+            for (int it = 0; it < col_iters; ++it) {
+                const LaneCols<V, W> at(j0 + it * (32 * V), lane, n);
+                if (!at.on)
+                    break;
+                float acc[V];
+                view_resume<V, W>(C + (r0 + r) * n + at.j, at, first > 0, acc);
+                row_chain<V, W, 8, false>(s_row, cnt, B + at.j, n, acc);
+                Vec<V, W>::store(C + (r0 + r) * n + at.j, acc, at.j, at.from);
+            }
+        }
     }
 }
 
@@ -732,13 +847,39 @@ cudaError_t launch_spdm_view(const gcoo_view &a, const float *B, int64_t n, floa
 {
     if (a.n_group <= 0 || n <= 0)
         return cudaSuccess;
-    const int64_t ny = (n + kViewThreads - 1) / kViewThreads;
-    if (ny > 65535)
+    if ((n + 127) / 128 > 65535) // the widest B this entry point takes
         return cudaErrorInvalidConfiguration;
-    dim3 grid(static_cast<unsigned>(a.n_group), static_cast<unsigned>(ny));
-    const size_t smem = sizeof(float) * static_cast<size_t>(a.rows_per_group) * kViewThreads;
-    spdm_view_kernel<<<grid, kViewThreads, smem, st>>>(a.vals, a.rows, a.cols, a.group_index, a.nnz_per_group,
-                                                       a.m, a.rows_per_group, B, n, C);
+    const int cpg = a.rows_per_group;
+    const int warps = cpg < kViewMaxWarps ? cpg : kViewMaxWarps;
+    gcoo_params p{};
+    p.rows_per_group = cpg;
+    p.warps = p.col_warps = 1;
+    LaunchShape s = pick_shape(p, a.m, n, a.nnz, 0, reinterpret_cast<uintptr_t>(B), reinterpret_cast<uintptr_t>(C));
+    // entries staged at once: a power of two above twice the mean group
+    const int64_t mean = a.nnz / a.n_group;
+    int chunk = 256;
+    while (chunk < kChunk && chunk < 2 * mean + 64)
+        chunk *= 2;
+    // as the row walk: about 768 columns per CTA, but four waves of CTAs
+    const int64_t tile = 32 * s.vec, tiles = (n + tile - 1) / tile;
+    const int64_t resident = static_cast<int64_t>(device_sms()) * kRowCtas * 4 / warps;
+    int64_t ci = a.n_group * tiles / (4 * resident);
+    ci = ci > 768 / tile ? 768 / tile : ci;
+    ci = ci < 1 ? 1 : ci;
+    while ((tiles + ci - 1) / ci > 65535)
+        ci *= 2;
+    const dim3 grid(static_cast<unsigned>(a.n_group), static_cast<unsigned>((tiles + ci - 1) / ci));
+    const size_t smem = static_cast<size_t>(chunk) * (2 * sizeof(Entry) + 1);
+#define GCOO_VIEW(V, W)                                                                                             \
+    spdm_view_kernel<V, W><<<grid, warps * 32, smem, st>>>(a.vals, a.rows, a.cols, a.group_index, a.nnz_per_group, \
+                                                           a.m, cpg, chunk, static_cast<int32_t>(ci), B, n, C)
+    if (s.vec == 4 && s.width == 4) GCOO_VIEW(4, 4);
+    else if (s.vec == 4 && s.width == 2) GCOO_VIEW(4, 2);
+    else if (s.vec == 4) GCOO_VIEW(4, 1);
+    else if (s.vec == 2 && s.width == 2) GCOO_VIEW(2, 2);
+    else if (s.vec == 2) GCOO_VIEW(2, 1);
+    else GCOO_VIEW(1, 1);
+#undef GCOO_VIEW
     count_launches(1);
     return cudaGetLastError();
 }
