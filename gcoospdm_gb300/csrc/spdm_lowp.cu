@@ -1,8 +1,8 @@
 // spdm_lowp.cu -- the reduced-precision forms of the multiply on the FMA
 // pipes (the tensor-core engine for block-structured matrices is in
-// spdm_tc.cu). Same CTA/warp mapping as the FP32 kernel (one CTA per GCOO
-// group and column tile, the group's entries staged to shared memory with
-// cp.async.bulk, one warp per row), with B read in a narrower format:
+// spdm_tc.cu). Same CTA/warp mapping as the FP32 row walk (one warp per row,
+// the CTA's entries staged to shared memory with cp.async.bulk and used for
+// several column tiles), with B read in a narrower format:
 //   BF16        B as bf16 (8 columns per 128-bit load), A values rounded to
 //               bf16, FP32 accumulation (the mixed-precision bf16 FMA of
 //               sm_100+: no widening of the B values);
@@ -10,8 +10,9 @@
 //               ah*Bl + al*Bh (three products, FP32 accumulation) -- FP32-level
 //               accuracy from bf16 operands;
 //   FP8_B       B as FP8 E4M3 scaled per column (s_j = the smallest power of
-//               two with max_c |B[c][j]| / s_j <= 448), 16 columns per 128-bit
-//               load, A kept FP32; the scale is applied once to the
+//               two with max_c |B[c][j]| / s_j <= 448), 16 columns per
+//               128-bit load (narrow B: each value as the BF16 that equals
+//               it), A kept FP32; the scale is applied once to the
 //               accumulated column.
 // B is converted into the handle's workspace by a pre-pass kernel per call.
 #include <cuda_bf16.h>
@@ -22,9 +23,9 @@
 namespace gcoo {
 
 struct LowpWork {
-    DevBuf<uint16_t> bf;     // k*n bf16
+    DevBuf<uint16_t> bf;     // k*n bf16 (FP8: E4M3 values as bf16)
     DevBuf<uint32_t> split;  // k*n (hi | lo << 16) bf16 pairs
-    DevBuf<uint8_t> f8;      // k*n e4m3
+    DevBuf<uint8_t> f8;      // k*n e4m3 (the group walk's)
     DevBuf<float> scale;     // n column scales
     DevBuf<unsigned> amax;   // n column absmax (float bits)
 };
@@ -34,19 +35,26 @@ void destroy_lowp_work(LowpWork *w) { delete w; }
 namespace {
 
 constexpr int kChunk = 2048;
-constexpr int kSmemBytes = 128 + (kChunk + 2) * static_cast<int>(sizeof(Entry));
+// Four-warp CTAs per SM (64 registers a thread) and entries per batch of the
+// row walk. 4096^2 at 2 %, n = 4096 (us; BF16 / split / FP8): batches of eight
+// 152 / 398 / 192, of four 159 / 418 / 196, ten CTAs 154 / 406 / 200; before,
+// two warps per row, a staging per tile, 16 KB of shared memory and the tail
+// entry by entry: 220 / 443 / 222.
+constexpr int kLowpCtas = 8, kLowpU = 8;
+constexpr int kLowpCols = 1024; // columns per staging at most (512: 1-2 % slower)
 
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-enum Form { kBF16 = 1, kSplit = 2, kFP8 = 3 };
+enum Form { kBF16 = 1, kSplit = 2, kFP8 = 3, kFP8Wide = 4 };
 
 // Columns per lane for each form (one 128-bit load per entry).
 template <int F> struct FormTraits;
 template <> struct FormTraits<kBF16> { static constexpr int V = 8; using T = uint16_t; };
 template <> struct FormTraits<kSplit> { static constexpr int V = 4; using T = uint32_t; };
 template <> struct FormTraits<kFP8> { static constexpr int V = 16; using T = uint8_t; };
+template <> struct FormTraits<kFP8Wide> { static constexpr int V = 8; using T = uint16_t; };
 
 // acc + a * b with bf16 a and b, one rounding (the mixed-precision FMA of
 // sm_100+): the same result as fmaf on the widened values, since a product of
@@ -58,157 +66,231 @@ __device__ __forceinline__ float fma_bf16(uint16_t a, uint16_t b, float c)
     return d;
 }
 
-template <int F>
-__device__ __forceinline__ void fma_entry(float a, const uint4 &w, float (&acc)[FormTraits<F>::V])
+// Two FP32 sums, each its own fma (one rounding each).
+__device__ __forceinline__ void fma_pair(uint64_t &c, uint64_t a, float b0, float b1)
 {
-    if constexpr (F == kBF16) {
-        // a is already a bf16 value: its top 16 bits are exact
-        const uint16_t ab = static_cast<uint16_t>(__float_as_uint(a) >> 16);
-        const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            acc[2 * i] = fma_bf16(ab, static_cast<uint16_t>(x[i] & 0xffffu), acc[2 * i]);
-            acc[2 * i + 1] = fma_bf16(ab, static_cast<uint16_t>(x[i] >> 16), acc[2 * i + 1]);
-        }
-    } else if constexpr (F == kFP8) {
-        const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(x[i] & 0xffffu), __NV_E4M3);
-            const __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(x[i] >> 16), __NV_E4M3);
-            const float2 f01 = __half22float2(*reinterpret_cast<const __half2 *>(&h01));
-            const float2 f23 = __half22float2(*reinterpret_cast<const __half2 *>(&h23));
-            acc[4 * i + 0] = fmaf(a, f01.x, acc[4 * i + 0]);
-            acc[4 * i + 1] = fmaf(a, f01.y, acc[4 * i + 1]);
-            acc[4 * i + 2] = fmaf(a, f23.x, acc[4 * i + 2]);
-            acc[4 * i + 3] = fmaf(a, f23.y, acc[4 * i + 3]);
-        }
-    }
+    uint64_t b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(b0), "f"(b1));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
+__device__ __forceinline__ uint64_t dup_f32(float a)
+{
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a));
+    return d;
+}
+
+__device__ __forceinline__ void split_f32x2(uint64_t x, float &lo, float &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x));
+}
+
+// A lane's V sums of one row tile, as the form multiplies them. BF16: the
+// mixed-precision FMA; the others in pairs (packed FMAs: half the issue
+// slots, which the widening of B's halves needs).
+template <int F>
+struct Sums {
+    static constexpr int V = FormTraits<F>::V;
+    uint64_t s[V / 2];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int v = 0; v < V / 2; ++v)
+            s[v] = 0ull;
+    }
+    __device__ __forceinline__ float get(int v) const
+    {
+        float lo, hi;
+        split_f32x2(s[v / 2], lo, hi);
+        return v & 1 ? hi : lo;
+    }
+    __device__ __forceinline__ void add(float val, const uint4 &w)
+    {
+        const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+        if constexpr (F == kFP8) {
+            const uint64_t a = dup_f32(val);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(x[i] & 0xffffu), __NV_E4M3);
+                const __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(x[i] >> 16), __NV_E4M3);
+                const float2 f01 = __half22float2(*reinterpret_cast<const __half2 *>(&h01));
+                const float2 f23 = __half22float2(*reinterpret_cast<const __half2 *>(&h23));
+                fma_pair(s[(2 * i) % (V / 2)], a, f01.x, f01.y);
+                fma_pair(s[(2 * i + 1) % (V / 2)], a, f23.x, f23.y);
+            }
+        } else if constexpr (F == kFP8Wide) {
+            const uint64_t a = dup_f32(val);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                fma_pair(s[i], a, bf_lo(x[i]), bf_hi(x[i]));
+        } else {
+            const float ah = round_bf16(val);
+            const uint64_t hi = dup_f32(ah), lo = dup_f32(round_bf16(val - ah));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                fma_pair(s[i], hi, bf_lo(x[2 * i]), bf_lo(x[2 * i + 1]));
+                fma_pair(s[i], hi, bf_hi(x[2 * i]), bf_hi(x[2 * i + 1]));
+                fma_pair(s[i], lo, bf_lo(x[2 * i]), bf_lo(x[2 * i + 1]));
+            }
+        }
+    }
+};
+
+template <>
+struct Sums<kBF16> {
+    static constexpr int V = 8;
+    float s[V];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            s[v] = 0.0f;
+    }
+    __device__ __forceinline__ float get(int v) const { return s[v]; }
+    __device__ __forceinline__ void add(float val, const uint4 &w)
+    {
+        const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+        const uint16_t ab = __bfloat16_as_ushort(__float2bfloat16_rn(val));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            s[2 * i] = fma_bf16(ab, static_cast<uint16_t>(x[i] & 0xffffu), s[2 * i]);
+            s[2 * i + 1] = fma_bf16(ab, static_cast<uint16_t>(x[i] >> 16), s[2 * i + 1]);
+        }
+    }
+};
+
 template <int F, int U>
-__device__ __forceinline__ void row_chain_lowp(const Entry *__restrict__ s, int cnt, const typename FormTraits<F>::T *__restrict__ Bj,
-                                               int64_t n, float (&acc)[FormTraits<F>::V])
+__device__ __forceinline__ void lowp_batch(const Entry *__restrict__ s, const typename FormTraits<F>::T *__restrict__ Bj,
+                                           int64_t n, Sums<F> &sum)
+{
+    Entry e[U];
+    uint4 w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        e[u] = s[u];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        w[u] = __ldg(reinterpret_cast<const uint4 *>(Bj + static_cast<int64_t>(e[u].col) * n));
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        sum.add(e[u].val, w[u]);
+}
+
+// One row's entries in order, U B loads in flight, the tail in halves too.
+template <int F, int U>
+__device__ __forceinline__ void row_chain_lowp(const Entry *__restrict__ s, int cnt,
+                                               const typename FormTraits<F>::T *__restrict__ Bj, int64_t n, Sums<F> &sum)
 {
     int i = 0;
 #pragma unroll 1
-    for (; i + U <= cnt; i += U) {
-        Entry e[U];
-        uint4 w[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            e[u] = s[i + u];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            w[u] = __ldg(reinterpret_cast<const uint4 *>(Bj + static_cast<int64_t>(e[u].col) * n));
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if constexpr (F == kSplit) {
-                const float ah = round_bf16(e[u].val);
-                const float al = round_bf16(e[u].val - ah);
-                const uint32_t x[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const float bh = bf_lo(x[v]), bl = bf_hi(x[v]);
-                    acc[v] = fmaf(al, bh, fmaf(ah, bl, fmaf(ah, bh, acc[v])));
-                }
-            } else {
-                fma_entry<F>(F == kBF16 ? round_bf16(e[u].val) : e[u].val, w[u], acc);
-            }
-        }
+    for (; i + U <= cnt; i += U)
+        lowp_batch<F, U>(s + i, Bj, n, sum);
+    if (U == 8 && i + 4 <= cnt) {
+        lowp_batch<F, 4>(s + i, Bj, n, sum);
+        i += 4;
     }
-#pragma unroll 1
-    for (; i < cnt; ++i) {
-        const Entry e = s[i];
-        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(Bj + static_cast<int64_t>(e.col) * n));
-        if constexpr (F == kSplit) {
-            const float ah = round_bf16(e.val);
-            const float al = round_bf16(e.val - ah);
-            const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+    if (i + 2 <= cnt) {
+        lowp_batch<F, 2>(s + i, Bj, n, sum);
+        i += 2;
+    }
+    if (i < cnt)
+        lowp_batch<F, 1>(s + i, Bj, n, sum);
+}
+
+template <int F>
+__device__ __forceinline__ void lowp_store(float *out, const float *__restrict__ scale, const Sums<F> &sum)
+{
+    constexpr int V = FormTraits<F>::V;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const float bh = bf_lo(x[v]), bl = bf_hi(x[v]);
-                acc[v] = fmaf(al, bh, fmaf(ah, bl, fmaf(ah, bh, acc[v])));
-            }
-        } else {
-            fma_entry<F>(F == kBF16 ? round_bf16(e.val) : e.val, w, acc);
+    for (int v = 0; v < V; v += 4) {
+        float4 o = make_float4(sum.get(v), sum.get(v + 1), sum.get(v + 2), sum.get(v + 3));
+        if constexpr (F == kFP8 || F == kFP8Wide) {
+            const float4 s = __ldg(reinterpret_cast<const float4 *>(scale + v));
+            o.x *= s.x; o.y *= s.y; o.z *= s.z; o.w *= s.w;
         }
+        *reinterpret_cast<float4 *>(out + v) = o;
     }
 }
 
-// One CTA per (group, column tile); warps = rows_per_group * col_warps.
-// n must be a multiple of the form's V and B/C suitably aligned (host checks).
+// One CTA per (`cpg` rows, col_iters column tiles), one warp per row: the
+// CTA's entries are staged once and each warp walks its row over all tiles
+// from there, as in the FP32 row walk; entries beyond the staged chunk (its
+// size is the launch's) are staged piecewise for each tile in turn. n must be
+// a multiple of the form's V and B / C 16-byte aligned (host checks).
 template <int F>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(128, kLowpCtas)
 spdm_lowp_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m, int32_t cpg,
                  const typename FormTraits<F>::T *__restrict__ B, const float *__restrict__ col_scale, int64_t n,
-                 float *__restrict__ C, int32_t col_warps, uint32_t *__restrict__ status)
+                 float *__restrict__ C, int32_t col_iters, int32_t chunk, uint32_t *__restrict__ status)
 {
     constexpr int V = FormTraits<F>::V;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
     Entry *s_nz = reinterpret_cast<Entry *>(smem + 128);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int slot = warp / col_warps, sub = warp - slot * col_warps;
     const int64_t r0 = static_cast<int64_t>(blockIdx.x) * cpg;
     const int64_t r_end = r0 + cpg < m ? r0 + cpg : m;
-    const int64_t row = r0 + slot;
-    const bool has_row = slot < cpg && row < r_end;
-    const int64_t j = (static_cast<int64_t>(blockIdx.y) * col_warps + sub) * (32 * V) + static_cast<int64_t>(lane) * V;
-    const bool has_col = j < n;
+    const int64_t row = r0 + warp;
+    const bool has_row = row < r_end;
+    const int64_t j0 = static_cast<int64_t>(blockIdx.y) * col_iters * (32 * V) + static_cast<int64_t>(lane) * V;
     const int64_t gs = row_ptr[r0], ge = row_ptr[r_end];
-    int64_t rs = 0, re = 0;
-    if (has_row) {
-        rs = row_ptr[row];
-        re = row_ptr[row + 1];
-    }
+    const int64_t rs = has_row ? row_ptr[row] : 0, re = has_row ? row_ptr[row + 1] : 0;
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
     }
     __syncthreads();
-    float acc[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v)
-        acc[v] = 0.0f;
-    const typename FormTraits<F>::T *Bj = B + j;
-    const int64_t nchunks = (ge - gs + kChunk - 1) / kChunk;
+    const int64_t nchunks = (ge - gs + chunk - 1) / chunk;
+    const bool once = nchunks <= 1;
     bool ok = true;
-    for (int64_t ch = 0; ch < nchunks && ok; ++ch) {
-        const int64_t cs = gs + ch * kChunk;
-        const int64_t ce = cs + kChunk < ge ? cs + kChunk : ge;
-        const int64_t a0 = cs & ~static_cast<int64_t>(1);
-        const int64_t a1 = (ce + 1) & ~static_cast<int64_t>(1);
-        if (threadIdx.x == 0) {
-            fence_proxy_async();
-            const uint32_t bytes = static_cast<uint32_t>((a1 - a0) * static_cast<int64_t>(sizeof(Entry)));
-            mbar_arrive_expect_tx(bar, bytes);
-            bulk_g2s(s_nz, packed + a0, bytes, bar);
-        }
-        const bool waited = mbar_wait(bar, static_cast<uint32_t>(ch & 1));
-        ok = __syncthreads_and(waited) != 0;
-        if (!ok) {
-            if (threadIdx.x == 0)
-                atomicOr(status, kStatusWaitTimeout);
-            mbar_wait(bar, static_cast<uint32_t>(ch & 1));
-            break;
-        }
-        const int64_t lo = rs > cs ? rs : cs, hi = re < ce ? re : ce;
-        if (has_col && lo < hi)
-            row_chain_lowp<F, 4>(s_nz + (lo - a0), static_cast<int>(hi - lo), Bj, n, acc);
-        __syncthreads();
-    }
-    if (has_row && has_col && ok) {
-        float *out = C + row * n + j;
-#pragma unroll
-        for (int v = 0; v < V; v += 4) {
-            float4 o = make_float4(acc[v], acc[v + 1], acc[v + 2], acc[v + 3]);
-            if constexpr (F == kFP8) {
-                const float4 s = *reinterpret_cast<const float4 *>(col_scale + j + v);
-                o.x *= s.x; o.y *= s.y; o.z *= s.z; o.w *= s.w;
+    uint32_t phase = 0;
+    for (int it = 0; it < (once ? 1 : col_iters) && ok; ++it) {
+        const int64_t j = j0 + it * (32 * V);
+        Sums<F> sum;
+        sum.clear();
+        for (int64_t ch = 0; ch < nchunks; ++ch, ++phase) {
+            const int64_t cs = gs + ch * chunk;
+            const int64_t ce = cs + chunk < ge ? cs + chunk : ge;
+            const int64_t a0 = cs & ~static_cast<int64_t>(1);
+            const int64_t a1 = (ce + 1) & ~static_cast<int64_t>(1);
+            if (threadIdx.x == 0) {
+                fence_proxy_async();
+                const uint32_t bytes = static_cast<uint32_t>((a1 - a0) * static_cast<int64_t>(sizeof(Entry)));
+                mbar_arrive_expect_tx(bar, bytes);
+                bulk_g2s(s_nz, packed + a0, bytes, bar);
             }
-            *reinterpret_cast<float4 *>(out + v) = o;
+            const bool waited = mbar_wait(bar, phase & 1);
+            ok = __syncthreads_and(waited) != 0;
+            if (!ok) {
+                if (threadIdx.x == 0)
+                    atomicOr(status, kStatusWaitTimeout);
+                mbar_wait(bar, phase & 1);
+                break;
+            }
+            if (once)
+                break; // staged for good: every tile below
+            const int64_t lo = rs > cs ? rs : cs, hi = re < ce ? re : ce;
+            if (j < n && lo < hi)
+                row_chain_lowp<F, kLowpU>(s_nz + (lo - a0), static_cast<int>(hi - lo), B + j, n, sum);
+            __syncthreads();
         }
+        if (!once && has_row && j < n && ok)
+            lowp_store<F>(C + row * n + j, col_scale + j, sum);
+    }
+    if (!once || !has_row || !ok)
+        return;
+    const Entry *s_row = s_nz + (rs - (gs & ~static_cast<int64_t>(1)));
+    const int cnt = static_cast<int>(re - rs);
+#pragma unroll 1
+    for (int it = 0; it < col_iters; ++it) {
+        const int64_t j = j0 + it * (32 * V);
+        if (j >= n)
+            break;
+        Sums<F> sum;
+        sum.clear();
+        row_chain_lowp<F, kLowpU>(s_row, cnt, B + j, n, sum);
+        lowp_store<F>(C + row * n + j, col_scale + j, sum);
     }
 }
 
@@ -242,60 +324,114 @@ __global__ void prep_split_kernel(const float4 *__restrict__ B, uint4 *__restric
     }
 }
 
-// Column absmax: each thread owns 4 columns and a slice of rows.
-__global__ void colmax_kernel(const float *__restrict__ B, int64_t k, int64_t n, unsigned *__restrict__ amax,
-                              int rows_per_cta)
+// FP8 passes over B: a CTA takes 128 columns x 128 rows, a warp 16 of the
+// rows, a lane 4 of the columns; the 16 rows' loads are in flight together.
+constexpr int kStripCols = 128, kStripRows = 128, kWarpRows = 16;
+
+// Column absmax: one atomic per column and CTA.
+__global__ void __launch_bounds__(256)
+colmax_kernel(const float *__restrict__ B, int64_t k, int64_t n, unsigned *__restrict__ amax)
 {
-    const int64_t j = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
-    if (j >= n)
-        return;
-    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * rows_per_cta;
-    const int64_t c1 = c0 + rows_per_cta < k ? c0 + rows_per_cta : k;
-    float m0 = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
-#pragma unroll 8
-    for (int64_t c = c0; c < c1; ++c) {
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(B + c * n + j));
-        m0 = fmaxf(m0, fabsf(v.x)); m1 = fmaxf(m1, fabsf(v.y));
-        m2 = fmaxf(m2, fabsf(v.z)); m3 = fmaxf(m3, fabsf(v.w));
+    __shared__ float s_max[kStripRows / kWarpRows][kStripCols];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t j = static_cast<int64_t>(blockIdx.x) * kStripCols + lane * 4;
+    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * kStripRows + warp * kWarpRows;
+    float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[kWarpRows];
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i)
+        v[i] = j < n && c0 + i < k ? __ldg(reinterpret_cast<const float4 *>(B + (c0 + i) * n + j)) : mx;
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i) {
+        mx.x = fmaxf(mx.x, fabsf(v[i].x)); mx.y = fmaxf(mx.y, fabsf(v[i].y));
+        mx.z = fmaxf(mx.z, fabsf(v[i].z)); mx.w = fmaxf(mx.w, fabsf(v[i].w));
     }
-    atomicMax(amax + j, __float_as_uint(m0));
-    atomicMax(amax + j + 1, __float_as_uint(m1));
-    atomicMax(amax + j + 2, __float_as_uint(m2));
-    atomicMax(amax + j + 3, __float_as_uint(m3));
+    *reinterpret_cast<float4 *>(&s_max[warp][lane * 4]) = mx;
+    __syncthreads();
+    const int t = threadIdx.x;
+    const int64_t jt = static_cast<int64_t>(blockIdx.x) * kStripCols + t;
+    if (t < kStripCols && jt < n) {
+        float x = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kStripRows / kWarpRows; ++w)
+            x = fmaxf(x, s_max[w][t]);
+        atomicMax(amax + jt, __float_as_uint(x));
+    }
 }
 
 // Per-column scale: the smallest power of two s with absmax / s <= 448 (the
 // largest E4M3 value). A power of two divides exactly, so both engines see
 // the same E4M3 values, and the tensor engine can fold s into its BF16 tiles
 // without a rounding (an E4M3 value times a power of two is a BF16 value).
+__device__ __forceinline__ float fp8_scale(unsigned amax_bits)
+{
+    const float a = __uint_as_float(amax_bits);
+    float s = 1.0f;
+    if (a > 0.0f && a < INFINITY) {
+        int e = 0;
+        const float mant = frexpf(a / 448.0f, &e); // a / 448 = mant * 2^e, mant in [0.5, 1)
+        s = ldexpf(1.0f, mant == 0.5f ? e - 1 : e);
+    }
+    return s;
+}
+
 __global__ void scale_kernel(const unsigned *__restrict__ amax, float *__restrict__ scale, int64_t n)
 {
     const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (j < n) {
-        const float a = __uint_as_float(amax[j]);
-        float s = 1.0f;
-        if (a > 0.0f && a < INFINITY) {
-            int e = 0;
-            const float mant = frexpf(a / 448.0f, &e); // a / 448 = mant * 2^e, mant in [0.5, 1)
-            s = ldexpf(1.0f, mant == 0.5f ? e - 1 : e);
-        }
-        scale[j] = s;
-    }
+    if (j < n)
+        scale[j] = fp8_scale(amax[j]);
 }
 
-__global__ void prep_fp8_kernel(const float4 *__restrict__ B, const float *__restrict__ scale, uint32_t *__restrict__ out,
-                                int64_t n4, int64_t n)
+// B in units of its columns' scales as E4M3; the scales, computed where they
+// are used, are written once for the multiply. WIDE: each E4M3 value as the
+// BF16 that equals it.
+template <bool WIDE>
+__global__ void __launch_bounds__(256)
+prep_fp8_kernel(const float *__restrict__ B, const unsigned *__restrict__ amax, float *__restrict__ scale,
+                void *__restrict__ out, int64_t k, int64_t n)
 {
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const float4 v = __ldcs(B + i);
-        const int64_t j = (i * 4) % n;
-        const float x[4] = {v.x / scale[j], v.y / scale[j + 1], v.z / scale[j + 2], v.w / scale[j + 3]};
-        uint32_t w = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t j = static_cast<int64_t>(blockIdx.x) * kStripCols + lane * 4;
+    const int64_t c0 = static_cast<int64_t>(blockIdx.y) * kStripRows + warp * kWarpRows;
+    if (j >= n)
+        return;
+    float4 v[kWarpRows];
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i)
+        v[i] = c0 + i < k ? __ldcs(reinterpret_cast<const float4 *>(B + (c0 + i) * n + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint4 am = *reinterpret_cast<const uint4 *>(amax + j);
+    const float s[4] = {fp8_scale(am.x), fp8_scale(am.y), fp8_scale(am.z), fp8_scale(am.w)};
+    if (blockIdx.y == 0 && warp == 0)
+        *reinterpret_cast<float4 *>(scale + j) = make_float4(s[0], s[1], s[2], s[3]);
+    // a power of two in the normal range has an exact reciprocal, so x * inv
+    // is x / s exactly; otherwise divide
+    bool by_inv = true;
+    float inv[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        by_inv = by_inv && s[q] >= 1.17549435e-38f && s[q] <= 8.50705917e37f;
+        inv[q] = 1.0f / s[q];
+    }
+#pragma unroll
+    for (int i = 0; i < kWarpRows; ++i) {
+        const float x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+        __nv_fp8_storage_t f[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            w |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(x[q], __NV_SATFINITE, __NV_E4M3)) << (8 * q);
-        out[i] = w;
+            f[q] = __nv_cvt_float_to_fp8(by_inv ? x[q] * inv[q] : x[q] / s[q], __NV_SATFINITE, __NV_E4M3);
+        if (c0 + i >= k)
+            break;
+        if constexpr (WIDE) {
+            uint32_t w[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) // an E4M3 value is an FP16 value and a BF16 value
+                w[q] = __float_as_uint(__half2float(__half(__nv_cvt_fp8_to_halfraw(f[q], __NV_E4M3)))) >> 16;
+            *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(out) + (c0 + i) * n + j) =
+                make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+        } else {
+            *reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(out) + (c0 + i) * n + j) =
+                f[0] | (static_cast<uint32_t>(f[1]) << 8) | (static_cast<uint32_t>(f[2]) << 16) | (static_cast<uint32_t>(f[3]) << 24);
+        }
     }
 }
 
@@ -309,24 +445,43 @@ unsigned grid_for(int64_t items, int threads)
 
 } // namespace
 
-cudaError_t launch_fp8_scales(const float *B, int64_t k, int64_t n, unsigned *amax, float *scale, cudaStream_t st)
+static dim3 strip_grid(int64_t k, int64_t n)
 {
-    cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(unsigned) * static_cast<size_t>(n), st);
+    return dim3(static_cast<unsigned>((n + kStripCols - 1) / kStripCols),
+                static_cast<unsigned>((k + kStripRows - 1) / kStripRows));
+}
+
+static cudaError_t launch_colmax(const float *B, int64_t k, int64_t n, unsigned *amax, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(unsigned) * static_cast<size_t>(n), st);
     if (e != cudaSuccess)
         return e;
-    // 32 rows per CTA: k / 32 CTAs per column strip, enough loads in flight
-    // to stream B (256 rows per CTA left the pass latency-bound: 64 CTAs at
-    // B 8192 x 1024)
-    const int rows_per_cta = 32;
-    dim3 g(static_cast<unsigned>((n / 4 + 127) / 128), static_cast<unsigned>((k + rows_per_cta - 1) / rows_per_cta));
-    colmax_kernel<<<g, 128, 0, st>>>(B, k, n, amax, rows_per_cta);
+    colmax_kernel<<<strip_grid(k, n), 256, 0, st>>>(B, k, n, amax);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fp8_scales(const float *B, int64_t k, int64_t n, unsigned *amax, float *scale, cudaStream_t st)
+{
+    const cudaError_t e = launch_colmax(B, k, n, amax, st);
+    if (e != cudaSuccess)
+        return e;
     scale_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(amax, scale, n);
-    count_launches(2);
+    count_launches(1);
     return cudaGetLastError();
 }
 
 // Width constraint of each form on the FMA engine.
 int lowp_vec(gcoo_precision prec) { return prec == GCOO_PREC_BF16 ? 8 : prec == GCOO_PREC_SPLIT_BF16 ? 4 : 16; }
+
+// FP8-B: B's E4M3 values as one byte or as the BF16 that equals each. Bytes:
+// half the gather, but two and a half instructions a value, and a warp's 16-byte
+// loads span 512 columns; BF16: one and a half instructions. Measured (us;
+// bytes / BF16): 8192^2 at 1 %, n = 2048 190 / 200; 4096^2 at 2 %, n = 4096
+// 192 / 198; 4001 x 3999 at 5 %, n = 1024 111 / 111; 2048^2 at 0.5 %, n = 512
+// 22 / 20; 8192 x 1200 at 3 %, n = 128 36 / 28. The group walk reads bytes.
+constexpr int64_t kFp8WideCols = 1024;
+static bool fp8_wide(const gcoo_handle *h, int64_t n) { return n <= kFp8WideCols && !group_order_chosen(h); }
 
 gcoo_status lowp_prepare(gcoo_handle *h, int64_t n, gcoo_precision prec)
 {
@@ -341,7 +496,10 @@ gcoo_status lowp_prepare(gcoo_handle *h, int64_t n, gcoo_precision prec)
     else if (prec == GCOO_PREC_SPLIT_BF16)
         ok = h->lowp->split.ensure(kn);
     else
-        ok = h->lowp->f8.ensure(kn) && h->lowp->scale.ensure(n) && h->lowp->amax.ensure(n);
+        // a width prepared once serves every smaller one, in either format
+        ok = (group_order_chosen(h) ||
+              h->lowp->bf.ensure(static_cast<size_t>(h->k) * static_cast<size_t>(n < kFp8WideCols ? n : kFp8WideCols))) &&
+             (fp8_wide(h, n) || h->lowp->f8.ensure(kn)) && h->lowp->scale.ensure(n) && h->lowp->amax.ensure(n);
     return ok ? GCOO_SUCCESS : fail(GCOO_ERROR_ALLOC, "device allocation of the form workspace failed");
 }
 
@@ -359,9 +517,11 @@ gcoo_status lowp_convert_b(gcoo_handle *h, const float *dB, int64_t n, gcoo_prec
                                                              reinterpret_cast<uint4 *>(w->split.ptr), n4);
         count_launches(1);
     } else {
-        GCOO_CUDA(launch_fp8_scales(dB, h->k, n, w->amax.ptr, w->scale.ptr, st));
-        prep_fp8_kernel<<<grid_for(n4, 256), 256, 0, st>>>(reinterpret_cast<const float4 *>(dB), w->scale.ptr,
-                                                           reinterpret_cast<uint32_t *>(w->f8.ptr), n4, n);
+        GCOO_CUDA(launch_colmax(dB, h->k, n, w->amax.ptr, st));
+        if (!fp8_wide(h, n))
+            prep_fp8_kernel<false><<<strip_grid(h->k, n), 256, 0, st>>>(dB, w->amax.ptr, w->scale.ptr, w->f8.ptr, h->k, n);
+        else
+            prep_fp8_kernel<true><<<strip_grid(h->k, n), 256, 0, st>>>(dB, w->amax.ptr, w->scale.ptr, w->bf.ptr, h->k, n);
         count_launches(1);
     }
     GCOO_LAUNCH("B conversion kernel");
@@ -370,16 +530,9 @@ gcoo_status lowp_convert_b(gcoo_handle *h, const float *dB, int64_t n, gcoo_prec
 
 gcoo_status lowp_spdm(gcoo_handle *h, int64_t n, float *dC, gcoo_precision prec, cudaStream_t st)
 {
-    const int V = lowp_vec(prec);
-    const int cpg = h->p.rows_per_group;
-    int cw = 8 / cpg;
-    if (cw < 1)
-        cw = 1;
-    while (cw > 1 && static_cast<int64_t>(cw / 2) * 32 * V >= n)
-        cw /= 2;
-    if (cw * cpg > 16)
-        cw = 16 / cpg > 0 ? 16 / cpg : 1;
-    if (cpg > 16)
+    const bool wide = prec == GCOO_PREC_FP8_B && fp8_wide(h, n);
+    const int V = wide ? 8 : lowp_vec(prec); // columns per lane
+    if (h->p.rows_per_group > 16)
         return fail(GCOO_ERROR_UNSUPPORTED, "reduced-precision forms on the FMA engine support rows_per_group <= 16");
     LowpWork *w = h->lowp;
     if (prec != GCOO_PREC_SPLIT_BF16 && n % 8 == 0 && group_order_chosen(h)) {
@@ -392,19 +545,40 @@ gcoo_status lowp_spdm(gcoo_handle *h, int64_t n, float *dC, gcoo_precision prec,
             return cuda_fail(e, "spdm_group_kernel launch (reduced precision)");
         return GCOO_SUCCESS;
     }
-    const int64_t tile = static_cast<int64_t>(cw) * 32 * V;
-    const int64_t ny = (n + tile - 1) / tile;
-    dim3 grid(static_cast<unsigned>(h->ng), static_cast<unsigned>(ny));
-    const int threads = cw * cpg * 32;
+    // one warp per row, up to four rows per CTA (any number gives the same
+    // chains), fewer where that makes their entries fit one staging
+    int rows = h->p.rows_per_group < 4 ? h->p.rows_per_group : 4;
+    while (rows > 1 && h->max_row_nnz * rows + 2 > kChunk)
+        rows /= 2;
+    const int64_t most = h->max_row_nnz * rows + 2;
+    const int chunk = static_cast<int>(most < kChunk ? (most < 64 ? 64 : most) : kChunk);
+    // as the FP32 row walk: several tiles per staging, at least four waves of CTAs
+    const int64_t tile = 32 * V, tiles = (n + tile - 1) / tile, groups = (h->m + rows - 1) / rows;
+    const int64_t resident = static_cast<int64_t>(device_sms()) * kLowpCtas;
+    int64_t ci = groups * tiles / (4 * resident);
+    ci = ci > kLowpCols / tile ? kLowpCols / tile : ci;
+    ci = ci < 1 ? 1 : ci;
+    while ((tiles + ci - 1) / ci > 65535)
+        ci *= 2;
+    const int64_t ny = (tiles + ci - 1) / ci;
+    // the widest B of this engine: 65535 strips of 8 warps over a group's rows
+    const int64_t strip = 32 * lowp_vec(prec) * (h->p.rows_per_group < 8 ? 8 / h->p.rows_per_group : 1);
+    if ((n + strip - 1) / strip > 65535 || groups > 0x7fffffffLL)
+        return cuda_fail(cudaErrorInvalidConfiguration, "spdm_lowp_kernel launch");
+    dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(ny));
+    const size_t smem = 128 + (static_cast<size_t>(chunk) + 2) * sizeof(Entry);
+#define GCOO_LOWP(F, DATA, SCALE)                                                                               \
+    spdm_lowp_kernel<F><<<grid, rows * 32, smem, st>>>(h->packed.ptr, h->row_ptr.ptr, h->m, rows, DATA, SCALE,  \
+                                                       n, dC, static_cast<int32_t>(ci), chunk, h->status.ptr)
     if (prec == GCOO_PREC_BF16)
-        spdm_lowp_kernel<kBF16><<<grid, threads, kSmemBytes, st>>>(h->packed.ptr, h->row_ptr.ptr, h->m, cpg, w->bf.ptr,
-                                                                  nullptr, n, dC, cw, h->status.ptr);
+        GCOO_LOWP(kBF16, w->bf.ptr, nullptr);
     else if (prec == GCOO_PREC_SPLIT_BF16)
-        spdm_lowp_kernel<kSplit><<<grid, threads, kSmemBytes, st>>>(h->packed.ptr, h->row_ptr.ptr, h->m, cpg,
-                                                                   w->split.ptr, nullptr, n, dC, cw, h->status.ptr);
+        GCOO_LOWP(kSplit, w->split.ptr, nullptr);
+    else if (wide)
+        GCOO_LOWP(kFP8Wide, w->bf.ptr, w->scale.ptr);
     else
-        spdm_lowp_kernel<kFP8><<<grid, threads, kSmemBytes, st>>>(h->packed.ptr, h->row_ptr.ptr, h->m, cpg, w->f8.ptr,
-                                                                 w->scale.ptr, n, dC, cw, h->status.ptr);
+        GCOO_LOWP(kFP8, w->f8.ptr, w->scale.ptr);
+#undef GCOO_LOWP
     count_launches(1);
     GCOO_LAUNCH("spdm_lowp_kernel");
     return GCOO_SUCCESS;
