@@ -369,7 +369,7 @@ gcoo_status finish_build(gcoo_handle *h, cudaStream_t st)
     h->pieces_bound = 0;
     if (row_lengths_skewed(h->m, h->nnz, h->max_row_nnz) && h->packed.count >= static_cast<size_t>(h->nnz) + 2) {
         const int64_t cap = h->nnz / long_row_min() + 1;
-        if (!h->long_rows.ensure(static_cast<size_t>(cap)) || !h->long_count.ensure(2))
+        if (!h->long_rows.ensure(2 * static_cast<size_t>(cap)) || !h->long_count.ensure(2))
             return fail(GCOO_ERROR_ALLOC, "device allocation of the long-row list failed");
         unsigned long long *d_cnt = h->long_count.ptr;
         GCOO_CUDA(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(*d_cnt), st));

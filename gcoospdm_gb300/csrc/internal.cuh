@@ -195,7 +195,8 @@ cudaError_t launch_fp8_scales(const float *B, int64_t k, int64_t n, unsigned *am
 int32_t long_row_min(); // 256 entries
 // n % 4 == 0 and a 16-byte aligned B (16-byte copies of B row pieces)
 bool long_rows_ok(int64_t n, const float *B);
-// list[0..min(*count, cap)) = the rows of at least long_row_min() entries (any order)
+// list[0..min(*count, cap)) = the rows of at least long_row_min() entries,
+// longest first to within 64 entries (list: 2 * cap elements)
 cudaError_t launch_collect_long(const int32_t *row_ptr, int64_t m, int32_t *list, int64_t cap,
                                 unsigned long long *count, cudaStream_t st);
 // ---- long rows summed in pieces (spdm_split.cu, gcoo_params.fp32_sum = split) --------------

@@ -394,7 +394,7 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 // CTA barrier -- a row of a dozen entries is all latency, and a staging round
 // trip and a group barrier would double it. The row's two pointers come in
 // one load (lanes 0 and 1) and are shuffled to the warp. Lane i loads entry i
-// of each 32-entry window; the B rows of eight entries at a time are loaded
+// of each 32-entry window; the B rows of four entries at a time are loaded
 // with their columns shuffled from the owning lanes; each column's fmaf chain
 // runs over the row's entries in column order from 0.0f, as in every other
 // FP32 kernel. Measured slower on the Zipf workload (0.148 ms for this
@@ -408,33 +408,38 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 // so one column slab of B is live in L2 instead of all of B: 0.150 -> 0.142
 // ms with the long rows beside it (B 65536 x 256, 67 MB, was read from DRAM
 // about twice in row-major order).
-template <int V>
+// Forty warps per SM with batches of four: 137 us on the Zipf workload with
+// the long rows beside it, against 145 for thirty-two with batches of eight
+// (forty-eight with four: 137, sixty-four 147, forty with eight 145).
+constexpr int kShortBatch = 4, kShortCtas = 20;
+
+template <int V, int U>
 __device__ __forceinline__ void short_window(const Entry &my, int nw, bool all_cols, bool has_col,
                                              const float *__restrict__ Bj, int64_t n, float (&acc)[V])
 {
     int u0 = 0;
     if (all_cols) { // warp-uniform: every lane takes part in the shuffles below
-        // whole batches of eight: no per-entry predicates
-        for (; u0 + 8 <= nw; u0 += 8) {
-            float a[8], b[8][V];
+        // whole batches: no per-entry predicates
+        for (; u0 + U <= nw; u0 += U) {
+            float a[U], b[U][V];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < U; ++u) {
                 const int col = __shfl_sync(0xffffffffu, my.col, u0 + u);
                 a[u] = __shfl_sync(0xffffffffu, my.val, u0 + u);
                 Piece<V>::load(Bj + static_cast<int64_t>(col) * n, b[u]);
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < U; ++u)
 #pragma unroll
                 for (int v = 0; v < V; ++v)
                     acc[v] = fmaf(a[u], b[u][v], acc[v]);
         }
     }
     // the tail batch (and lanes past n: shuffles only)
-    for (; u0 < nw; u0 += 8) {
-        float a[8], b[8][V];
+    for (; u0 < nw; u0 += U) {
+        float a[U], b[U][V];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int col = __shfl_sync(0xffffffffu, my.col, (u0 + u) & 31);
             a[u] = __shfl_sync(0xffffffffu, my.val, (u0 + u) & 31);
             if (u0 + u < nw && has_col) {
@@ -446,7 +451,7 @@ __device__ __forceinline__ void short_window(const Entry &my, int nw, bool all_c
             }
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < U; ++u)
             if (u0 + u < nw)
 #pragma unroll
                 for (int v = 0; v < V; ++v)
@@ -458,7 +463,7 @@ __device__ __forceinline__ void short_window(const Entry &my, int nw, bool all_c
 constexpr int64_t kShortTileMajorBytes = 32ll << 20;
 
 template <int V>
-__global__ void __launch_bounds__(64, 16)
+__global__ void __launch_bounds__(64, kShortCtas)
 spdm_short_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m,
                   const float *__restrict__ B, int64_t n, float *__restrict__ C, int32_t tiles, int32_t long_min,
                   int32_t tile_major)
@@ -498,7 +503,7 @@ spdm_short_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
         my.val = 0.0f;
         if (lane < nw)
             my = packed[rs + w0 + lane];
-        short_window<V>(my, nw, all_cols, has_col, Bj, n, acc);
+        short_window<V, kShortBatch>(my, nw, all_cols, has_col, Bj, n, acc);
     }
     if (has_col)
         Piece<V>::store(C + row * n + j, acc);
