@@ -180,82 +180,94 @@ __global__ void tile_fill_kernel(const Entry *__restrict__ packed, const int32_t
 // With fp8_scale (FP8-B): each value is first quantized to E4M3 in units of
 // its column's power-of-two scale, then stored as the exact BF16 value of
 // E4M3 x scale, so the BF16 MMA multiplies the FP8-B operand exactly.
-// One CTA per tile: the 16 x N block of B is staged in shared memory with
-// coalesced 16-byte loads (64 lanes per 256 columns of a row), then thread
-// jj builds tile row jj (output column jt*N + jj: 16 values read down a
+// One CTA per 256-column tile (two 128-column ones): the 16 x N block of B is
+// staged in shared memory with coalesced 16-byte loads, all of a thread's in
+// flight together, then thread jj builds tile row jj (output column jt*N + jj: 16 values read down a
 // shared-memory column, conflict-free across the warp) and writes its 32
-// bytes with two 16-byte stores, so a warp writes 1 KB contiguous. (Lanes
-// loading 4-byte values down B's columns directly: 20 us for B 8192 x 1024.)
+// bytes with two 16-byte stores, so a warp writes 1 KB contiguous. B 8192 x
+// 1024: 9.5 us (50 MB), split 17 us (84 MB); the terms computed whatever the
+// form and the loads in a loop took 14 and 25.5 us.
 __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo_half, __nv_bfloat16 hi_half)
 {
     return static_cast<uint32_t>(__bfloat16_as_ushort(lo_half)) |
            (static_cast<uint32_t>(__bfloat16_as_ushort(hi_half)) << 16);
 }
 
-constexpr int kBTileMaxN = 256;
-
-// Needs n % 4 == 0 and B 16-byte aligned (the tensor engine takes n % 16 == 0).
+// N = 256 columns (the pair kernel), or 128 with SPLIT. SPLIT: the lo and lo2
+// terms too; FP8: through E4M3 first. Needs n % 4 == 0 and B 16-byte aligned
+// (the tensor engine takes n % 16 == 0).
+template <bool SPLIT, bool FP8>
 __global__ void __launch_bounds__(256)
-b_tiles_kernel(const float *__restrict__ B, int64_t k, int64_t n, int N, int64_t kb, __nv_bfloat16 *__restrict__ hi,
+b_tiles_kernel(const float *__restrict__ B, int64_t k, int64_t n, int64_t kb, __nv_bfloat16 *__restrict__ hi,
                __nv_bfloat16 *__restrict__ lo, const float *__restrict__ fp8_scale)
 {
-    __shared__ __align__(16) float blk[kTileK][kBTileMaxN];
-    const int64_t cb = blockIdx.x;
+    constexpr int N = SPLIT ? 128 : 256, kT = 256 / N; // kT tiles (column blocks of 16 k) per CTA
+    constexpr int kLoads = kTileK * N * kT / 4 / 256;  // float4 per thread
+    __shared__ __align__(16) float blk[kT][kTileK][N];
+    const int64_t cb0 = static_cast<int64_t>(blockIdx.x) * kT;
     const int64_t jt = blockIdx.y;
-    const int64_t tile = jt * kb + cb;
-    const size_t tile_elems = static_cast<size_t>(N) * kTileK;
-    const int n4 = N / 4; // float4 columns per block row
-    for (int i = threadIdx.x; i < kTileK * n4; i += blockDim.x) {
-        const int r = i / n4, c4 = i - r * n4;
-        const int64_t c = cb * kTileK + r;
-        const int64_t j = jt * N + c4 * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < k && j < n)
-            v = __ldg(reinterpret_cast<const float4 *>(B + c * n + j));
-        *reinterpret_cast<float4 *>(&blk[r][c4 * 4]) = v;
+    constexpr size_t tile_elems = static_cast<size_t>(N) * kTileK;
+    float4 v4[kLoads];
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+        const int i = u * 256 + threadIdx.x;
+        const int r = i / (N / 4), c4 = i % (N / 4); // r: row inside the kT blocks
+        const int64_t c = cb0 * kTileK + r, j = jt * N + c4 * 4;
+        v4[u] = c < k && j < n ? __ldg(reinterpret_cast<const float4 *>(B + c * n + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+        const int i = u * 256 + threadIdx.x;
+        *reinterpret_cast<float4 *>(&blk[0][0][0] + i * 4) = v4[u];
     }
     __syncthreads();
-    for (int jj = threadIdx.x; jj < N; jj += blockDim.x) {
-        const int64_t j = jt * N + jj;
-        float sc = 1.0f;
-        if (fp8_scale && j < n)
-            sc = fp8_scale[j];
-        // a power of two in the normal range has an exact reciprocal, so
-        // v * inv is v / sc exactly; otherwise divide
-        const bool by_inv = sc >= 1.17549435e-38f && sc <= 8.50705917e37f;
-        const float inv = by_inv ? 1.0f / sc : 0.0f;
-        uint32_t wh[8], wl[8], wl2[8];
+    const int t = threadIdx.x / N, jj = threadIdx.x % N;
+    const int64_t tile = jt * kb + cb0 + t;
+    if (cb0 + t >= kb)
+        return;
+    const int64_t j = jt * N + jj;
+    float sc = 1.0f;
+    if (FP8 && j < n)
+        sc = fp8_scale[j];
+    // a power of two in the normal range has an exact reciprocal, so
+    // v * inv is v / sc exactly; otherwise divide
+    const bool by_inv = sc >= 1.17549435e-38f && sc <= 8.50705917e37f;
+    const float inv = by_inv ? 1.0f / sc : 0.0f;
+    uint32_t wh[8], wl[8], wl2[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            __nv_bfloat16 h2[2], l2[2], m2[2];
+    for (int q = 0; q < 8; ++q) {
+        __nv_bfloat16 h2[2], l2[2], m2[2];
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                float v = blk[q * 2 + e][jj];
-                if (fp8_scale && j < n) {
-                    const __nv_fp8_storage_t f8 =
-                        __nv_cvt_float_to_fp8(by_inv ? v * inv : v / sc, __NV_SATFINITE, __NV_E4M3);
-                    v = __half2float(__half(__nv_cvt_fp8_to_halfraw(f8, __NV_E4M3))) * sc;
-                }
-                h2[e] = __float2bfloat16_rn(v);
+        for (int e = 0; e < 2; ++e) {
+            float v = blk[t][q * 2 + e][jj];
+            if (FP8 && j < n) {
+                const __nv_fp8_storage_t f8 =
+                    __nv_cvt_float_to_fp8(by_inv ? v * inv : v / sc, __NV_SATFINITE, __NV_E4M3);
+                v = __half2float(__half(__nv_cvt_fp8_to_halfraw(f8, __NV_E4M3))) * sc;
+            }
+            h2[e] = __float2bfloat16_rn(v);
+            if (SPLIT) {
                 const float r1 = v - __bfloat162float(h2[e]); // exact
                 l2[e] = __float2bfloat16_rn(r1);
                 m2[e] = __float2bfloat16_rn(r1 - __bfloat162float(l2[e]));
             }
-            wh[q] = pack_bf16(h2[0], h2[1]);
+        }
+        wh[q] = pack_bf16(h2[0], h2[1]);
+        if (SPLIT) {
             wl[q] = pack_bf16(l2[0], l2[1]);
             wl2[q] = pack_bf16(m2[0], m2[1]);
         }
+    }
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const uint32_t off = sw32_offset(static_cast<uint32_t>(jj), static_cast<uint32_t>(half * 8)) / 2;
-            const int w0 = half * 4;
-            *reinterpret_cast<uint4 *>(hi + tile * tile_elems + off) = make_uint4(wh[w0], wh[w0 + 1], wh[w0 + 2], wh[w0 + 3]);
-            if (lo) {
-                *reinterpret_cast<uint4 *>(lo + 2 * tile * tile_elems + off) =
-                    make_uint4(wl[w0], wl[w0 + 1], wl[w0 + 2], wl[w0 + 3]);
-                *reinterpret_cast<uint4 *>(lo + (2 * tile + 1) * tile_elems + off) =
-                    make_uint4(wl2[w0], wl2[w0 + 1], wl2[w0 + 2], wl2[w0 + 3]);
-            }
+    for (int half = 0; half < 2; ++half) {
+        const uint32_t off = sw32_offset(static_cast<uint32_t>(jj), static_cast<uint32_t>(half * 8)) / 2;
+        const int w0 = half * 4;
+        *reinterpret_cast<uint4 *>(hi + tile * tile_elems + off) = make_uint4(wh[w0], wh[w0 + 1], wh[w0 + 2], wh[w0 + 3]);
+        if (SPLIT) {
+            *reinterpret_cast<uint4 *>(lo + 2 * tile * tile_elems + off) =
+                make_uint4(wl[w0], wl[w0 + 1], wl[w0 + 2], wl[w0 + 3]);
+            *reinterpret_cast<uint4 *>(lo + (2 * tile + 1) * tile_elems + off) =
+                make_uint4(wl2[w0], wl2[w0 + 1], wl2[w0 + 2], wl2[w0 + 3]);
         }
     }
 }
@@ -829,10 +841,15 @@ gcoo_status tc_spdm(gcoo_handle *h, const float *dB, int64_t n, float *dC, bool 
     const int N = tile_n_for(p.split);
     if (fp8)
         GCOO_CUDA(launch_fp8_scales(dB, h->k, n, p.b_amax.ptr, p.b_scale.ptr, st));
-    dim3 g(static_cast<unsigned>(p.kb), static_cast<unsigned>((n + N - 1) / N));
-    b_tiles_kernel<<<g, 256, 0, st>>>(dB, h->k, n, N, p.kb, reinterpret_cast<__nv_bfloat16 *>(p.b_hi.ptr),
-                                      p.split ? reinterpret_cast<__nv_bfloat16 *>(p.b_lo.ptr) : nullptr,
-                                      fp8 ? p.b_scale.ptr : nullptr);
+    const int per_cta = p.split ? 2 : 1;
+    dim3 g(static_cast<unsigned>((p.kb + per_cta - 1) / per_cta), static_cast<unsigned>((n + N - 1) / N));
+    __nv_bfloat16 *hi = reinterpret_cast<__nv_bfloat16 *>(p.b_hi.ptr), *lo = reinterpret_cast<__nv_bfloat16 *>(p.b_lo.ptr);
+    if (p.split)
+        b_tiles_kernel<true, false><<<g, 256, 0, st>>>(dB, h->k, n, p.kb, hi, lo, nullptr);
+    else if (fp8)
+        b_tiles_kernel<false, true><<<g, 256, 0, st>>>(dB, h->k, n, p.kb, hi, nullptr, p.b_scale.ptr);
+    else
+        b_tiles_kernel<false, false><<<g, 256, 0, st>>>(dB, h->k, n, p.kb, hi, nullptr, nullptr);
     count_launches(1);
     GCOO_LAUNCH("b_tiles_kernel");
     if (p.split) {
