@@ -20,8 +20,9 @@
 // stage with tensor-map bulk copies (cta_group::2, completing on the first
 // CTA's barrier), and the first CTA issues tcgen05.mma.cta_group::2 (M=256,
 // N=256, K=16) into both CTAs' tensor memory, one accumulator per 256
-// columns. Split-BF16 kernel (spdm_tc_kernel): one CTA per (128-row panel,
-// 128 columns), one stage per tile, six MMAs per tile. Every wait is bounded.
+// columns. Split-BF16 kernel (spdm_tc_split_kernel): equal shares of the
+// (tile, 128 columns) products, two CTAs per SM, one stage per tile, six MMAs
+// per tile. Every wait is bounded.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -37,6 +38,7 @@ namespace gcoo {
 constexpr int kPanel = 128;   // rows of a tile half (one CTA's MMA rows)
 constexpr int kTileK = 16;    // columns per tile (MMA K)
 constexpr int kTileBytes = kPanel * kTileK * 2; // one 128-row half
+constexpr uint64_t kDrainNs = 2000000; // after a wait gives up: time for copies in flight to land
 
 struct TcPlan {
     int64_t panels = 0, kb = 0, tiles = 0;
@@ -50,6 +52,7 @@ struct TcPlan {
     DevBuf<int64_t> scratch;
     // B workspace (per call)
     DevBuf<uint16_t> b_hi, b_lo; // b_lo (split only): lo then lo2 per B tile
+    DevBuf<float> part;          // split only: sums of (panel, 128 columns) that lie in several shares
     int64_t b_n = 0;
     // FP8-B: per-column power-of-two scales (and their absmax scratch)
     DevBuf<float> b_scale;
@@ -115,6 +118,21 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
 #pragma unroll
     for (int i = 0; i < 32; ++i)
         v[i] = __uint_as_float(r[i]);
+}
+
+// 32 consecutive columns of a row of C, `left` of them inside it
+__device__ __forceinline__ void store_row32(float *out, const float (&v)[32], int64_t left)
+{
+    if (left >= 32) {
+#pragma unroll
+        for (int q = 0; q < 32; q += 4)
+            *reinterpret_cast<float4 *>(out + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+            if (q < left)
+                out[q] = v[q];
+    }
 }
 
 // Byte offset of element (row r, column c) of a 32-byte-row K-major tile in
@@ -272,57 +290,102 @@ b_tiles_kernel(const float *__restrict__ B, int64_t k, int64_t n, int64_t kb, __
     }
 }
 
-// ---- the MMA kernel ---------------------------------------------------------------------
-template <int N, int S, bool SPLIT>
-struct TcCfg {
-    static constexpr int kABytes = kTileBytes * (SPLIT ? 3 : 1); // hi (, lo, lo2)
-    static constexpr int kBBytes = N * 32 * (SPLIT ? 3 : 1);
-    static constexpr int kStage = kABytes + kBBytes;
-    static constexpr int kBanks = SPLIT ? 2 : 1;       // accumulators of N columns each
-    static constexpr int kTmemCols = N * kBanks;       // a power of two in [32, 512]
-    static constexpr int kSmem = 1024 /* barriers, tmem slot */ + S * kStage + 1024 /* alignment slack */;
-    static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0,
-                  "tensor memory is allocated in powers of two of at most 512 columns");
-    static_assert(kSmem <= 227 * 1024, "the ring must fit one CTA's shared memory");
+// ---- split-BF16: one CTA per equal share of the tiles ---------------------------------
+// The tile products (tile t of the plan x 128 output columns jt) are ordered
+// w = jt * tiles + t and cut into equal consecutive shares, one per CTA, two
+// CTAs per SM: no wave of CTAs is nearly empty and a few panels fill the GPU.
+// Measured with 16 x 16 blocks at 25 % (us; a CTA per panel and 128 columns
+// before): 8192^2, n = 1024 458 -> 407 (the kernel 424 -> 362, 2.05 PFLOP/s of
+// MMAs, and 14 of fix-up), n = 128 216 -> 87; 2048 x 8192, n = 256 222 -> 58;
+// 2048^2, n = 1024 67 -> 52; 1024^2 at 15 %, n = 64 32 -> 28. A share is
+// walked panel by panel; a (panel, jt) that lies in one share is written to
+// C, the others' sums go to a workspace and tc_fixup_kernel adds them in
+// order. Every CTA's share and every place of the workspace follow from
+// (tiles, columns, CTAs) alone, so the sums are the same on every run.
+constexpr int kSplitN = 128;  // output columns of a tile product (MMA N)
+constexpr int kSplitS = 4;    // stages of one tile each
+constexpr int kSplitABytes = 3 * kTileBytes, kSplitBBytes = 3 * kSplitN * 32;
+constexpr int kSplitStage = kSplitABytes + kSplitBBytes; // hi, lo, lo2 of both
+constexpr int kSplitSmem = 1024 /* barriers, tmem slot */ + kSplitS * kSplitStage + 1024 /* alignment slack */;
+constexpr int kSplitThreads = 192; // warps 0-3: epilogue (their tensor-memory lanes); 4: copies; 5: MMAs
+constexpr int64_t kSplitMinTiles = 16; // tiles per CTA at least, where there are so many
+constexpr int kPartFloats = kPanel * kSplitN;
+static_assert(2 * kSplitSmem <= 227 * 1024, "two CTAs per SM: 2 x 256 tensor-memory columns");
+
+__host__ __device__ __forceinline__ int64_t share_begin(int64_t work, int64_t ctas, int64_t g) { return work * g / ctas; }
+
+// The consecutive pieces of a share: (panel, jt, tiles [t0, t1)), `first`: the
+// share starts with it; `whole`: all of the panel's tiles.
+struct ShareWalk {
+    const int32_t *pf;
+    int64_t kb, panels, tiles, w, end, begin;
+    int64_t panel, jt, t0, t1;
+    bool first, whole;
+    __device__ __forceinline__ ShareWalk(const int32_t *pf_, int64_t kb_, int64_t panels_, int64_t tiles_, int64_t work,
+                                         int64_t ctas, int64_t g)
+        : pf(pf_), kb(kb_), panels(panels_), tiles(tiles_), w(share_begin(work, ctas, g)),
+          end(share_begin(work, ctas, g + 1)), begin(w)
+    {
+    }
+    __device__ __forceinline__ bool next()
+    {
+        if (w >= end)
+            return false;
+        first = w == begin;
+        jt = w / tiles;
+        t0 = w - jt * tiles;
+        int64_t lo = 0, hi = panels; // the panel with pf[panel * kb] <= t0 < pf[(panel + 1) * kb]
+        while (hi - lo > 1) {
+            const int64_t mid = (lo + hi) / 2;
+            if (pf[mid * kb] <= t0)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        panel = lo;
+        const int64_t p0 = pf[panel * kb], p1 = pf[(panel + 1) * kb];
+        const int64_t left = end - w;
+        t1 = p1 - t0 <= left ? p1 : t0 + left;
+        whole = t0 == p0 && t1 == p1;
+        w += t1 - t0;
+        return true;
+    }
 };
 
-template <int N, int S, bool SPLIT>
-__global__ void __launch_bounds__(128, 1)
-spdm_tc_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__ tile_cb, const uint16_t *__restrict__ a_hi,
-               const uint16_t *__restrict__ a_lo, const uint16_t *__restrict__ b_hi, const uint16_t *__restrict__ b_lo,
-               int64_t m, int64_t n, int64_t kb, float *__restrict__ C, uint32_t *__restrict__ status)
+__global__ void __launch_bounds__(kSplitThreads, 1)
+spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__ tile_cb,
+                     const uint16_t *__restrict__ a_hi, const uint16_t *__restrict__ a_lo,
+                     const uint16_t *__restrict__ b_hi, const uint16_t *__restrict__ b_lo, int64_t m, int64_t n,
+                     int64_t kb, int64_t panels, int64_t tiles, int64_t work, float *__restrict__ C,
+                     float *__restrict__ part, uint32_t *__restrict__ status)
 {
-    using Cfg = TcCfg<N, S, SPLIT>;
+    constexpr int N = kSplitN, S = kSplitS;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // carve: [0,1024) control, then 1024-aligned stages
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(base);
     uint64_t *empty = full + S;
-    uint64_t *done = empty + S;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
+    uint64_t *done = empty + S;   // a piece's MMAs have completed
+    uint64_t *drained = done + 1; // its sums have been read out of tensor memory
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     unsigned char *stages = base + 1024;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t panel = blockIdx.x;
-    const int64_t jt = blockIdx.y;
-    const int64_t t0 = pf[panel * kb];
-    const int64_t t1 = pf[(panel + 1) * kb];
-    const int64_t ntiles = t1 - t0;
-
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         mbar_init(done, 1);
+        mbar_init(drained, 4); // one arrival per epilogue warp
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 2) {
+    if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(Cfg::kTmemCols)
+                     "r"(2 * N)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -330,125 +393,191 @@ spdm_tc_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__ tile_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // split-BF16 keeps the leading products (ah * bh) in bank 0 and the five
-    // correction products in bank 1, so each correction is rounded at its
-    // own (2^-8 smaller) magnitude, not at the running total's; the epilogue
-    // adds bank 1 to bank 0
-    constexpr int BANKS = Cfg::kBanks;
-    const int banks_used = BANKS;
+    // The leading products (ah * bh) go to bank 0 and the five correction
+    // products to bank 1, so each correction is rounded at its own (2^-8
+    // smaller) magnitude, not at the running total's; the epilogue adds bank
+    // 1 to bank 0.
+    ShareWalk sh(pf, kb, panels, tiles, work, gridDim.x, blockIdx.x);
 
-    if (ntiles > 0) {
-        if (warp == 0 && lane == 0) {
-            // producer
-            for (int64_t i = 0; i < ntiles; ++i) {
-                const int s = static_cast<int>(i % S);
-                if (i >= S && !mbar_wait(&empty[s], static_cast<uint32_t>(((i / S) - 1) & 1))) {
-                    atomicOr(status, kStatusWaitTimeout);
-                    *abort_flag = 1;
-                    break;
-                }
-                if (*abort_flag)
-                    break;
-                unsigned char *st = stages + static_cast<size_t>(s) * Cfg::kStage;
-                const int64_t tile = t0 + i;
-                const int64_t btile = jt * kb + tile_cb[tile];
-                mbar_arrive_expect_tx(&full[s], Cfg::kStage);
-                bulk_g2s(st, a_hi + tile * (kTileBytes / 2), kTileBytes, &full[s]);
-                bulk_g2s(st + Cfg::kABytes, b_hi + btile * (N * 16), N * 32, &full[s]);
-                if (SPLIT) { // lo and lo2 of A, then of B: one contiguous copy each
+    if (warp == 4) {
+        if (lane == 0) {
+            // copies: the ring runs on over the pieces
+            int64_t i = 0;
+            bool ok = true;
+            while (ok && sh.next()) {
+                for (int64_t tile = sh.t0; tile < sh.t1; ++tile, ++i) {
+                    const int s = static_cast<int>(i % S);
+                    if (*abort_flag || (i >= S && !mbar_wait(&empty[s], static_cast<uint32_t>(((i / S) - 1) & 1)))) {
+                        atomicOr(status, kStatusWaitTimeout);
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    unsigned char *st = stages + static_cast<size_t>(s) * kSplitStage;
+                    const int64_t btile = sh.jt * kb + tile_cb[tile];
+                    mbar_arrive_expect_tx(&full[s], kSplitStage);
+                    bulk_g2s(st, a_hi + tile * (kTileBytes / 2), kTileBytes, &full[s]);
+                    bulk_g2s(st + kSplitABytes, b_hi + btile * (N * 16), N * 32, &full[s]);
+                    // lo and lo2 of A, then of B: one contiguous copy each
                     bulk_g2s(st + kTileBytes, a_lo + tile * kTileBytes, 2 * kTileBytes, &full[s]);
-                    bulk_g2s(st + Cfg::kABytes + N * 32, b_lo + btile * (N * 32), 2 * N * 32, &full[s]);
+                    bulk_g2s(st + kSplitABytes + N * 32, b_lo + btile * (N * 32), 2 * N * 32, &full[s]);
                 }
             }
-        } else if (warp == 1 && lane == 0) {
-            // MMA issuer
+        }
+    } else if (warp == 5) {
+        if (lane == 0) {
             const uint32_t idesc = idesc_bf16(kPanel, N);
             int64_t i = 0;
-            for (; i < ntiles; ++i) {
-                const int s = static_cast<int>(i % S);
-                if (!mbar_wait(&full[s], static_cast<uint32_t>((i / S) & 1))) {
-                    atomicOr(status, kStatusWaitTimeout);
-                    *abort_flag = 1;
-                    break;
-                }
+            uint32_t piece = 0;
+            bool ok = true;
+            while (ok && sh.next()) {
+                // the piece before this one has been read out
+                if (piece > 0 && !mbar_wait(drained, (piece - 1) & 1))
+                    ok = false;
                 tc_fence_after();
-                const uint32_t st = smem_u32(stages + static_cast<size_t>(s) * Cfg::kStage);
-                const uint64_t ah = smem_desc_sw32(st);
-                const uint64_t bh = smem_desc_sw32(st + Cfg::kABytes);
-                tc_mma(tmem, ah, bh, idesc, i > 0 ? 1u : 0u);
-                if (SPLIT) {
+                for (int64_t tile = sh.t0; ok && tile < sh.t1; ++tile, ++i) {
+                    const int s = static_cast<int>(i % S);
+                    if (!mbar_wait(&full[s], static_cast<uint32_t>((i / S) & 1))) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t acc = tile > sh.t0 ? 1u : 0u;
+                    const uint32_t st = smem_u32(stages + static_cast<size_t>(s) * kSplitStage);
+                    const uint64_t ah = smem_desc_sw32(st);
+                    const uint64_t bh = smem_desc_sw32(st + kSplitABytes);
+                    tc_mma(tmem, ah, bh, idesc, acc);
                     // (ah + al + al2)(bh + bl + bl2): every product above 2^-24
                     // of the leading one (al * bl2, al2 * bl, al2 * bl2 dropped),
                     // into the correction bank
                     const uint32_t dx = tmem + static_cast<uint32_t>(N);
                     const uint64_t al = smem_desc_sw32(st + kTileBytes);
                     const uint64_t al2 = smem_desc_sw32(st + 2 * kTileBytes);
-                    const uint64_t bl = smem_desc_sw32(st + Cfg::kABytes + N * 32);
-                    const uint64_t bl2 = smem_desc_sw32(st + Cfg::kABytes + 2 * N * 32);
-                    tc_mma(dx, ah, bl, idesc, i > 0 ? 1u : 0u);
+                    const uint64_t bl = smem_desc_sw32(st + kSplitABytes + N * 32);
+                    const uint64_t bl2 = smem_desc_sw32(st + kSplitABytes + 2 * N * 32);
+                    tc_mma(dx, ah, bl, idesc, acc);
                     tc_mma(dx, al, bh, idesc, 1u);
                     tc_mma(dx, al, bl, idesc, 1u);
                     tc_mma(dx, ah, bl2, idesc, 1u);
                     tc_mma(dx, al2, bh, idesc, 1u);
+                    tc_commit(&empty[s]); // slot reusable once these MMAs have read it
                 }
-                tc_commit(&empty[s]); // slot reusable once these MMAs have read it
+                tc_commit(done); // arrives when every MMA issued above has completed
+                ++piece;
             }
-            tc_commit(done); // arrives when every MMA issued above has completed
-        }
-        __syncwarp();
-        // epilogue: all four warps (warp w owns TMEM lanes 32w..32w+31 = panel rows)
-        const bool ok = mbar_wait(done, 0);
-        if (!ok && lane == 0)
-            atomicOr(status, kStatusWaitTimeout);
-        tc_fence_after();
-        const int64_t row = panel * kPanel + warp * 32 + lane;
-        if (__all_sync(0xffffffffu, ok ? 1 : 0) && !*abort_flag) {
-#pragma unroll 1
-            for (int c = 0; c < N; c += 32) {
-                float v[32];
-                tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c), v);
-                for (int bank = 1; bank < banks_used; ++bank) {
-                    float w[32];
-                    tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(bank * N + c), w);
-#pragma unroll
-                    for (int q = 0; q < 32; ++q)
-                        v[q] += w[q];
-                }
-                const int64_t j = jt * N + c;
-                if (row < m && j < n) {
-                    float *out = C + row * n + j;
-                    if (j + 32 <= n) {
-#pragma unroll
-                        for (int q = 0; q < 32; q += 4)
-                            *reinterpret_cast<float4 *>(out + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 32; ++q)
-                            if (j + q < n)
-                                out[q] = v[q];
-                    }
-                }
+            if (!ok) {
+                atomicOr(status, kStatusWaitTimeout);
+                *abort_flag = 1;
             }
-        }
-        // the producer's copies in flight must land before the CTA exits
-        if (*abort_flag && threadIdx.x == 0) {
-            for (int s = 0; s < S; ++s)
-                mbar_wait(&full[s], 0);
         }
     } else {
-        // panel without entries: C rows are zero
-        const int64_t row = panel * kPanel + warp * 32 + lane;
-        if (row < m)
-            for (int64_t j = jt * N; j < (jt + 1) * N && j < n; ++j)
-                C[row * n + j] = 0.0f;
+        // epilogue: warp w owns TMEM lanes 32w..32w+31 = panel rows
+        uint32_t piece = 0;
+        while (sh.next()) {
+            const bool ok = mbar_wait(done, piece & 1);
+            if (!__all_sync(0xffffffffu, ok ? 1 : 0) || *abort_flag) {
+                if (lane == 0) {
+                    atomicOr(status, kStatusWaitTimeout);
+                    *abort_flag = 1;
+                }
+                break;
+            }
+            tc_fence_after();
+            const int lr = warp * 32 + lane;
+            const int64_t row = sh.panel * kPanel + lr;
+            float *slot = part + (2 * static_cast<int64_t>(blockIdx.x) + (sh.first ? 0 : 1)) * kPartFloats;
+#pragma unroll 1
+            for (int c = 0; c < N; c += 32) {
+                float v[32], w[32];
+                tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c), v);
+                tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(N + c), w);
+#pragma unroll
+                for (int q = 0; q < 32; ++q)
+                    v[q] += w[q];
+                const int64_t j = sh.jt * N + c;
+                if (!sh.whole) { // [column][row]: contiguous across the warp
+#pragma unroll
+                    for (int q = 0; q < 32; ++q)
+                        slot[(c + q) * kPanel + lr] = v[q];
+                } else if (row < m && j < n) {
+                    store_row32(C + row * n + j, v, n - j);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(drained);
+            ++piece;
+        }
+    }
+    __syncwarp(); // warps 4 and 5: their one working lane is back
+    __syncthreads();
+    // after a wait gave up, copies already issued may still be landing in
+    // this CTA's shared memory: give them a bounded time before it is released
+    if (threadIdx.x == 0 && *abort_flag) {
+        const uint64_t t_end = global_ns() + kDrainNs;
+        while (global_ns() < t_end)
+            __nanosleep(10000);
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 2) {
+    if (warp == 5) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::kTmemCols)
-                     : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * N) : "memory");
     }
+}
+
+// C of the (panel, 128 columns) whose tiles lie in several shares (their
+// parts added in order) or that have none (zeros). One thread per row, 32 of
+// the columns per CTA.
+__global__ void __launch_bounds__(kPanel)
+tc_fixup_kernel(const int32_t *__restrict__ pf, int64_t m, int64_t n, int64_t kb, int64_t tiles, int64_t work,
+                int64_t ctas, const float *__restrict__ part, float *__restrict__ C)
+{
+    const int64_t panel = blockIdx.x, jt = blockIdx.y;
+    const int64_t p0 = pf[panel * kb], p1 = pf[(panel + 1) * kb];
+    const int64_t row = panel * kPanel + threadIdx.x;
+    const int64_t w0 = jt * tiles + p0, w1 = jt * tiles + p1;
+    int64_t g0 = 0, g1 = -1; // the shares with tiles of it
+    if (p1 > p0) {
+        // share g holds w where share_begin(g) <= w < share_begin(g + 1)
+        g0 = w0 * ctas / work;
+        while (g0 > 0 && share_begin(work, ctas, g0) > w0)
+            --g0;
+        while (share_begin(work, ctas, g0 + 1) <= w0)
+            ++g0;
+        g1 = g0;
+        while (share_begin(work, ctas, g1 + 1) < w1)
+            ++g1;
+        if (g1 == g0)
+            return; // in one share: written there
+    }
+    const int c = blockIdx.z * 32;
+    float v[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+        v[q] = 0.0f;
+    for (int64_t g = g0; g <= g1; g += 2) { // two parts' loads in flight together
+        float x[32], y[32];
+        // a share's first piece starts where the share does
+        const float *sx = part + (2 * g + (share_begin(work, ctas, g) >= w0 ? 0 : 1)) * kPartFloats + c * kPanel + threadIdx.x;
+        const float *sy = part + 2 * (g + 1) * kPartFloats + c * kPanel + threadIdx.x; // never the panel's first share
+        const bool two = g < g1;
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            x[q] = sx[q * kPanel];
+            y[q] = two ? sy[q * kPanel] : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            v[q] += x[q];
+            if (two)
+                v[q] += y[q];
+        }
+    }
+    const int64_t j = jt * kSplitN + c;
+    if (row < m && j < n)
+        store_row32(C + row * n + j, v, n - j);
 }
 
 // ---- the pair kernel (BF16, FP8-B) ----------------------------------------------------
@@ -505,7 +634,6 @@ constexpr int kPairHalf = kTileBytes;      // 4 KB: a tile's 128-row half, or a 
 constexpr int kPairStage = (1 + kPairMaxNT) * kPairK * kPairHalf; // [A halves][B halves, accumulator 0][... 1]
 constexpr int kPairS = 2;                  // stages of 96 KB: 194 KB, so one CTA per SM
 constexpr int kPairSmem = 1024 + kPairS * kPairStage + 1024;
-constexpr uint64_t kPairDrainNs = 2000000; // after a wait gives up: time for copies in flight to land
 static_assert(kPairSmem <= 227 * 1024 && 2 * kPairSmem > 228 * 1024,
               "one pair CTA per SM: its tensor-memory allocation never waits for another");
 
@@ -625,19 +753,8 @@ spdm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                 float v[32];
                 tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c), v);
                 const int64_t j = jt * nt_cta * N + c;
-                if (row < m && j < n) {
-                    float *out = C + row * n + j;
-                    if (j + 32 <= n) {
-#pragma unroll
-                        for (int q = 0; q < 32; q += 4)
-                            *reinterpret_cast<float4 *>(out + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 32; ++q)
-                            if (j + q < n)
-                                out[q] = v[q];
-                    }
-                }
+                if (row < m && j < n)
+                    store_row32(C + row * n + j, v, n - j);
             }
         }
     } else {
@@ -651,7 +768,7 @@ spdm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     // issued may still be landing in this CTA or signalling the first CTA's
     // barriers: give them a bounded time before the pair leaves
     if (threadIdx.x == 0 && (gave_up || (*reinterpret_cast<volatile uint32_t *>(status) & kStatusWaitTimeout))) {
-        const uint64_t t_end = global_ns() + kPairDrainNs;
+        const uint64_t t_end = global_ns() + kDrainNs;
         while (global_ns() < t_end)
             __nanosleep(10000);
     }
@@ -749,17 +866,30 @@ cudaError_t launch_pair(TcPlan &p, int64_t m, int64_t n, float *C, uint32_t *sta
     return cudaGetLastError();
 }
 
-template <int N, int S, bool SPLIT>
-cudaError_t launch_tc(const TcPlan &p, int64_t m, int64_t n, float *C, uint32_t *status, cudaStream_t st)
+// CTAs of the split kernel: two per SM, fewer where a share would be short
+int64_t split_ctas(int64_t work)
 {
-    using Cfg = TcCfg<N, S, SPLIT>;
-    auto kern = spdm_tc_kernel<N, S, SPLIT>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
-    if (e != cudaSuccess)
-        return e;
-    dim3 grid(static_cast<unsigned>(p.panels), static_cast<unsigned>((n + N - 1) / N));
-    kern<<<grid, 128, Cfg::kSmem, st>>>(p.pf.ptr, p.tile_cb.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n,
-                                        p.kb, C, status);
+    const int64_t most = 2 * static_cast<int64_t>(device_sms());
+    const int64_t by_work = work / kSplitMinTiles;
+    return by_work < 1 ? 1 : (by_work > most ? most : by_work);
+}
+
+cudaError_t launch_split(const TcPlan &p, int64_t m, int64_t n, float *C, uint32_t *status, cudaStream_t st)
+{
+    const int64_t njt = (n + kSplitN - 1) / kSplitN, work = p.tiles * njt, ctas = split_ctas(work);
+    if (njt > 65535 || p.panels > 0x7fffffffLL)
+        return cudaErrorInvalidConfiguration;
+    if (work > 0) {
+        const cudaError_t e = cudaFuncSetAttribute(spdm_tc_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+        if (e != cudaSuccess)
+            return e;
+        spdm_tc_split_kernel<<<static_cast<unsigned>(ctas), kSplitThreads, kSplitSmem, st>>>(
+            p.pf.ptr, p.tile_cb.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n, p.kb, p.panels, p.tiles, work,
+            C, p.part.ptr, status);
+        count_launches(1);
+    }
+    const dim3 grid(static_cast<unsigned>(p.panels), static_cast<unsigned>(njt), kSplitN / 32);
+    tc_fixup_kernel<<<grid, kPanel, 0, st>>>(p.pf.ptr, m, n, p.kb, p.tiles, work, ctas, p.part.ptr, C);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -828,7 +958,9 @@ gcoo_status tc_prepare_b(gcoo_handle *h, int64_t n, bool fp8)
     const int N = tile_n_for(p.split);
     const int64_t nt = (n + N - 1) / N;
     const size_t elems = static_cast<size_t>(nt) * p.kb * N * kTileK;
-    if (!p.b_hi.ensure(elems) || (p.split && !p.b_lo.ensure(2 * elems)) ||
+    // the parts of the split kernel's shares: two per CTA, whatever the width
+    const size_t parts = p.split ? 4 * static_cast<size_t>(device_sms()) * kPartFloats : 0;
+    if (!p.b_hi.ensure(elems) || (p.split && (!p.b_lo.ensure(2 * elems) || !p.part.ensure(parts))) ||
         (fp8 && (!p.b_scale.ensure(static_cast<size_t>(n)) || !p.b_amax.ensure(static_cast<size_t>(n)))))
         return fail(GCOO_ERROR_ALLOC, "device allocation of the B tiles failed");
     p.b_n = n;
@@ -853,9 +985,9 @@ gcoo_status tc_spdm(gcoo_handle *h, const float *dB, int64_t n, float *dC, bool 
     count_launches(1);
     GCOO_LAUNCH("b_tiles_kernel");
     if (p.split) {
-        const cudaError_t e = launch_tc<128, 4, true>(p, h->m, n, dC, h->status.ptr, st);
+        const cudaError_t e = launch_split(p, h->m, n, dC, h->status.ptr, st);
         if (e != cudaSuccess)
-            return cuda_fail(e, "spdm_tc_kernel launch");
+            return cuda_fail(e, "spdm_tc_split_kernel launch");
         return GCOO_SUCCESS;
     }
     const cudaError_t e = launch_pair(p, h->m, n, dC, h->status.ptr, st);
