@@ -15,12 +15,12 @@
 //   * B is converted per call into tiles of N output columns x 16 k (the
 //     same layout, N rows of 32 bytes).
 // BF16 / FP8-B kernel (spdm_tc_pair_kernel): a cluster of two CTAs on two
-// SMs per (256-row panel, 256 or 512 output columns); each CTA streams its
-// 128-row half of four tiles and its 128-column halves of their B tiles per
-// stage with tensor-map bulk copies (cta_group::2, completing on the first
-// CTA's barrier), and the first CTA issues tcgen05.mma.cta_group::2 (M=256,
-// N=256, K=16) into both CTAs' tensor memory, one accumulator per 256
-// columns. Split-BF16 kernel (spdm_tc_split_kernel): equal shares of the
+// SMs per (256-row panel, 256 or 512 output columns), or per equal share of
+// the products where those would leave SMs idle; each CTA streams its 128-row
+// half of four tiles and its 128-column halves of their B tiles per stage
+// with tensor-map bulk copies (cta_group::2, completing on the first CTA's
+// barrier), and the first CTA issues tcgen05.mma.cta_group::2 (M=256, N=256,
+// K=16) into both CTAs' tensor memory, one accumulator per 256 columns. Split-BF16 kernel (spdm_tc_split_kernel): equal shares of the
 // (tile, 128 columns) products, two CTAs per SM, one stage per tile, six MMAs
 // per tile. Every wait is bounded.
 #include <cuda_bf16.h>
@@ -47,20 +47,17 @@ struct TcPlan {
     int64_t nnz = 0;
     DevBuf<int32_t> pf;       // exclusive prefix over (panel, cb) flags, size panels*kb + 1
     DevBuf<int32_t> tile_cb;  // cb of each tile (ascending within a panel)
+    DevBuf<int32_t> tile_panel; // panel of each tile
     DevBuf<uint16_t> a_hi;    // tiles * (panel_rows / 128) * 2048 bf16 (swizzled halves)
     DevBuf<uint16_t> a_lo;    // split only: tiles * 2 * 2048 bf16 (lo, then lo2, per tile)
     DevBuf<int64_t> scratch;
     // B workspace (per call)
     DevBuf<uint16_t> b_hi, b_lo; // b_lo (split only): lo then lo2 per B tile
-    DevBuf<float> part;          // split only: sums of (panel, 128 columns) that lie in several shares
+    DevBuf<float> part;          // sums of (panel, strip of columns) that lie in several shares
     int64_t b_n = 0;
     // FP8-B: per-column power-of-two scales (and their absmax scratch)
     DevBuf<float> b_scale;
     DevBuf<unsigned> b_amax;
-    // tensor maps of the pair kernel's copies (host copies, passed by value)
-    CUtensorMap map_a, map_b;
-    const void *map_a_base = nullptr, *map_b_base = nullptr;
-    uint64_t map_a_rows = 0, map_b_rows = 0;
 };
 
 void destroy_tc_plan(TcPlan *p) { delete p; }
@@ -102,6 +99,14 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// One lane of a converged warp, the same at every call
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
 {
     uint32_t r[32];
@@ -135,6 +140,30 @@ __device__ __forceinline__ void store_row32(float *out, const float (&v)[32], in
     }
 }
 
+// The same for a warp's 32 rows from C row `row`, columns from j, through a
+// 32 x kStageRow staging tile of its own: each store instruction writes four
+// rows' 128 contiguous bytes instead of 16 bytes of 32 rows. m, n: C's
+// extents (n a multiple of 4).
+constexpr int kStageRow = 36; // floats: 16-byte rows that a quarter warp writes without bank conflicts
+
+__device__ __forceinline__ void store_warp32(float *stage, const float (&v)[32], float *__restrict__ C, int64_t row,
+                                             int64_t j, int64_t m, int64_t n)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < 32; q += 4)
+        *reinterpret_cast<float4 *>(stage + lane * kStageRow + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+    __syncwarp();
+    const int r0 = lane >> 3, c = (lane & 7) * 4;
+#pragma unroll
+    for (int r = r0; r < 32; r += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(stage + r * kStageRow + c);
+        if (row + r < m && j + c < n)
+            *reinterpret_cast<float4 *>(C + (row + r) * n + j + c) = x;
+    }
+    __syncwarp(); // the tile is rewritten by the next call
+}
+
 // Byte offset of element (row r, column c) of a 32-byte-row K-major tile in
 // the 32B-swizzled layout.
 __host__ __device__ __forceinline__ uint32_t sw32_offset(uint32_t r, uint32_t c)
@@ -157,12 +186,15 @@ __global__ void tile_flags_kernel(const Entry *__restrict__ packed, const int32_
     }
 }
 
-__global__ void tile_list_kernel(const int32_t *__restrict__ pf, int64_t total, int64_t kb, int32_t *__restrict__ tile_cb)
+__global__ void tile_list_kernel(const int32_t *__restrict__ pf, int64_t total, int64_t kb, int32_t *__restrict__ tile_cb,
+                                 int32_t *__restrict__ tile_panel)
 {
     for (int64_t f = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; f < total;
          f += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        if (pf[f + 1] != pf[f])
+        if (pf[f + 1] != pf[f]) {
             tile_cb[pf[f]] = static_cast<int32_t>(f % kb);
+            tile_panel[pf[f]] = static_cast<int32_t>(f / kb);
+        }
 }
 
 // lo (split-BF16 only) is filled with 128-row panels.
@@ -295,9 +327,9 @@ b_tiles_kernel(const float *__restrict__ B, int64_t k, int64_t n, int64_t kb, __
 // w = jt * tiles + t and cut into equal consecutive shares, one per CTA, two
 // CTAs per SM: no wave of CTAs is nearly empty and a few panels fill the GPU.
 // Measured with 16 x 16 blocks at 25 % (us; a CTA per panel and 128 columns
-// before): 8192^2, n = 1024 458 -> 407 (the kernel 424 -> 362, 2.05 PFLOP/s of
-// MMAs, and 14 of fix-up), n = 128 216 -> 87; 2048 x 8192, n = 256 222 -> 58;
-// 2048^2, n = 1024 67 -> 52; 1024^2 at 15 %, n = 64 32 -> 28. A share is
+// before): 8192^2, n = 1024 458 -> 393 (the kernel 424 -> 352, 2.1 PFLOP/s of
+// MMAs, and 13 of fix-up), n = 128 216 -> 84; 2048 x 8192, n = 256 222 -> 57;
+// 2048^2, n = 1024 67 -> 49; 1024^2 at 15 %, n = 64 32 -> 24. A share is
 // walked panel by panel; a (panel, jt) that lies in one share is written to
 // C, the others' sums go to a workspace and tc_fixup_kernel adds them in
 // order. Every CTA's share and every place of the workspace follow from
@@ -312,20 +344,42 @@ constexpr int64_t kSplitMinTiles = 16; // tiles per CTA at least, where there ar
 constexpr int kPartFloats = kPanel * kSplitN;
 static_assert(2 * kSplitSmem <= 227 * 1024, "two CTAs per SM: 2 x 256 tensor-memory columns");
 
-__host__ __device__ __forceinline__ int64_t share_begin(int64_t work, int64_t ctas, int64_t g) { return work * g / ctas; }
+struct ShareCut {
+    int64_t work, shares, q, r; // the first r shares have q + 1 units, the others q
+    __host__ explicit ShareCut(int64_t work_ = 0, int64_t shares_ = 1)
+        : work(work_), shares(shares_), q(work_ / shares_), r(work_ % shares_)
+    {
+    }
+    __host__ __device__ __forceinline__ int64_t begin(int64_t g) const { return g * q + (g < r ? g : r); }
+    // the share of unit w < work
+    __host__ __device__ __forceinline__ int64_t of(int64_t w) const
+    {
+        const int64_t big = r * (q + 1);
+        return w < big ? w / (q + 1) : r + (w - big) / q;
+    }
+};
 
 // The consecutive pieces of a share: (panel, jt, tiles [t0, t1)), `first`: the
 // share starts with it; `whole`: all of the panel's tiles.
 struct ShareWalk {
-    const int32_t *pf;
-    int64_t kb, panels, tiles, w, end, begin;
+    const int32_t *pf, *tile_panel;
+    int64_t kb, tiles, w, end, begin;
     int64_t panel, jt, t0, t1;
     bool first, whole;
-    __device__ __forceinline__ ShareWalk(const int32_t *pf_, int64_t kb_, int64_t panels_, int64_t tiles_, int64_t work,
-                                         int64_t ctas, int64_t g)
-        : pf(pf_), kb(kb_), panels(panels_), tiles(tiles_), w(share_begin(work, ctas, g)),
-          end(share_begin(work, ctas, g + 1)), begin(w)
+    __device__ __forceinline__ ShareWalk(const int32_t *pf_, const int32_t *tile_panel_, int64_t kb_, int64_t tiles_,
+                                         const ShareCut &cut, int64_t g)
+        : pf(pf_), tile_panel(tile_panel_), kb(kb_), tiles(tiles_), w(cut.begin(g)), end(cut.begin(g + 1)), begin(w)
     {
+    }
+    // not a share: panel g % panels in strip g / panels, whole (maybe empty)
+    __device__ __forceinline__ ShareWalk(const int32_t *pf_, const int32_t *tile_panel_, int64_t kb_, int64_t tiles_,
+                                         int64_t panels, int64_t g)
+        : pf(pf_), tile_panel(tile_panel_), kb(kb_), tiles(tiles_)
+    {
+        jt = g / panels;
+        panel = g - jt * panels;
+        w = begin = jt * tiles + pf[panel * kb];
+        end = jt * tiles + pf[(panel + 1) * kb];
     }
     __device__ __forceinline__ bool next()
     {
@@ -334,15 +388,7 @@ struct ShareWalk {
         first = w == begin;
         jt = w / tiles;
         t0 = w - jt * tiles;
-        int64_t lo = 0, hi = panels; // the panel with pf[panel * kb] <= t0 < pf[(panel + 1) * kb]
-        while (hi - lo > 1) {
-            const int64_t mid = (lo + hi) / 2;
-            if (pf[mid * kb] <= t0)
-                lo = mid;
-            else
-                hi = mid;
-        }
-        panel = lo;
+        panel = tile_panel[t0];
         const int64_t p0 = pf[panel * kb], p1 = pf[(panel + 1) * kb];
         const int64_t left = end - w;
         t1 = p1 - t0 <= left ? p1 : t0 + left;
@@ -354,10 +400,11 @@ struct ShareWalk {
 
 __global__ void __launch_bounds__(kSplitThreads, 1)
 spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__ tile_cb,
+                     const int32_t *__restrict__ tile_panel,
                      const uint16_t *__restrict__ a_hi, const uint16_t *__restrict__ a_lo,
                      const uint16_t *__restrict__ b_hi, const uint16_t *__restrict__ b_lo, int64_t m, int64_t n,
-                     int64_t kb, int64_t panels, int64_t tiles, int64_t work, float *__restrict__ C,
-                     float *__restrict__ part, uint32_t *__restrict__ status)
+                     int64_t kb, int64_t tiles, const ShareCut cut, float *__restrict__ C, float *__restrict__ part,
+                     uint32_t *__restrict__ status)
 {
     constexpr int N = kSplitN, S = kSplitS;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -397,24 +444,29 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
     // products to bank 1, so each correction is rounded at its own (2^-8
     // smaller) magnitude, not at the running total's; the epilogue adds bank
     // 1 to bank 0.
-    ShareWalk sh(pf, kb, panels, tiles, work, gridDim.x, blockIdx.x);
+    ShareWalk sh(pf, tile_panel, kb, tiles, cut, blockIdx.x);
 
+    // Warps 4 and 5 walk together and one elected lane issues (a lane's own
+    // branch costs the descriptors' moves to uniform registers at each MMA)
     if (warp == 4) {
-        if (lane == 0) {
-            // copies: the ring runs on over the pieces
-            int64_t i = 0;
-            bool ok = true;
-            while (ok && sh.next()) {
-                for (int64_t tile = sh.t0; tile < sh.t1; ++tile, ++i) {
-                    const int s = static_cast<int>(i % S);
-                    if (*abort_flag || (i >= S && !mbar_wait(&empty[s], static_cast<uint32_t>(((i / S) - 1) & 1)))) {
+        // copies: the ring runs on over the pieces
+        int s = 0;
+        uint32_t phase = 1; // the first turn of the ring waits for nothing
+        bool ok = true;
+        while (ok && sh.next()) {
+            for (int64_t tile = sh.t0; tile < sh.t1; ++tile) {
+                const int64_t btile = sh.jt * kb + tile_cb[tile];
+                ok = mbar_wait(&empty[s], phase) && !*abort_flag;
+                ok = __all_sync(0xffffffffu, ok ? 1 : 0);
+                if (!ok) {
+                    if (lane == 0) {
                         atomicOr(status, kStatusWaitTimeout);
                         *abort_flag = 1;
-                        ok = false;
-                        break;
                     }
-                    unsigned char *st = stages + static_cast<size_t>(s) * kSplitStage;
-                    const int64_t btile = sh.jt * kb + tile_cb[tile];
+                    break;
+                }
+                unsigned char *st = stages + s * kSplitStage;
+                if (elect_one()) {
                     mbar_arrive_expect_tx(&full[s], kSplitStage);
                     bulk_g2s(st, a_hi + tile * (kTileBytes / 2), kTileBytes, &full[s]);
                     bulk_g2s(st + kSplitABytes, b_hi + btile * (N * 16), N * 32, &full[s]);
@@ -422,39 +474,39 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
                     bulk_g2s(st + kTileBytes, a_lo + tile * kTileBytes, 2 * kTileBytes, &full[s]);
                     bulk_g2s(st + kSplitABytes + N * 32, b_lo + btile * (N * 32), 2 * N * 32, &full[s]);
                 }
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1;
+                }
             }
         }
     } else if (warp == 5) {
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(kPanel, N);
-            int64_t i = 0;
-            uint32_t piece = 0;
-            bool ok = true;
-            while (ok && sh.next()) {
-                // the piece before this one has been read out
-                if (piece > 0 && !mbar_wait(drained, (piece - 1) & 1))
-                    ok = false;
+        const uint32_t idesc = idesc_bf16(kPanel, N);
+        int s = 0;
+        uint32_t phase = 0, piece = 0;
+        bool ok = true;
+        while (ok && sh.next()) {
+            // the piece before this one has been read out
+            if (piece > 0)
+                ok = __all_sync(0xffffffffu, mbar_wait(drained, (piece - 1) & 1) ? 1 : 0);
+            tc_fence_after();
+            for (int64_t tile = sh.t0; ok && tile < sh.t1; ++tile) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[s], phase) ? 1 : 0);
+                if (!ok)
+                    break;
                 tc_fence_after();
-                for (int64_t tile = sh.t0; ok && tile < sh.t1; ++tile, ++i) {
-                    const int s = static_cast<int>(i % S);
-                    if (!mbar_wait(&full[s], static_cast<uint32_t>((i / S) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t acc = tile > sh.t0 ? 1u : 0u;
-                    const uint32_t st = smem_u32(stages + static_cast<size_t>(s) * kSplitStage);
-                    const uint64_t ah = smem_desc_sw32(st);
-                    const uint64_t bh = smem_desc_sw32(st + kSplitABytes);
+                const uint32_t acc = tile > sh.t0 ? 1u : 0u;
+                const uint64_t ah = smem_desc_sw32(smem_u32(stages + s * kSplitStage));
+                if (elect_one()) {
+                    const uint64_t bh = ah + (kSplitABytes >> 4);
                     tc_mma(tmem, ah, bh, idesc, acc);
                     // (ah + al + al2)(bh + bl + bl2): every product above 2^-24
                     // of the leading one (al * bl2, al2 * bl, al2 * bl2 dropped),
                     // into the correction bank
                     const uint32_t dx = tmem + static_cast<uint32_t>(N);
-                    const uint64_t al = smem_desc_sw32(st + kTileBytes);
-                    const uint64_t al2 = smem_desc_sw32(st + 2 * kTileBytes);
-                    const uint64_t bl = smem_desc_sw32(st + kSplitABytes + N * 32);
-                    const uint64_t bl2 = smem_desc_sw32(st + kSplitABytes + 2 * N * 32);
+                    const uint64_t al = ah + (kTileBytes >> 4), al2 = ah + (2 * kTileBytes >> 4);
+                    const uint64_t bl = bh + (N * 32 >> 4), bl2 = bh + (2 * N * 32 >> 4);
                     tc_mma(dx, ah, bl, idesc, acc);
                     tc_mma(dx, al, bh, idesc, 1u);
                     tc_mma(dx, al, bl, idesc, 1u);
@@ -462,13 +514,20 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
                     tc_mma(dx, al2, bh, idesc, 1u);
                     tc_commit(&empty[s]); // slot reusable once these MMAs have read it
                 }
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1;
+                }
+            }
+            if (elect_one())
                 tc_commit(done); // arrives when every MMA issued above has completed
-                ++piece;
-            }
-            if (!ok) {
-                atomicOr(status, kStatusWaitTimeout);
-                *abort_flag = 1;
-            }
+            __syncwarp();
+            ++piece;
+        }
+        if (!ok && lane == 0) {
+            atomicOr(status, kStatusWaitTimeout);
+            *abort_flag = 1;
         }
     } else {
         // epilogue: warp w owns TMEM lanes 32w..32w+31 = panel rows
@@ -527,32 +586,30 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
     }
 }
 
-// C of the (panel, 128 columns) whose tiles lie in several shares (their
-// parts added in order) or that have none (zeros). One thread per row, 32 of
-// the columns per CTA.
-__global__ void __launch_bounds__(kPanel)
-tc_fixup_kernel(const int32_t *__restrict__ pf, int64_t m, int64_t n, int64_t kb, int64_t tiles, int64_t work,
-                int64_t ctas, const float *__restrict__ part, float *__restrict__ C)
+// C of the (panel of `blockDim.x` rows, strip of `cols` columns) whose tiles
+// lie in several shares (their parts added in order) or that have none
+// (zeros). One thread per row, 32 of the columns per CTA.
+__global__ void __launch_bounds__(2 * kPanel)
+tc_fixup_kernel(const int32_t *__restrict__ pf, int64_t m, int64_t n, int64_t kb, int64_t tiles, const ShareCut cut,
+                int cols, const float *__restrict__ part, float *__restrict__ C)
 {
+    __shared__ __align__(16) float staging[2 * kPanel * kStageRow];
+    const int R = blockDim.x;
     const int64_t panel = blockIdx.x, jt = blockIdx.y;
+    const int c = blockIdx.z * 32;
+    const int64_t j = jt * cols + c;
+    if (j >= n)
+        return;
     const int64_t p0 = pf[panel * kb], p1 = pf[(panel + 1) * kb];
-    const int64_t row = panel * kPanel + threadIdx.x;
     const int64_t w0 = jt * tiles + p0, w1 = jt * tiles + p1;
     int64_t g0 = 0, g1 = -1; // the shares with tiles of it
     if (p1 > p0) {
-        // share g holds w where share_begin(g) <= w < share_begin(g + 1)
-        g0 = w0 * ctas / work;
-        while (g0 > 0 && share_begin(work, ctas, g0) > w0)
-            --g0;
-        while (share_begin(work, ctas, g0 + 1) <= w0)
-            ++g0;
-        g1 = g0;
-        while (share_begin(work, ctas, g1 + 1) < w1)
-            ++g1;
-        if (g1 == g0)
+        g0 = cut.of(w0);
+        if (cut.begin(g0 + 1) >= w1)
             return; // in one share: written there
+        g1 = cut.of(w1 - 1);
     }
-    const int c = blockIdx.z * 32;
+    const int64_t part_floats = static_cast<int64_t>(R) * cols;
     float v[32];
 #pragma unroll
     for (int q = 0; q < 32; ++q)
@@ -560,13 +617,13 @@ tc_fixup_kernel(const int32_t *__restrict__ pf, int64_t m, int64_t n, int64_t kb
     for (int64_t g = g0; g <= g1; g += 2) { // two parts' loads in flight together
         float x[32], y[32];
         // a share's first piece starts where the share does
-        const float *sx = part + (2 * g + (share_begin(work, ctas, g) >= w0 ? 0 : 1)) * kPartFloats + c * kPanel + threadIdx.x;
-        const float *sy = part + 2 * (g + 1) * kPartFloats + c * kPanel + threadIdx.x; // never the panel's first share
+        const float *sx = part + (2 * g + (cut.begin(g) >= w0 ? 0 : 1)) * part_floats + c * R + threadIdx.x;
+        const float *sy = part + 2 * (g + 1) * part_floats + c * R + threadIdx.x; // the share's first piece
         const bool two = g < g1;
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
-            x[q] = sx[q * kPanel];
-            y[q] = two ? sy[q * kPanel] : 0.0f;
+            x[q] = sx[q * R];
+            y[q] = two ? sy[q * R] : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
@@ -575,9 +632,8 @@ tc_fixup_kernel(const int32_t *__restrict__ pf, int64_t m, int64_t n, int64_t kb
                 v[q] += y[q];
         }
     }
-    const int64_t j = jt * kSplitN + c;
-    if (row < m && j < n)
-        store_row32(C + row * n + j, v, n - j);
+    const int warp = threadIdx.x >> 5;
+    store_warp32(staging + warp * (32 * kStageRow), v, C, panel * R + warp * 32, j, m, n);
 }
 
 // ---- the pair kernel (BF16, FP8-B) ----------------------------------------------------
@@ -601,13 +657,30 @@ __device__ __forceinline__ void cluster_sync_all()
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// One box of a 2-D tensor map into this CTA's shared memory, completing on an
-// mbarrier in either CTA of the pair.
-__device__ __forceinline__ void tma_2d_pair(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar)
+// Arrives on an mbarrier of either CTA of the pair (a shared::cluster address)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr)
 {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-                 " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+
+__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
+
+// One box of a 3-D / 4-D tensor map into this CTA's shared memory, completing
+// on an mbarrier in either CTA of the pair.
+__device__ __forceinline__ void tma_3d_pair(uint32_t dst, const CUtensorMap *map, int32_t y, int32_t z, uint32_t mbar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(z), "r"(mbar)
+                 : "memory");
+}
+
+__device__ __forceinline__ void tma_4d_pair(uint32_t dst, const CUtensorMap *map, int32_t y, int32_t z, int32_t w,
+                                            uint32_t mbar)
+{
+    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(z), "r"(w), "r"(mbar)
                  : "memory");
 }
 
@@ -629,59 +702,99 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t *bar)
 
 constexpr int kPairN = 256;                // output columns per accumulator (MMA N)
 constexpr int kPairMaxNT = 2;              // accumulators per CTA: all 512 tensor-memory columns
-constexpr int kPairK = 8;                  // tiles per stage (4 x 4 stages: 3 % slower; 2 x 8: 12 %)
+constexpr int kPairK = 4;                  // tiles per stage
 constexpr int kPairHalf = kTileBytes;      // 4 KB: a tile's 128-row half, or a B tile's 128-column half
-constexpr int kPairStage = (1 + kPairMaxNT) * kPairK * kPairHalf; // [A halves][B halves, accumulator 0][... 1]
-constexpr int kPairS = 2;                  // stages of 96 KB: 194 KB, so one CTA per SM
-constexpr int kPairSmem = 1024 + kPairS * kPairStage + 1024;
+// A stage holds the A halves of kPairK tiles, then per tile its B half of
+// each accumulator: 32 KB or 48 KB, and the ring as many as fit 192 KB (with
+// the one CTA per SM that the tensor memory allows).
+constexpr int kPairRing = 192 * 1024;
+constexpr int kPairMaxS = kPairRing / (2 * kPairK * kPairHalf);
+constexpr int kPairStaging = 4 * 32 * kStageRow * 4; // the epilogue warps' staging tiles
+constexpr int kPairSmem = 1024 + kPairRing + kPairStaging + 1024;
+__host__ __device__ constexpr int pair_stages(int nt) { return kPairRing / ((1 + nt) * kPairK * kPairHalf); }
 static_assert(kPairSmem <= 227 * 1024 && 2 * kPairSmem > 228 * 1024,
               "one pair CTA per SM: its tensor-memory allocation never waits for another");
 
-// One cluster of two CTAs per (256-row panel, nt * 256 output columns). CTA
-// `rank` holds rows [128 rank, 128 rank + 128) of the panel: per stage its
-// halves of up to kPairK of the panel's tiles and the matching 128-column
-// halves of the B tiles, copied by its warp 0 with tensor-map bulk copies
-// that complete on the first CTA's `full` barrier (which expects both CTAs'
-// bytes). Warp 1 of the first CTA issues, per tile and accumulator, one
-// tcgen05.mma.cta_group::2 (M=256, N=256, K=16) reading both CTAs' shared
-// memory, and tcgen05.commit frees the slot in both CTAs. Each CTA drains
-// its 128 rows of the accumulators from its own tensor memory.
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1)
-spdm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                    const int32_t *__restrict__ pf, const int32_t *__restrict__ tile_cb, int64_t m, int64_t n,
-                    int64_t kb, int nt_cta, float *__restrict__ C, uint32_t *__restrict__ status)
+// The MMAs of a stage's nq tiles into NT accumulators (of a strip's last
+// column tile past n: the map's zeros). One thread's issue rate bounds the
+// kernel, so the tiles are unrolled and a descriptor is one addition.
+template <int NT>
+__device__ __forceinline__ void pair_stage_mmas(uint32_t tmem, uint32_t st, uint32_t idesc, int nq, uint32_t acc)
 {
-    constexpr int N = kPairN, S = kPairS;
+    const uint64_t da = smem_desc_sw32(st), db = smem_desc_sw32(st + kPairK * kPairHalf);
+#pragma unroll
+    for (int q = 0; q < kPairK; ++q) {
+        if (q >= nq)
+            break;
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+            tc_mma_pair(tmem + static_cast<uint32_t>(t * kPairN), da + static_cast<uint64_t>(q * kPairHalf >> 4),
+                        db + static_cast<uint64_t>((q * NT + t) * kPairHalf >> 4), idesc, q > 0 ? 1u : acc);
+    }
+}
+
+// A cluster of two CTAs per (256-row panel, nt * 256 output columns), or, with
+// `shares`, per equal share of the (tile, 256 columns) products (a panel's
+// parts go to the workspace, see the split kernel). CTA `rank` holds rows
+// [128 rank, 128 rank + 128) of the panel: per stage its halves of up to
+// kPairK of the panel's tiles and the matching 128-column halves of the B
+// tiles, copied by its warp 4 with tensor-map bulk copies that complete on
+// the first CTA's `full` barrier (which expects both CTAs' bytes). Warp 5 of
+// the first CTA issues, per tile and accumulator, one
+// tcgen05.mma.cta_group::2 (M=256, N=256, K=16) reading both CTAs' shared
+// memory, and tcgen05.commit frees the slot in both CTAs. Warps 0-3 of each
+// CTA drain its 128 rows of the accumulators from its own tensor memory.
+//
+// The MMAs bound it (8192^2 of 16 x 16 blocks at 25 %, n = 1024: 68 us at the
+// peak rate of 128 SMs, 83 measured, 125 before), as long as one thread can
+// issue them: a loop over run-time counts that built each descriptor took
+// ~155 cycles per 128-cycle MMA and ~300 per stage, which is why an elected
+// lane runs them unrolled, and a copy per tile and operand ~85 ns each, which
+// is why one box carries A's stage and a lane each B's tiles. 4 tiles per
+// stage and the ring as deep as 192 KB: 8 per stage is 5 % slower at two
+// accumulators (and 5 % faster at one). C leaves through a staging tile, four
+// rows' 128 bytes per store: 3 us of the 83 less than 16 bytes of 32 rows.
+constexpr int kPairThreads = 192;
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+spdm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
+                    const int32_t *__restrict__ pf, const int32_t *__restrict__ tile_cb,
+                    const int32_t *__restrict__ tile_panel, int64_t m, int64_t n, int64_t kb, int64_t panels,
+                    int64_t tiles, const ShareCut cut, bool shares, int nt_cta,
+                    float *__restrict__ C, float *__restrict__ part, uint32_t *__restrict__ status)
+{
+    constexpr int N = kPairN;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // the same carve in both CTAs: the MMA reads the second CTA's operands at the first's offsets
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(base);
-    uint64_t *empty = full + S;
-    uint64_t *done = empty + S;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
+    uint64_t *empty = full + kPairMaxS;
+    uint64_t *done = empty + kPairMaxS; // [bank]: a piece's MMAs have completed
+    uint64_t *drained = done + 2;       // [bank] (first CTA's): both CTAs have read a piece's sums
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 2);
     unsigned char *stages = base + 1024;
+    float *staging = reinterpret_cast<float *>(stages + kPairRing);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
-    const int64_t panel = blockIdx.x >> 1;
-    const int64_t jt = blockIdx.y; // nt_cta accumulators of 256 columns
-    const int64_t t0 = pf[panel * kb];
-    const int64_t ntiles = pf[(panel + 1) * kb] - t0;
-    const int64_t nstages = (ntiles + kPairK - 1) / kPairK;
+    const int64_t pair = blockIdx.x >> 1;
+    const int S = pair_stages(nt_cta), stage_bytes = (1 + nt_cta) * kPairK * kPairHalf;
     const int64_t ntn = (n + N - 1) / N;
-    const int nt = static_cast<int>(ntn - jt * nt_cta < nt_cta ? ntn - jt * nt_cta : nt_cta);
     bool gave_up = false;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S; ++s) {
+        for (int s = 0; s < kPairMaxS; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(done, 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&done[b], 1);
+            mbar_init(&drained[b], 8); // one arrival per epilogue warp of the two CTAs
+        }
         fence_mbar_init();
     }
-    if (warp == 2) {
+    if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(kPairMaxNT * N)
                      : "memory");
@@ -691,90 +804,159 @@ spdm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     cluster_sync_all(); // both CTAs' barriers initialised and tensor memory allocated
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    ShareWalk sh = shares ? ShareWalk(pf, tile_panel, kb, tiles, cut, pair)
+                          : ShareWalk(pf, tile_panel, kb, tiles, panels, pair);
+    // with one accumulator a piece's sums are drained while the next piece's
+    // products go to the other half of the tensor memory
+    const uint32_t bank_mask = nt_cta == 1 ? 1u : 0u;
+    // accumulators of a strip of columns
+    const auto strip_nt = [&](int64_t jt) { return static_cast<int>(ntn - jt * nt_cta < nt_cta ? ntn - jt * nt_cta : nt_cta); };
 
-    if (ntiles > 0) {
-        if (warp == 0 && lane == 0) {
-            // producer (both CTAs)
-            for (int64_t i = 0; i < nstages; ++i) {
-                const int s = static_cast<int>(i % S);
-                if (i >= S && !mbar_wait(&empty[s], static_cast<uint32_t>(((i / S) - 1) & 1))) {
-                    atomicOr(status, kStatusWaitTimeout);
+    if (warp == 4) {
+        // copies (both CTAs); the ring runs on over the pieces. Lane 0 copies
+        // the A halves of a stage's tiles (one box), lane q the B halves of
+        // tile q (one box for all accumulators), so that no lane waits for
+        // another tile's column block.
+        int s = 0;
+        uint32_t phase = 1; // the first turn of the ring waits for nothing
+        while (!gave_up && sh.next()) {
+            // read a stage ahead
+            int32_t cb = 0, cb_next = lane < kPairK && lane < sh.t1 - sh.t0 ? tile_cb[sh.t0 + lane] : 0;
+            for (int64_t q0 = sh.t0; q0 < sh.t1; q0 += kPairK) {
+                const int nq = sh.t1 - q0 < kPairK ? static_cast<int>(sh.t1 - q0) : kPairK;
+                cb = cb_next;
+                if (lane < kPairK && q0 + kPairK + lane < sh.t1)
+                    cb_next = tile_cb[q0 + kPairK + lane];
+                const bool ok = mbar_wait(&empty[s], phase);
+                if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
+                    if (lane == 0)
+                        atomicOr(status, kStatusWaitTimeout);
                     gave_up = true;
                     break;
                 }
-                const int64_t q0 = i * kPairK;
-                const int nq = ntiles - q0 < kPairK ? static_cast<int>(ntiles - q0) : kPairK;
-                if (rank == 0) // both CTAs' bytes
-                    mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(2 * (1 + nt) * nq * kPairHalf));
-                const uint32_t st = smem_u32(stages + static_cast<size_t>(s) * kPairStage);
+                const uint32_t st = smem_u32(stages + s * stage_bytes);
                 const uint32_t leader_full = mapa_rank(smem_u32(&full[s]), 0);
-                for (int q = 0; q < nq; ++q) {
-                    const int64_t tile = t0 + q0 + q;
-                    const int64_t cb = tile_cb[tile];
-                    // maps in rows of 512 B: a tile is 16 rows, a half 8
-                    tma_2d_pair(st + q * kPairHalf, &tm_a, 0, static_cast<int32_t>(tile * 16 + rank * 8), leader_full);
-                    for (int t = 0; t < nt; ++t)
-                        tma_2d_pair(st + ((1 + t) * kPairK + q) * kPairHalf, &tm_b, 0,
-                                    static_cast<int32_t>(((jt * nt_cta + t) * kb + cb) * 16 + rank * 8), leader_full);
+                if (lane == 0) {
+                    if (rank == 0) // both CTAs' bytes; boxes count whole, also past the maps' ends
+                        mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(2 * (kPairK + nq * nt_cta) * kPairHalf));
+                    tma_3d_pair(st, &tm_a, static_cast<int32_t>(rank * 8), static_cast<int32_t>(q0), leader_full);
+                }
+                __syncwarp();
+                if (lane < nq)
+                    tma_4d_pair(st + (kPairK + lane * nt_cta) * kPairHalf, &tm_b, static_cast<int32_t>(rank * 8), cb,
+                                static_cast<int32_t>(sh.jt * nt_cta), leader_full);
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1;
                 }
             }
-        } else if (warp == 1 && lane == 0 && rank == 0) {
-            // MMA issuer (first CTA only)
-            const uint32_t idesc = idesc_bf16(2 * kPanel, N);
-            for (int64_t i = 0; i < nstages; ++i) {
-                const int s = static_cast<int>(i % S);
-                if (!mbar_wait(&full[s], static_cast<uint32_t>((i / S) & 1))) {
-                    atomicOr(status, kStatusWaitTimeout);
-                    gave_up = true;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t st = smem_u32(stages + static_cast<size_t>(s) * kPairStage);
-                const int64_t q0 = i * kPairK;
-                const int nq = ntiles - q0 < kPairK ? static_cast<int>(ntiles - q0) : kPairK;
-                for (int q = 0; q < nq; ++q)
-                    for (int t = 0; t < nt; ++t)
-                        tc_mma_pair(tmem + static_cast<uint32_t>(t * N), smem_desc_sw32(st + q * kPairHalf),
-                                    smem_desc_sw32(st + ((1 + t) * kPairK + q) * kPairHalf), idesc,
-                                    (i > 0 || q > 0) ? 1u : 0u);
-                tc_commit_pair(&empty[s]); // the slot is free in both CTAs once these MMAs have read it
-            }
-            tc_commit_pair(done); // arrives in both CTAs when every MMA issued above has completed
         }
-        __syncwarp();
-        const bool ok = mbar_wait(done, 0);
-        if (!ok && lane == 0)
-            atomicOr(status, kStatusWaitTimeout);
-        tc_fence_after();
-        const int64_t row = panel * (2 * kPanel) + rank * kPanel + warp * 32 + lane;
-        if (__all_sync(0xffffffffu, ok ? 1 : 0)) {
+    } else if (warp == 5) {
+        if (rank == 0) {
+            // MMA issuer (first CTA only): the warp walks together and one
+            // elected lane issues a stage's MMAs, unrolled, descriptors
+            // advanced by constants
+            const uint32_t idesc = idesc_bf16(2 * kPanel, N);
+            int s = 0;
+            uint32_t phase = 0, piece = 0;
+            while (!gave_up && sh.next()) {
+                const uint32_t bank = piece & bank_mask, turn = piece >> bank_mask;
+                const uint32_t acc0 = tmem + bank * N;
+                if (turn > 0) {
+                    const bool ok = mbar_wait(&drained[bank], (turn - 1) & 1);
+                    if (!__all_sync(0xffffffffu, ok ? 1 : 0))
+                        gave_up = true;
+                    fence_cluster(); // the other CTA's arrivals
+                }
+                for (int64_t q0 = sh.t0; !gave_up && q0 < sh.t1; q0 += kPairK) {
+                    const bool ok = mbar_wait(&full[s], phase);
+                    if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
+                        gave_up = true;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t st = smem_u32(stages + s * stage_bytes);
+                    const int nq = sh.t1 - q0 < kPairK ? static_cast<int>(sh.t1 - q0) : kPairK;
+                    const uint32_t acc = q0 > sh.t0 ? 1u : 0u;
+                    if (elect_one()) {
+                        if (nt_cta == 2)
+                            pair_stage_mmas<2>(acc0, st, idesc, nq, acc);
+                        else
+                            pair_stage_mmas<1>(acc0, st, idesc, nq, acc);
+                        tc_commit_pair(&empty[s]); // the slot is free in both CTAs once these MMAs have read it
+                    }
+                    __syncwarp();
+                    if (++s == S) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+                if (elect_one())
+                    tc_commit_pair(&done[bank]); // arrives in both CTAs when every MMA issued above has completed
+                __syncwarp();
+                ++piece;
+            }
+            if (gave_up && lane == 0)
+                atomicOr(status, kStatusWaitTimeout);
+        }
+    } else {
+        uint32_t piece = 0;
+        const int lr = static_cast<int>(rank) * kPanel + warp * 32 + lane;
+        if (!shares && sh.w == sh.end) {
+            // panel without entries: its C rows are zero
+            const int64_t row = sh.panel * (2 * kPanel) + lr;
+            if (row < m)
+                for (int64_t j = sh.jt * nt_cta * N; j < (sh.jt + 1) * nt_cta * N && j < n; ++j)
+                    C[row * n + j] = 0.0f;
+        }
+        while (sh.next()) {
+            const int nt = strip_nt(sh.jt);
+            const uint32_t bank = piece & bank_mask, turn = piece >> bank_mask;
+            const bool ok = mbar_wait(&done[bank], turn & 1);
+            if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
+                if (lane == 0)
+                    atomicOr(status, kStatusWaitTimeout);
+                gave_up = true;
+                break;
+            }
+            tc_fence_after();
+            const int64_t row = sh.panel * (2 * kPanel) + lr;
+            float *slot = part + (2 * pair + (sh.first ? 0 : 1)) * static_cast<int64_t>(2 * kPanel) * nt_cta * N;
 #pragma unroll 1
             for (int c = 0; c < nt * N; c += 32) {
                 float v[32];
-                tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c), v);
-                const int64_t j = jt * nt_cta * N + c;
-                if (row < m && j < n)
-                    store_row32(C + row * n + j, v, n - j);
+                tmem_ld32(tmem + bank * N + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c), v);
+                const int64_t j = sh.jt * nt_cta * N + c;
+                if (!sh.whole) { // [column][row]: contiguous across the warp
+                    if (j < n) {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q)
+                            slot[(c + q) * (2 * kPanel) + lr] = v[q];
+                    }
+                } else {
+                    store_warp32(staging + warp * (32 * kStageRow), v, C, row - lane, j, m, n);
+                }
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive_cluster(mapa_rank(smem_u32(&drained[bank]), 0));
+            ++piece;
         }
-    } else {
-        // panel without entries: its C rows are zero
-        const int64_t row = panel * (2 * kPanel) + rank * kPanel + warp * 32 + lane;
-        if (row < m)
-            for (int64_t j = jt * nt_cta * N; j < (jt + 1) * nt_cta * N && j < n; ++j)
-                C[row * n + j] = 0.0f;
     }
+    __syncwarp(); // warps 4 and 5: their one working lane is back
     // after a wait gave up (in either CTA: the status word), copies already
     // issued may still be landing in this CTA or signalling the first CTA's
     // barriers: give them a bounded time before the pair leaves
-    if (threadIdx.x == 0 && (gave_up || (*reinterpret_cast<volatile uint32_t *>(status) & kStatusWaitTimeout))) {
+    if (lane == 0 && (gave_up || (*reinterpret_cast<volatile uint32_t *>(status) & kStatusWaitTimeout))) {
         const uint64_t t_end = global_ns() + kDrainNs;
         while (global_ns() < t_end)
             __nanosleep(10000);
     }
+    __syncwarp();
     tc_fence_before();
     cluster_sync_all(); // neither CTA leaves while the pair's MMAs or copies may touch it
-    if (warp == 2) {
+    if (warp == 5) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kPairMaxNT * N)
                      : "memory");
@@ -807,61 +989,86 @@ EncodeTiledFn encode_tiled_fn()
     return fn;
 }
 
-// A buffer of swizzled tiles as a 2-D map of 512-byte rows (256 bf16),
-// boxes of 8 rows: one box is one contiguous 4 KB half. The bytes are
-// already in the MMA's shared-memory layout, so the copy is unswizzled.
-// `halves` counts the buffer's 4 KB halves.
-bool encode_halves_map(CUtensorMap *map, const void *base, uint64_t halves)
+// A map of a buffer of tiles. Their bytes are already in the MMA's
+// shared-memory layout, so the copies are unswizzled.
+bool encode_map(CUtensorMap *map, const void *base, cuuint32_t rank, const cuuint64_t (&dims)[4],
+                const cuuint64_t (&strides)[3], const cuuint32_t (&box)[4])
 {
     EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn || halves == 0)
+    if (!fn)
         return false;
-    const cuuint64_t dims[2] = {256, halves * 8};
-    const cuuint64_t strides[1] = {512};
-    const cuuint32_t box[2] = {256, 8};
-    const cuuint32_t elem_strides[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, elem_strides,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    const cuuint32_t elem[4] = {1, 1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, rank, const_cast<void *>(base), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Accumulators per CTA: two (each A half then feeds two MMAs) unless one per
-// CTA still leaves the grid within one wave of one CTA per SM.
-int pair_accumulators(int64_t panels, int64_t ntn)
+// How a BF16 / FP8-B multiply of `ntn` 256-column tiles is cut over the GPU's
+// pairs of SMs. Whole: a pair per (panel, strip of one or two accumulators:
+// two, each A half then feeding two MMAs, unless one per pair still leaves
+// the grid within one wave). Shares: equal parts of the products with one
+// accumulator, one per pair, where their estimate is shorter, in MMA times of
+// one tile: a product of a share costs kPairShareRate (its A half feeds one
+// MMA), and the exposed last drain with the fix-up kPairShareCost. Measured,
+// 16 x 16 blocks, whole / shares: 8192^2 at 25 %, n = 128 68 / 50 us, n = 512
+// 72 / 80, n = 1024 94 / 125; 10240 x 8192 at 25 %, n = 1024 (80 units on 76
+// pairs) 172 / 147; 2048 x 8192 at 25 %, n = 256 63 / 35; 1024 x 16384 at 10 %,
+// n = 1024 110 / 61; 4096^2, n = 256 38 / 32; 2048^2, n = 1024 28 / 33;
+// 12288 x 4096, n = 1024 102 / 105; 4096^2, n = 2048 61 / 84.
+struct PairCut {
+    int64_t pairs;
+    int nt;
+    bool shares;
+};
+constexpr double kPairShareRate = 1.45, kPairShareCost = 150.0;
+constexpr int64_t kPairShareCols = 128; // column tiles at most: beyond, whole units fill the waves
+
+PairCut pair_cut(int64_t panels, int64_t tiles, int64_t ntn)
 {
-    const int64_t pairs = static_cast<int64_t>(device_sms()) / 2;
-    return panels * ntn <= pairs ? 1 : kPairMaxNT;
+    const int64_t slots = static_cast<int64_t>(device_sms()) / 2;
+    const int nt_whole = panels * ntn <= slots ? 1 : kPairMaxNT;
+    const int64_t units = panels * ((ntn + nt_whole - 1) / nt_whole);
+    const int64_t work = tiles * ntn;
+    // in tiles of one accumulator
+    const double whole = static_cast<double>((units + slots - 1) / slots) * nt_whole * tiles / (panels > 0 ? panels : 1);
+    const double share = kPairShareRate * static_cast<double>(work) / slots + kPairShareCost;
+    if (share < whole && work >= slots * kPairK && ntn <= kPairShareCols)
+        return PairCut{slots, 1, true};
+    return PairCut{units, nt_whole, false};
 }
 
 cudaError_t launch_pair(TcPlan &p, int64_t m, int64_t n, float *C, uint32_t *status, cudaStream_t st)
 {
     const int64_t ntn = (n + kPairN - 1) / kPairN;
-    const uint64_t a_halves = static_cast<uint64_t>(p.tiles) * 2, b_halves = static_cast<uint64_t>(ntn * p.kb) * 2;
-    if (p.map_a_base != p.a_hi.ptr || p.map_a_rows != a_halves) {
-        if (!encode_halves_map(&p.map_a, p.a_hi.ptr, a_halves))
-            return cudaErrorInvalidValue;
-        p.map_a_base = p.a_hi.ptr;
-        p.map_a_rows = a_halves;
-    }
-    if (p.map_b_base != p.b_hi.ptr || p.map_b_rows != b_halves) {
-        if (!encode_halves_map(&p.map_b, p.b_hi.ptr, b_halves))
-            return cudaErrorInvalidValue;
-        p.map_b_base = p.b_hi.ptr;
-        p.map_b_rows = b_halves;
-    }
-    // y coordinates of the maps are int32
-    if (static_cast<int64_t>(a_halves * 8) > 0x7fffffffLL || static_cast<int64_t>(b_halves * 8) > 0x7fffffffLL)
+    const PairCut cut = pair_cut(p.panels, p.tiles, ntn);
+    // a tile: 16 rows of 512 B, 8 per half. A: (512 B, row, tile), boxes of a
+    // half of kPairK tiles; B: (512 B, row, column block, 256-column tile),
+    // boxes of a half of one column block in cut.nt column tiles. Boxes past
+    // the last tile are filled with zeros there.
+    const cuuint64_t tiles = static_cast<cuuint64_t>(p.tiles > 0 ? p.tiles : 1);
+    if (tiles > 0x7fffffffULL || p.kb > 0x7fffffffLL)
+        return cudaErrorInvalidValue; // int32 coordinates
+    CUtensorMap map_a, map_b; // passed by value
+    if (!encode_map(&map_a, p.a_hi.ptr, 3, {256, 16, tiles, 1}, {512, 8192, 0}, {256, 8, kPairK, 1}) ||
+        !encode_map(&map_b, p.b_hi.ptr, 4, {256, 16, static_cast<cuuint64_t>(p.kb), static_cast<cuuint64_t>(ntn)},
+                    {512, 8192, 8192 * static_cast<cuuint64_t>(p.kb)}, {256, 8, 1, static_cast<cuuint32_t>(cut.nt)}))
         return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(spdm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
     if (e != cudaSuccess)
         return e;
-    const int nt_cta = pair_accumulators(p.panels, ntn);
-    const int64_t gy = (ntn + nt_cta - 1) / nt_cta;
-    if (2 * p.panels > 0x7fffffffLL || gy > 65535)
+    const int64_t strips = (ntn + cut.nt - 1) / cut.nt;
+    const ShareCut shares(p.tiles * strips, cut.pairs > 0 ? cut.pairs : 1);
+    if (2 * p.panels > 0x7fffffffLL || strips > 65535 || 2 * cut.pairs > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    dim3 grid(static_cast<unsigned>(2 * p.panels), static_cast<unsigned>(gy));
-    spdm_tc_pair_kernel<<<grid, 128, kPairSmem, st>>>(p.map_a, p.map_b, p.pf.ptr, p.tile_cb.ptr, m, n, p.kb, nt_cta, C,
-                                                      status);
+    spdm_tc_pair_kernel<<<static_cast<unsigned>(2 * cut.pairs), kPairThreads, kPairSmem, st>>>(
+        map_a, map_b, p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, m, n, p.kb, p.panels, p.tiles, shares, cut.shares, cut.nt,
+        C, p.part.ptr, status);
+    if (cut.shares) {
+        const int cols = cut.nt * kPairN;
+        const dim3 grid(static_cast<unsigned>(p.panels), static_cast<unsigned>(strips), static_cast<unsigned>(cols / 32));
+        tc_fixup_kernel<<<grid, 2 * kPanel, 0, st>>>(p.pf.ptr, m, n, p.kb, p.tiles, shares, cols, p.part.ptr, C);
+        count_launches(1);
+    }
     count_launches(1);
     return cudaGetLastError();
 }
@@ -877,6 +1084,7 @@ int64_t split_ctas(int64_t work)
 cudaError_t launch_split(const TcPlan &p, int64_t m, int64_t n, float *C, uint32_t *status, cudaStream_t st)
 {
     const int64_t njt = (n + kSplitN - 1) / kSplitN, work = p.tiles * njt, ctas = split_ctas(work);
+    const ShareCut cut(work, ctas);
     if (njt > 65535 || p.panels > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
     if (work > 0) {
@@ -884,12 +1092,12 @@ cudaError_t launch_split(const TcPlan &p, int64_t m, int64_t n, float *C, uint32
         if (e != cudaSuccess)
             return e;
         spdm_tc_split_kernel<<<static_cast<unsigned>(ctas), kSplitThreads, kSplitSmem, st>>>(
-            p.pf.ptr, p.tile_cb.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n, p.kb, p.panels, p.tiles, work,
-            C, p.part.ptr, status);
+            p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n, p.kb, p.tiles,
+            cut, C, p.part.ptr, status);
         count_launches(1);
     }
     const dim3 grid(static_cast<unsigned>(p.panels), static_cast<unsigned>(njt), kSplitN / 32);
-    tc_fixup_kernel<<<grid, kPanel, 0, st>>>(p.pf.ptr, m, n, p.kb, p.tiles, work, ctas, p.part.ptr, C);
+    tc_fixup_kernel<<<grid, kPanel, 0, st>>>(p.pf.ptr, m, n, p.kb, p.tiles, cut, kSplitN, p.part.ptr, C);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -926,12 +1134,12 @@ gcoo_status tc_build_plan(gcoo_handle *h, bool split, cudaStream_t st)
     GCOO_CUDA(cudaStreamSynchronize(st));
     p.tiles = total;
     const size_t tile_elems = static_cast<size_t>(p.panel_rows / kPanel) * (kTileBytes / 2);
-    if (!p.tile_cb.ensure(total + 1) || !p.a_hi.ensure(total * tile_elems + 1) ||
+    if (!p.tile_cb.ensure(total + 1) || !p.tile_panel.ensure(total + 1) || !p.a_hi.ensure(total * tile_elems + 1) ||
         (split && !p.a_lo.ensure(2 * total * tile_elems + 1)))
         return fail(GCOO_ERROR_ALLOC, "device allocation of the dense tiles failed");
     if (total > 0) {
-        tile_list_kernel<<<static_cast<unsigned>(std::min<int64_t>((L + 255) / 256, 4096)), 256, 0, st>>>(p.pf.ptr, L,
-                                                                                                          p.kb, p.tile_cb.ptr);
+        tile_list_kernel<<<static_cast<unsigned>(std::min<int64_t>((L + 255) / 256, 4096)), 256, 0, st>>>(
+            p.pf.ptr, L, p.kb, p.tile_cb.ptr, p.tile_panel.ptr);
         GCOO_CUDA(cudaMemsetAsync(p.a_hi.ptr, 0, total * tile_elems * 2, st));
         if (split)
             GCOO_CUDA(cudaMemsetAsync(p.a_lo.ptr, 0, 2 * total * kTileBytes, st));
@@ -958,9 +1166,15 @@ gcoo_status tc_prepare_b(gcoo_handle *h, int64_t n, bool fp8)
     const int N = tile_n_for(p.split);
     const int64_t nt = (n + N - 1) / N;
     const size_t elems = static_cast<size_t>(nt) * p.kb * N * kTileK;
-    // the parts of the split kernel's shares: two per CTA, whatever the width
-    const size_t parts = p.split ? 4 * static_cast<size_t>(device_sms()) * kPartFloats : 0;
-    if (!p.b_hi.ensure(elems) || (p.split && (!p.b_lo.ensure(2 * elems) || !p.part.ensure(parts))) ||
+    // the parts of the shares, whatever the width: two per CTA (split) or pair
+    size_t parts = 0;
+    if (p.split)
+        parts = 4 * static_cast<size_t>(device_sms()) * kPartFloats;
+    else
+        for (int64_t t = 1; t <= std::min<int64_t>(nt, kPairShareCols) && parts == 0; ++t)
+            if (pair_cut(p.panels, p.tiles, t).shares)
+                parts = static_cast<size_t>(device_sms()) * (2 * kPanel * kPairN);
+    if (!p.b_hi.ensure(elems) || (p.split && !p.b_lo.ensure(2 * elems)) || (parts > 0 && !p.part.ensure(parts)) ||
         (fp8 && (!p.b_scale.ensure(static_cast<size_t>(n)) || !p.b_amax.ensure(static_cast<size_t>(n)))))
         return fail(GCOO_ERROR_ALLOC, "device allocation of the B tiles failed");
     p.b_n = n;
