@@ -194,24 +194,28 @@ gcoo_status spdm_fp32(gcoo_handle *h, const float *dB, int64_t n, float *dC, cud
     }
     // a skewed matrix (explicit launch-shape overrides aside): its long rows go
     // to their own kernel, the short rest to a kernel without staging
-    if (!override_params && h->n_long > 0 && h->side && h->ev_fork && h->ev_join && long_rows_ok(n, dB)) {
-        const bool split = h->p.fp32_sum == GCOO_SUM_SPLIT && h->pieces_bound > 0;
+    if (!override_params && h->n_long > 0 && h->side && h->ev_fork && h->ev_join && long_rows_ok(h->m, n)) {
+        // the pieces' kernel copies 16 bytes at a time; other widths keep the chain
+        const bool split = h->p.fp32_sum == GCOO_SUM_SPLIT && h->pieces_bound > 0 && n % 4 == 0 &&
+                           (reinterpret_cast<uintptr_t>(dB) & 15) == 0;
         if (split) {
             gcoo_status ws = ensure_split_work(h, n);
             if (ws != GCOO_SUCCESS)
                 return ws;
         }
-        // the two kernels write disjoint rows of C: the long rows run on the
-        // side stream, forked from and joined back into the caller's stream
+        // The two kernels write disjoint rows of C: the short rows run on the
+        // side stream, forked from and joined back into the caller's stream.
+        // The long rows are on the caller's so that they start first: their
+        // CTAs spread over idle SMs and the short rows fill what is left.
         GCOO_CUDA(cudaEventRecord(h->ev_fork, st));
         GCOO_CUDA(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
         const cudaError_t el =
             split ? launch_spdm_split(h->packed.ptr, h->row_ptr.ptr, h->long_rows.ptr, h->n_long, h->piece_first.ptr,
                                       h->piece_row.ptr, h->piece_total.ptr, h->pieces_bound, dB, n,
-                                      h->split_part.ptr, dC, h->side)
-                  : launch_spdm_long(h->packed.ptr, h->row_ptr.ptr, h->long_rows.ptr, h->n_long, dB, n, dC, h->side);
+                                      h->split_part.ptr, dC, st)
+                  : launch_spdm_long(h->packed.ptr, h->row_ptr.ptr, h->long_rows.ptr, h->n_long, dB, n, dC, st);
         const cudaError_t es = el == cudaSuccess
-                                   ? launch_spdm_short(h->packed.ptr, h->row_ptr.ptr, h->m, h->k, dB, n, dC, long_row_min(), st)
+                                   ? launch_spdm_short(h->packed.ptr, h->row_ptr.ptr, h->m, h->k, dB, n, dC, long_row_min(), h->side)
                                    : cudaSuccess;
         // joined whatever happened: nothing of this call runs past it on the side stream
         GCOO_CUDA(cudaEventRecord(h->ev_join, h->side));

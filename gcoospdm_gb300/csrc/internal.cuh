@@ -193,8 +193,8 @@ cudaError_t launch_spdm_short(const Entry *packed, const int32_t *row_ptr, int64
 cudaError_t launch_fp8_scales(const float *B, int64_t k, int64_t n, unsigned *amax, float *scale, cudaStream_t st);
 // ---- long rows of skewed matrices (spdm_long.cu) -----------------------------------------
 int32_t long_row_min(); // 256 entries
-// n % 4 == 0 and a 16-byte aligned B (16-byte copies of B row pieces)
-bool long_rows_ok(int64_t n, const float *B);
+// Widths within the grids of the long and the short rows' kernels
+bool long_rows_ok(int64_t m, int64_t n);
 // list[0..min(*count, cap)) = the rows of at least long_row_min() entries,
 // longest first to within 64 entries (list: 2 * cap elements)
 cudaError_t launch_collect_long(const int32_t *row_ptr, int64_t m, int32_t *list, int64_t cap,
