@@ -36,7 +36,8 @@ namespace {
 
 constexpr int kChunk = 2048;
 // Four-warp CTAs per SM (64 registers a thread) and entries per batch of the
-// row walk. 4096^2 at 2 %, n = 4096 (us; BF16 / split / FP8): batches of eight
+// row walk. 4096^2 at 2 %, n = 4096 (us; BF16 / split / FP8, the latter two
+// before their mixed-precision FMAs: 324 / 173 with them): batches of eight
 // 152 / 398 / 192, of four 159 / 418 / 196, ten CTAs 154 / 406 / 200; before,
 // two warps per row, a staging per tile, 16 KB of shared memory and the tail
 // entry by entry: 220 / 443 / 222.
@@ -45,7 +46,6 @@ constexpr int kLowpCols = 1024; // columns per staging at most (512: 1-2 % slowe
 
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
-__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 enum Form { kBF16 = 1, kSplit = 2, kFP8 = 3, kFP8Wide = 4 };
 
@@ -86,9 +86,21 @@ __device__ __forceinline__ void split_f32x2(uint64_t x, float &lo, float &hi)
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x));
 }
 
-// A lane's V sums of one row tile, as the form multiplies them. BF16: the
-// mixed-precision FMA; the others in pairs (packed FMAs: half the issue
-// slots, which the widening of B's halves needs).
+// An FP16 value in FP32 (1 * h - 0, exact, signed zeros too) by the
+// mixed-precision FMA, which runs at the FMA's rate; the conversion
+// instruction at half of it bounded the FP8 rows (4096^2 at 2 %, n = 4096: 189
+// us with it, 173 without).
+__device__ __forceinline__ float widen_f16(uint16_t h)
+{
+    float d;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"(h), "h"(static_cast<uint16_t>(0x3c00)), "f"(-0.0f));
+    return d;
+}
+
+// A lane's V sums of one row tile, as the form multiplies them. BF16 and
+// split-BF16: mixed-precision FMAs on the bf16 halves as they are (split, 4096^2
+// at 2 %, n = 4096: 324 us; its halves widened and packed FMAs, half as many
+// instructions for the products, 399). FP8: packed FMAs, A being FP32.
 template <int F>
 struct Sums {
     static constexpr int V = FormTraits<F>::V;
@@ -114,32 +126,22 @@ struct Sums {
             for (int i = 0; i < 4; ++i) {
                 const __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(x[i] & 0xffffu), __NV_E4M3);
                 const __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(x[i] >> 16), __NV_E4M3);
-                const float2 f01 = __half22float2(*reinterpret_cast<const __half2 *>(&h01));
-                const float2 f23 = __half22float2(*reinterpret_cast<const __half2 *>(&h23));
-                fma_pair(s[(2 * i) % (V / 2)], a, f01.x, f01.y);
-                fma_pair(s[(2 * i + 1) % (V / 2)], a, f23.x, f23.y);
+                fma_pair(s[(2 * i) % (V / 2)], a, widen_f16(h01.x), widen_f16(h01.y));
+                fma_pair(s[(2 * i + 1) % (V / 2)], a, widen_f16(h23.x), widen_f16(h23.y));
             }
-        } else if constexpr (F == kFP8Wide) {
+        } else {
             const uint64_t a = dup_f32(val);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 fma_pair(s[i], a, bf_lo(x[i]), bf_hi(x[i]));
-        } else {
-            const float ah = round_bf16(val);
-            const uint64_t hi = dup_f32(ah), lo = dup_f32(round_bf16(val - ah));
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                fma_pair(s[i], hi, bf_lo(x[2 * i]), bf_lo(x[2 * i + 1]));
-                fma_pair(s[i], hi, bf_hi(x[2 * i]), bf_hi(x[2 * i + 1]));
-                fma_pair(s[i], lo, bf_lo(x[2 * i]), bf_lo(x[2 * i + 1]));
-            }
         }
     }
 };
 
-template <>
-struct Sums<kBF16> {
-    static constexpr int V = 8;
+// BF16 and split-BF16
+template <int F>
+struct MixedSums {
+    static constexpr int V = FormTraits<F>::V;
     float s[V];
     __device__ __forceinline__ void clear()
     {
@@ -151,14 +153,30 @@ struct Sums<kBF16> {
     __device__ __forceinline__ void add(float val, const uint4 &w)
     {
         const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-        const uint16_t ab = __bfloat16_as_ushort(__float2bfloat16_rn(val));
+        const __nv_bfloat16 a = __float2bfloat16_rn(val);
+        const uint16_t ah = __bfloat16_as_ushort(a);
+        if constexpr (F == kBF16) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            s[2 * i] = fma_bf16(ab, static_cast<uint16_t>(x[i] & 0xffffu), s[2 * i]);
-            s[2 * i + 1] = fma_bf16(ab, static_cast<uint16_t>(x[i] >> 16), s[2 * i + 1]);
+            for (int i = 0; i < 4; ++i) {
+                s[2 * i] = fma_bf16(ah, static_cast<uint16_t>(x[i] & 0xffffu), s[2 * i]);
+                s[2 * i + 1] = fma_bf16(ah, static_cast<uint16_t>(x[i] >> 16), s[2 * i + 1]);
+            }
+        } else {
+            const uint16_t al = __bfloat16_as_ushort(__float2bfloat16_rn(val - __bfloat162float(a)));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint16_t bh = static_cast<uint16_t>(x[i] & 0xffffu), bl = static_cast<uint16_t>(x[i] >> 16);
+                s[i] = fma_bf16(ah, bh, s[i]);
+                s[i] = fma_bf16(ah, bl, s[i]);
+                s[i] = fma_bf16(al, bh, s[i]);
+            }
         }
     }
 };
+template <>
+struct Sums<kBF16> : MixedSums<kBF16> {};
+template <>
+struct Sums<kSplit> : MixedSums<kSplit> {};
 
 template <int F, int U>
 __device__ __forceinline__ void lowp_batch(const Entry *__restrict__ s, const typename FormTraits<F>::T *__restrict__ Bj,
@@ -477,10 +495,10 @@ int lowp_vec(gcoo_precision prec) { return prec == GCOO_PREC_BF16 ? 8 : prec == 
 // FP8-B: B's E4M3 values as one byte or as the BF16 that equals each. Bytes:
 // half the gather, but two and a half instructions a value, and a warp's 16-byte
 // loads span 512 columns; BF16: one and a half instructions. Measured (us;
-// bytes / BF16): 8192^2 at 1 %, n = 2048 190 / 200; 4096^2 at 2 %, n = 4096
-// 192 / 198; 4001 x 3999 at 5 %, n = 1024 111 / 111; 2048^2 at 0.5 %, n = 512
-// 22 / 20; 8192 x 1200 at 3 %, n = 128 36 / 28. The group walk reads bytes.
-constexpr int64_t kFp8WideCols = 1024;
+// bytes / BF16): 4096^2 at 2 %, n = 4096 175 / 198, n = 1024 55 / 62, n = 512 39 /
+// 41, n = 256 36 / 30; 2048^2 at 0.5 %, n = 512 21 / 20; 8192 x 1200 at 3 %,
+// n = 128 33 / 27. The group walk reads bytes.
+constexpr int64_t kFp8WideCols = 512;
 static bool fp8_wide(const gcoo_handle *h, int64_t n) { return n <= kFp8WideCols && !group_order_chosen(h); }
 
 gcoo_status lowp_prepare(gcoo_handle *h, int64_t n, gcoo_precision prec)
