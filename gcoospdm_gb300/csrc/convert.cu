@@ -361,6 +361,8 @@ prefix_scan_kernel(int32_t *__restrict__ cnt, int64_t S, int32_t *__restrict__ d
                    int64_t *__restrict__ d_total, unsigned int *__restrict__ ticket,
                    int64_t *__restrict__ host_words, uint32_t *__restrict__ status)
 {
+    grid_wait_previous();
+    grid_launch_next();
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * (kTopThreads / 32) + (threadIdx.x >> 5);
@@ -778,10 +780,9 @@ cudaError_t launch_prefix_scan(int32_t *cnt, int64_t segments, int32_t *row_ptr,
                                int64_t *host_words, uint32_t *status, cudaStream_t st)
 {
     const int64_t blocks = (m + kTopThreads / 32 - 1) / (kTopThreads / 32);
-    prefix_scan_kernel<<<static_cast<unsigned>(blocks), kTopThreads, 0, st>>>(
-        cnt, segments, row_ptr, m, cpg, group_index, nnz_per_group, d_total, ticket, host_words, status);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_after(prefix_scan_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kTopThreads), 0, st, cnt, segments,
+                        row_ptr, m, cpg, group_index, nnz_per_group, d_total, ticket, host_words, status);
 }
 
 cudaError_t launch_scatter(const float *A, int64_t m, int64_t k, int32_t cpg, const int32_t *group_index,

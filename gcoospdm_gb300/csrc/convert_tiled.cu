@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kTileThreads)
 seg_count_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, int64_t S,
                  int32_t *__restrict__ cnt, unsigned long long *__restrict__ distinct)
 {
+    grid_launch_next();
     __shared__ int s_dist[kSegsPerCta];
     const SegUnit u = seg_unit<CPG>(m, k, tiles, blockIdx.x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -241,6 +242,7 @@ seg_scatter_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t ti
                    const int32_t *__restrict__ row_ptr, float *__restrict__ vals, int32_t *__restrict__ rows,
                    int32_t *__restrict__ cols, Entry *__restrict__ packed)
 {
+    grid_wait_previous();
     scatter_segment<CPG, AL>(A, m, k, S, seg_unit<CPG>(m, k, tiles, blockIdx.x), pref, group_index, row_ptr, vals, rows,
                          cols, packed);
 }
@@ -296,6 +298,7 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
              int32_t *__restrict__ tile_tot, int32_t *__restrict__ over_list,
              unsigned long long *__restrict__ over_count, uint32_t *__restrict__ status)
 {
+    grid_launch_next();
     constexpr int kWarps = 1024 / L / 32;
     constexpr int kSegPerWarp = L / 4;
     static_assert(CPG * L <= 32, "a lane's nonzeros are one 32-bit mask");
@@ -500,6 +503,7 @@ place_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
              Entry *__restrict__ packed, const int64_t *__restrict__ d_total, int64_t cap, int64_t packed_cap,
              int64_t staged_blocks, int32_t *__restrict__ clear_rows)
 {
+    grid_wait_previous();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool staged_block = static_cast<int64_t>(blockIdx.x) < staged_blocks;
     const int64_t b = static_cast<int64_t>(blockIdx.x) * kSegsPerCta + warp;
@@ -643,8 +647,9 @@ cudaError_t launch_tile_scatter(const float *A, int64_t m, int64_t k, int32_t cp
         return cudaSuccess;
     const unsigned grid = static_cast<unsigned>(units);
     const bool al = rows_aligned(A, k);
+    cudaError_t le = cudaSuccess;
 #define GCOO_SEG_SCATTER(C)                                                                                     \
-    (al ? seg_scatter_kernel<C, true> : seg_scatter_kernel<C, false>)<<<grid, kTileThreads, 0, st>>>(           \
+    le = launch_after(al ? seg_scatter_kernel<C, true> : seg_scatter_kernel<C, false>, dim3(grid), dim3(kTileThreads), 0, st, \
         A, m, k, tiles, S, pref, group_index, row_ptr, vals, rows, cols, packed)
     switch (cpg) {
     case 1: GCOO_SEG_SCATTER(1); break;
@@ -655,7 +660,7 @@ cudaError_t launch_tile_scatter(const float *A, int64_t m, int64_t k, int32_t cp
     }
 #undef GCOO_SEG_SCATTER
     count_launches(1);
-    return cudaGetLastError();
+    return le;
 }
 
 bool staged_convert_ok(const float *A, int64_t m, int64_t k, int32_t cpg)
@@ -718,8 +723,9 @@ cudaError_t launch_place(const float *A, int64_t m, int64_t k, int32_t cpg, int3
         rescan_blocks = units;
     const unsigned grid = static_cast<unsigned>(staged_blocks + rescan_blocks);
     const bool al = rows_aligned(A, k);
+    cudaError_t le = cudaSuccess;
 #define GCOO_PLACE(C)                                                                                 \
-    (al ? place_kernel<C, true> : place_kernel<C, false>)<<<grid, kTileThreads, 0, st>>>(             \
+    le = launch_after(al ? place_kernel<C, true> : place_kernel<C, false>, dim3(grid), dim3(kTileThreads), 0, st, \
         A, m, k, tiles, S, units, slot, stage, tile_tot, over_list, over_count, pref, group_index,    \
         row_ptr, vals, rc, packed, d_total, cap, packed_cap, staged_blocks, clear_rows)
     switch (cpg) {
@@ -731,7 +737,7 @@ cudaError_t launch_place(const float *A, int64_t m, int64_t k, int32_t cpg, int3
     }
 #undef GCOO_PLACE
     count_launches(1);
-    return cudaGetLastError();
+    return le;
 }
 
 } // namespace gcoo

@@ -64,6 +64,8 @@ template <bool VI, bool VO>
 __global__ void __launch_bounds__(256)
 transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t R, int64_t Cc)
 {
+    grid_wait_previous();
+    grid_launch_next();
     __shared__ float tile[kTr][kTr + 1];
     const int64_t c0 = static_cast<int64_t>(blockIdx.x) * kTr, r0 = static_cast<int64_t>(blockIdx.y) * kTr;
     const int t = threadIdx.x;
@@ -114,10 +116,10 @@ cudaError_t transpose(const float *in, float *out, int64_t R, int64_t Cc, cudaSt
     const bool vi = Cc % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0;
     const bool vo = R % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-    (vi ? vo ? transpose_kernel<true, true> : transpose_kernel<true, false>
-        : vo ? transpose_kernel<false, true> : transpose_kernel<false, false>)<<<grid, 256, 0, st>>>(in, out, R, Cc);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_after(vi ? vo ? transpose_kernel<true, true> : transpose_kernel<true, false>
+                        : vo ? transpose_kernel<false, true> : transpose_kernel<false, false>,
+                        grid, dim3(256), 0, st, in, out, R, Cc);
 }
 
 int bits_for_left(uint64_t maxkey)

@@ -275,6 +275,8 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
                  int32_t cpg, const float *__restrict__ B, int64_t n, float *__restrict__ C,
                  int32_t col_warps, int32_t col_iters, int32_t chunk_cap, uint32_t *__restrict__ status)
 {
+    grid_wait_previous();
+    grid_launch_next();
     if (!MULTI)
         col_iters = 1;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -786,10 +788,10 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
 #define GCOO_FP32_LAUNCH(V, W, T, P)                                                                       \
     do {                                                                                                \
         if (s.col_iters > 1)                                                                            \
-            spdm_fp32_kernel<V, W, T, P, true><<<grid, threads, smem, st>>>(                               \
+            le = launch_after(spdm_fp32_kernel<V, W, T, P, true>, grid, dim3(threads), smem, st,          \
                 packed, row_ptr, m, cpg, B, n, C, s.col_warps, s.col_iters, chunk, status);             \
         else                                                                                            \
-            spdm_fp32_kernel<V, W, T, P, false><<<grid, threads, smem, st>>>(                              \
+            le = launch_after(spdm_fp32_kernel<V, W, T, P, false>, grid, dim3(threads), smem, st,         \
                 packed, row_ptr, m, cpg, B, n, C, s.col_warps, 1, chunk, status);                       \
     } while (0)
 #define GCOO_FP32_VEC(T, P)                                                                             \
@@ -802,6 +804,7 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
         else GCOO_FP32_LAUNCH(1, 1, T, P);                                                              \
     } while (0)
     const bool pipe = s.depth >= 2;
+    cudaError_t le = cudaSuccess;
     if (threads <= 128 && !pipe) {
         GCOO_FP32_VEC(128, false);
     } else if (threads <= 512) {
@@ -814,7 +817,7 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
 #undef GCOO_FP32_VEC
 #undef GCOO_FP32_LAUNCH
     count_launches(1);
-    return cudaGetLastError();
+    return le;
 }
 
 cudaError_t launch_spdm_short(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k, const float *B,

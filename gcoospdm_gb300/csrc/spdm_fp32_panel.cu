@@ -125,6 +125,8 @@ spdm_panel_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
                   const int32_t *__restrict__ pref, int64_t S, int64_t m, const float *__restrict__ B, int64_t n,
                   float *__restrict__ C)
 {
+    grid_wait_previous();
+    grid_launch_next();
     extern __shared__ __align__(16) unsigned char smem[];
     float *s_a = reinterpret_cast<float *>(smem);                             // [listed column][kPanelRows]
     float *s_b = s_a + kWinCols * kPanelRows;                                 // [warp][kRing][kCols]
@@ -448,9 +450,8 @@ cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, 
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
         return e;
-    kern<<<grid, warps * 32, smem, st>>>(packed, row_ptr, pref, S, m, B, n, C);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_after(kern, grid, dim3(warps * 32), smem, st, packed, row_ptr, pref, S, m, B, n, C);
 }
 
 } // namespace gcoo

@@ -242,6 +242,7 @@ spdm_lowp_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
                  const typename FormTraits<F>::T *__restrict__ B, const float *__restrict__ col_scale, int64_t n,
                  float *__restrict__ C, int32_t col_iters, int32_t chunk, uint32_t *__restrict__ status)
 {
+    grid_wait_previous();
     constexpr int V = FormTraits<F>::V;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
@@ -315,6 +316,7 @@ spdm_lowp_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 // ---- B pre-pass kernels (grid-stride over k*n / 4) ----------------------------------
 __global__ void prep_bf16_kernel(const float4 *__restrict__ B, uint2 *__restrict__ out, int64_t n4)
 {
+    grid_launch_next();
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const float4 v = __ldcs(B + i);
@@ -326,6 +328,7 @@ __global__ void prep_bf16_kernel(const float4 *__restrict__ B, uint2 *__restrict
 
 __global__ void prep_split_kernel(const float4 *__restrict__ B, uint4 *__restrict__ out, int64_t n4)
 {
+    grid_launch_next();
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const float4 v = __ldcs(B + i);
@@ -350,6 +353,7 @@ constexpr int kStripCols = 128, kStripRows = 128, kWarpRows = 16;
 __global__ void __launch_bounds__(256)
 colmax_kernel(const float *__restrict__ B, int64_t k, int64_t n, unsigned *__restrict__ amax)
 {
+    grid_launch_next();
     __shared__ float s_max[kStripRows / kWarpRows][kStripCols];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t j = static_cast<int64_t>(blockIdx.x) * kStripCols + lane * 4;
@@ -408,6 +412,8 @@ __global__ void __launch_bounds__(256)
 prep_fp8_kernel(const float *__restrict__ B, const unsigned *__restrict__ amax, float *__restrict__ scale,
                 void *__restrict__ out, int64_t k, int64_t n)
 {
+    grid_wait_previous();
+    grid_launch_next();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t j = static_cast<int64_t>(blockIdx.x) * kStripCols + lane * 4;
     const int64_t c0 = static_cast<int64_t>(blockIdx.y) * kStripRows + warp * kWarpRows;
@@ -537,9 +543,11 @@ gcoo_status lowp_convert_b(gcoo_handle *h, const float *dB, int64_t n, gcoo_prec
     } else {
         GCOO_CUDA(launch_colmax(dB, h->k, n, w->amax.ptr, st));
         if (!fp8_wide(h, n))
-            prep_fp8_kernel<false><<<strip_grid(h->k, n), 256, 0, st>>>(dB, w->amax.ptr, w->scale.ptr, w->f8.ptr, h->k, n);
+            GCOO_CUDA(launch_after(prep_fp8_kernel<false>, strip_grid(h->k, n), dim3(256), 0, st, dB, w->amax.ptr,
+                                   w->scale.ptr, w->f8.ptr, h->k, n));
         else
-            prep_fp8_kernel<true><<<strip_grid(h->k, n), 256, 0, st>>>(dB, w->amax.ptr, w->scale.ptr, w->bf.ptr, h->k, n);
+            GCOO_CUDA(launch_after(prep_fp8_kernel<true>, strip_grid(h->k, n), dim3(256), 0, st, dB, w->amax.ptr,
+                                   w->scale.ptr, w->bf.ptr, h->k, n));
         count_launches(1);
     }
     GCOO_LAUNCH("B conversion kernel");
@@ -586,8 +594,8 @@ gcoo_status lowp_spdm(gcoo_handle *h, int64_t n, float *dC, gcoo_precision prec,
     dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(ny));
     const size_t smem = 128 + (static_cast<size_t>(chunk) + 2) * sizeof(Entry);
 #define GCOO_LOWP(F, DATA, SCALE)                                                                               \
-    spdm_lowp_kernel<F><<<grid, rows * 32, smem, st>>>(h->packed.ptr, h->row_ptr.ptr, h->m, rows, DATA, SCALE,  \
-                                                       n, dC, static_cast<int32_t>(ci), chunk, h->status.ptr)
+    GCOO_CUDA(launch_after(spdm_lowp_kernel<F>, grid, dim3(rows * 32), smem, st, h->packed.ptr, h->row_ptr.ptr,  \
+                           h->m, rows, DATA, SCALE, n, dC, static_cast<int32_t>(ci), chunk, h->status.ptr))
     if (prec == GCOO_PREC_BF16)
         GCOO_LOWP(kBF16, w->bf.ptr, nullptr);
     else if (prec == GCOO_PREC_SPLIT_BF16)

@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(256)
 b_tiles_kernel(const float *__restrict__ B, int64_t k, int64_t n, int64_t kb, __nv_bfloat16 *__restrict__ hi,
                __nv_bfloat16 *__restrict__ lo, const float *__restrict__ fp8_scale)
 {
+    grid_launch_next();
     constexpr int N = SPLIT ? 128 : 256, kT = 256 / N; // kT tiles (column blocks of 16 k) per CTA
     constexpr int kLoads = kTileK * N * kT / 4 / 256;  // float4 per thread
     __shared__ __align__(16) float blk[kT][kTileK][N];
@@ -436,6 +437,8 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    grid_wait_previous(); // barriers and tensor memory are the CTA's own
+    grid_launch_next();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -593,6 +596,7 @@ __global__ void __launch_bounds__(2 * kPanel)
 tc_fixup_kernel(const int32_t *__restrict__ pf, int64_t m, int64_t n, int64_t kb, int64_t tiles, const ShareCut cut,
                 int cols, const float *__restrict__ part, float *__restrict__ C)
 {
+    grid_wait_previous();
     __shared__ __align__(16) float staging[2 * kPanel * kStageRow];
     const int R = blockDim.x;
     const int64_t panel = blockIdx.x, jt = blockIdx.y;
@@ -800,6 +804,8 @@ spdm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    grid_wait_previous(); // barriers and tensor memory are the CTA's own
+    grid_launch_next();
     tc_fence_before();
     cluster_sync_all(); // both CTAs' barriers initialised and tensor memory allocated
     tc_fence_after();
@@ -1060,13 +1066,18 @@ cudaError_t launch_pair(TcPlan &p, int64_t m, int64_t n, float *C, uint32_t *sta
     const ShareCut shares(p.tiles * strips, cut.pairs > 0 ? cut.pairs : 1);
     if (2 * p.panels > 0x7fffffffLL || strips > 65535 || 2 * cut.pairs > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    spdm_tc_pair_kernel<<<static_cast<unsigned>(2 * cut.pairs), kPairThreads, kPairSmem, st>>>(
-        map_a, map_b, p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, m, n, p.kb, p.panels, p.tiles, shares, cut.shares, cut.nt,
+    e = launch_after(
+        spdm_tc_pair_kernel, dim3(static_cast<unsigned>(2 * cut.pairs)), dim3(kPairThreads), kPairSmem, st, map_a, map_b, p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, m, n, p.kb, p.panels, p.tiles, shares, cut.shares, cut.nt,
         C, p.part.ptr, status);
+    if (e != cudaSuccess)
+        return e;
     if (cut.shares) {
         const int cols = cut.nt * kPairN;
         const dim3 grid(static_cast<unsigned>(p.panels), static_cast<unsigned>(strips), static_cast<unsigned>(cols / 32));
-        tc_fixup_kernel<<<grid, 2 * kPanel, 0, st>>>(p.pf.ptr, m, n, p.kb, p.tiles, shares, cols, p.part.ptr, C);
+        e = launch_after(tc_fixup_kernel, grid, dim3(2 * kPanel), 0, st, p.pf.ptr, m, n, p.kb, p.tiles, shares, cols,
+                         p.part.ptr, C);
+        if (e != cudaSuccess)
+            return e;
         count_launches(1);
     }
     count_launches(1);
@@ -1088,18 +1099,20 @@ cudaError_t launch_split(const TcPlan &p, int64_t m, int64_t n, float *C, uint32
     if (njt > 65535 || p.panels > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
     if (work > 0) {
-        const cudaError_t e = cudaFuncSetAttribute(spdm_tc_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
+        cudaError_t e = cudaFuncSetAttribute(spdm_tc_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
         if (e != cudaSuccess)
             return e;
-        spdm_tc_split_kernel<<<static_cast<unsigned>(ctas), kSplitThreads, kSplitSmem, st>>>(
-            p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n, p.kb, p.tiles,
+        e = launch_after(
+            spdm_tc_split_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kSplitThreads), kSplitSmem, st, p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n, p.kb, p.tiles,
             cut, C, p.part.ptr, status);
+        if (e != cudaSuccess)
+            return e;
         count_launches(1);
     }
     const dim3 grid(static_cast<unsigned>(p.panels), static_cast<unsigned>(njt), kSplitN / 32);
-    tc_fixup_kernel<<<grid, kPanel, 0, st>>>(p.pf.ptr, m, n, p.kb, p.tiles, cut, kSplitN, p.part.ptr, C);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_after(tc_fixup_kernel, grid, dim3(kPanel), 0, st, p.pf.ptr, m, n, p.kb, p.tiles, cut, kSplitN,
+                        p.part.ptr, C);
 }
 
 } // namespace
