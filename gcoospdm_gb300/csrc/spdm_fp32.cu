@@ -752,11 +752,17 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
         // about 768 columns per CTA (0.5-0.9 K columns measured best from
         // 2048^2 to 16384^2 at 1 % to 0.1 % density), but at least four waves
         // of CTAs on small matrices: the last wave's share of the time (4096^2
-        // at 5 % 623 us with two, 604 with four; 2048^2 at 10 % 148 and 141)
+        // at 5 % 623 us with two, 604 with four; 2048^2 at 10 % 148 and 141;
+        // 4096^2 at 1.5 %, n = 2048 108 with one, 107 and 100). Short rows: a
+        // CTA's staging is the larger share, so one wave under 8 entries
+        // (2048^2 at 0.1 % 8.1 us, 9.2 with two, 11.2 with four; 2880 x 1527
+        // at 0.28 %, n = 1568 11.3, 11.4 and 14.0) and two under 16 (2048^2 at
+        // 0.5 % 16.0, 15.1 and 16.5)
         int64_t ci = 768 / tile;
         const int64_t groups = (m + s.rows - 1) / s.rows;
         const int64_t resident = static_cast<int64_t>(device_sms()) * (s.warps <= 4 ? kRowCtas : 6);
-        const int64_t by_grid = groups * ny / (4 * resident);
+        const int64_t waves = nnz < 8 * m ? 1 : (nnz < 16 * m ? 2 : 4);
+        const int64_t by_grid = groups * ny / (waves * resident);
         ci = ci > by_grid ? by_grid : ci;
         ci = ci < 1 ? 1 : (ci > ny ? ny : ci);
         s.col_iters = static_cast<int>(ci > 64 ? 64 : ci);
