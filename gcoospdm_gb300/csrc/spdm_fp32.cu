@@ -413,6 +413,8 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 // Forty warps per SM with batches of four: 137 us on the Zipf workload with
 // the long rows beside it, against 145 for thirty-two with batches of eight
 // (forty-eight with four: 137, sixty-four 147, forty with eight 145).
+// With the long rows in their copy-and-chain kernel: 118, forty-eight warps 118,
+// thirty-two with batches of eight 127, of six 130.
 constexpr int kShortBatch = 4, kShortCtas = 20;
 
 template <int V, int U>
