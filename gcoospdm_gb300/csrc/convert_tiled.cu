@@ -289,8 +289,8 @@ __device__ __forceinline__ RowPiece row_piece(const float *p, int w)
 
 // AL: as in seg_load. Otherwise a row piece sits in shared memory shifted by
 // its 0..3 floats against 16 bytes: its whole granules arrive by bulk copy,
-// the up to three floats on either side by plain loads, and each lane reads
-// one float4 more and shifts.
+// the up to three floats on either side by plain loads, and the lanes shift
+// their bits, not their floats (4001 x 3999: 21.7 -> 17.6 us).
 template <int CPG, int L, bool AL>
 __global__ void __launch_bounds__(1024 / L, L == 8 ? 12 : (CPG <= 4 ? 8 : 6))
 stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, int64_t S, int32_t *__restrict__ cnt,
@@ -373,32 +373,45 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
         }
         return;
     }
+    constexpr uint32_t kCol = (CPG == 4) ? (L == 8 ? 0x11111111u : 0x1111u)
+                            : (CPG == 2) ? (L == 8 ? 0x5555u : 0x55u)
+                            : (CPG == 1) ? (L == 8 ? 0xffu : 0xfu) : 0x01010101u;
     // the lane's nonzeros as one mask in GCOO order: bit q * CPG + r = (row r, column c + q)
     uint32_t msk = 0;
+    if constexpr (!AL) {
+        // the same of its shared-memory floats, then each row's bits moved by
+        // that row's shift, the last ones from the next lane (lane 31: from the
+        // four floats past the warp's), and the columns past the row cut off
+        uint32_t own = 0;
+#pragma unroll
+        for (int r = 0; r < CPG; ++r)
+            if (r < nrows) {
+#pragma unroll
+                for (int h = 0; h < L / 4; ++h) {
+                    const float4 x = *reinterpret_cast<const float4 *>(&s_a[r][sc + 4 * h]);
+                    const int q0 = 4 * h;
+                    own |= (nzb(x.x) << (q0 * CPG + r)) | (nzb(x.y) << ((q0 + 1) * CPG + r)) |
+                           (nzb(x.z) << ((q0 + 2) * CPG + r)) | (nzb(x.w) << ((q0 + 3) * CPG + r));
+                }
+            }
+        const bool at_edge = lane < 4 * CPG && s_a[lane % CPG][(warp + 1) * (32 * L) + (lane / CPG) % 4] != 0.0f;
+        const uint32_t edge = __ballot_sync(0xffffffffu, at_edge);
+        uint32_t next = __shfl_down_sync(0xffffffffu, own, 1);
+        next = lane == 31 ? edge : next;
+#pragma unroll
+        for (int r = 0; r < CPG; ++r)
+            if (r < nrows) {
+                const unsigned by = ((sh0 + static_cast<unsigned>(r) * k3) & 3u) * CPG;
+                const uint32_t moved = L * CPG == 32 ? __funnelshift_r(own, next, by)
+                                                     : (own | (next << (L * CPG % 32))) >> by;
+                msk |= moved & (kCol << r);
+            }
+        const int64_t left = k - c;
+        if (left < L)
+            msk = left > 0 ? msk & ((1u << (static_cast<int>(left) * CPG)) - 1u) : 0u;
+    }
 #pragma unroll
     for (int r = 0; r < CPG; ++r) {
-        if (!AL && r < nrows) {
-            const unsigned shift = (sh0 + static_cast<unsigned>(r) * k3) & 3u;
-            float x[L + 4];
-#pragma unroll
-            for (int h = 0; h < L / 4 + 1; ++h) {
-                const float4 y = *reinterpret_cast<const float4 *>(&s_a[r][sc + 4 * h]);
-                x[4 * h] = y.x; x[4 * h + 1] = y.y; x[4 * h + 2] = y.z; x[4 * h + 3] = y.w;
-            }
-            if (shift & 1u) {
-#pragma unroll
-                for (int i = 0; i < L + 3; ++i)
-                    x[i] = x[i + 1];
-            }
-            if (shift & 2u) {
-#pragma unroll
-                for (int i = 0; i < L + 1; ++i)
-                    x[i] = x[i + 2];
-            }
-#pragma unroll
-            for (int q = 0; q < L; ++q)
-                msk |= (c + q < k ? nzb(x[q]) : 0u) << (q * CPG + r);
-        }
         if (AL && r < nrows) {
 #pragma unroll
             for (int h = 0; h < L / 4; ++h) {
@@ -411,9 +424,6 @@ stage_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
             }
         }
     }
-    constexpr uint32_t kCol = (CPG == 4) ? (L == 8 ? 0x11111111u : 0x1111u)
-                            : (CPG == 2) ? (L == 8 ? 0x5555u : 0x55u)
-                            : (CPG == 1) ? (L == 8 ? 0xffu : 0xfu) : 0x01010101u;
     // per-row counts of the warp's segment(s): lanes 16..31 cover the second one (L = 8),
     // so one reduction of (first | second << 16) counts both
     const uint32_t hi = (L == 8 && lane >= 16) ? 16u : 0u;
