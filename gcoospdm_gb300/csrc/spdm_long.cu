@@ -163,6 +163,7 @@ constexpr int kDepth = V == 1 ? 3 : 4; // steps of B pieces in flight
 template <int V>
 constexpr int kLongSmem = kDepth<V> * kBatch<V> * 32 * V * 4 + 2 * kDepth<V> * kBatch<V> * 8;
 constexpr int kFewCtas = 12; // CTAs of V = 1 per SM up to which the chain is the time
+constexpr int kMostSmem = 227 * 1024; // of one CTA
 
 // The items (row, tile), longest rows first, over the CTAs that start
 // together, `per_sm` on each SM: those of one SM, whether it gets consecutive
@@ -286,12 +287,14 @@ cudaError_t launch_long(const Entry *packed, const int32_t *row_ptr, const int32
     // beside the short rows the scheduler otherwise puts a dozen on one SM and
     // leaves others empty (25 rows of 4096, n = 192: 103 us against 36)
     const int64_t sms = device_sms();
-    const int most = static_cast<int>(227 * 1024 / (kLongSmem<V> + 1024));
+    const int most = static_cast<int>(kMostSmem / (kLongSmem<V> + 1024));
     const int per_sm = static_cast<int>(std::min<int64_t>(most, (ctas + sms - 1) / sms));
-    const int smem = std::max(kLongSmem<V>, 227 * 1024 / per_sm / 128 * 128 - 1024);
+    const int smem = std::max(kLongSmem<V>, kMostSmem / per_sm / 128 * 128 - 1024);
     const Spread spread{static_cast<unsigned>(per_sm), static_cast<unsigned>(sms),
                         static_cast<unsigned>(std::min<int64_t>(ctas, per_sm * sms))};
-    const cudaError_t e = cudaFuncSetAttribute(spdm_long_kernel<V, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the most that any call asks for, not this call's: the attribute belongs to
+    // every thread of the process, one of which may launch right after another
+    const cudaError_t e = cudaFuncSetAttribute(spdm_long_kernel<V, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
     if (e != cudaSuccess)
         return e;
     spdm_long_kernel<V, W><<<static_cast<unsigned>(ctas), 32 * (1 + kCopyWarps<V>), smem, st>>>(
