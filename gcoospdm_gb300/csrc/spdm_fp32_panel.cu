@@ -52,6 +52,11 @@ constexpr int kCols = 32 * kV; // output columns per warp
 constexpr int kRing = 8;       // B rows a warp keeps in flight, two per commit group
 constexpr int kBatch = 8;      // entries a thread loads at once while staging
 
+constexpr int panel_smem(int warps)
+{
+    return kWinCols * (kPanelRows * 4 + 8 + 4 + 4 + 2) + warps * kRing * kCols * 4 + kRing * 8 + 8;
+}
+
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
 {
     uint64_t d;
@@ -445,13 +450,13 @@ cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, 
         return cudaErrorInvalidConfiguration;
     const dim3 grid(static_cast<unsigned>(nx), static_cast<unsigned>(ny));
     const int64_t S = conv_segments(k);
-    const int smem = kWinCols * (kPanelRows * 4 + 8 + 4 + 4 + 2) + warps * kRing * kCols * 4 + kRing * 8 + 8;
     const auto kern = vec4 ? spdm_panel_kernel<true> : spdm_panel_kernel<false>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the most that any call asks for: the attribute belongs to every thread of the process
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem(kMaxWarps));
     if (e != cudaSuccess)
         return e;
     count_launches(1);
-    return launch_after(kern, grid, dim3(warps * 32), smem, st, packed, row_ptr, pref, S, m, B, n, C);
+    return launch_after(kern, grid, dim3(warps * 32), panel_smem(warps), st, packed, row_ptr, pref, S, m, B, n, C);
 }
 
 } // namespace gcoo

@@ -59,3 +59,11 @@ def test_long_rows_of_two_handles(native):
     few, many = long_rows(2, 64, 2000, 1), long_rows(3, 4800, 2000, 400)
     B = rng.standard_normal((2000, 64)).astype(np.float32)
     at_once(native, 2 * [(few, B), (many, B)], passes=8000)
+
+
+def test_panels_of_two_handles(native):
+    """One warp per CTA (n = 128) beside four (n = 512)."""
+    rng = np.random.default_rng(4)
+    A = np.repeat(rng.standard_normal((2, 256)), 16, axis=0).astype(np.float32)
+    jobs = [(A, rng.standard_normal((256, n)).astype(np.float32)) for n in (128, 512)]
+    at_once(native, jobs, fp32_order="groups")
