@@ -396,7 +396,7 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 // CTA barrier -- a row of a dozen entries is all latency, and a staging round
 // trip and a group barrier would double it. The row's two pointers come in
 // one load (lanes 0 and 1) and are shuffled to the warp. Lane i loads entry i
-// of each 32-entry window; the B rows of four entries at a time are loaded
+// of each 32-entry window; the B rows of U entries at a time are loaded
 // with their columns shuffled from the owning lanes; each column's fmaf chain
 // runs over the row's entries in column order from 0.0f, as in every other
 // FP32 kernel. Measured slower on the Zipf workload (0.148 ms for this
@@ -415,7 +415,14 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 // (forty-eight with four: 137, sixty-four 147, forty with eight 145).
 // With the long rows in their copy-and-chain kernel: 118, forty-eight warps 118,
 // thirty-two with batches of eight 127, of six 130.
-constexpr int kShortBatch = 4, kShortCtas = 20;
+// Thirty-two with batches of eight where the long rows are summed in pieces, so
+// that the short ones take longer, and all warps fit four waves: a row of some
+// hundred entries is then the time, and twice the loads in flight shorten it
+// (us, split sums, batches of four / eight: 8192 warps 23.3 / 20.3, 16384 26.6 /
+// 25.0, 24000 32.1 / 31.1, 30000 37.9 / 40.1, 65536 52 / 58; chains, 16346
+// warps 33.8 / 35.2, 24000 34.6 / 36.7).
+constexpr int64_t kShortDeepWaves = 4;
+constexpr int short_ctas(int batch) { return batch == 4 ? 20 : 16; } // per SM
 
 template <int V, int U>
 __device__ __forceinline__ void short_window(const Entry &my, int nw, bool all_cols, bool has_col,
@@ -466,8 +473,8 @@ __device__ __forceinline__ void short_window(const Entry &my, int nw, bool all_c
 // B larger than this walks tile-major (see spdm_short_kernel)
 constexpr int64_t kShortTileMajorBytes = 32ll << 20;
 
-template <int V>
-__global__ void __launch_bounds__(64, kShortCtas)
+template <int V, int U>
+__global__ void __launch_bounds__(64, short_ctas(U))
 spdm_short_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m,
                   const float *__restrict__ B, int64_t n, float *__restrict__ C, int32_t tiles, int32_t long_min,
                   int32_t tile_major)
@@ -507,7 +514,7 @@ spdm_short_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
         my.val = 0.0f;
         if (lane < nw)
             my = packed[rs + w0 + lane];
-        short_window<V, kShortBatch>(my, nw, all_cols, has_col, Bj, n, acc);
+        short_window<V, U>(my, nw, all_cols, has_col, Bj, n, acc);
     }
     if (has_col)
         Piece<V>::store(C + row * n + j, acc);
@@ -829,7 +836,7 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
 }
 
 cudaError_t launch_spdm_short(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k, const float *B,
-                              int64_t n, float *C, int32_t long_min, cudaStream_t st)
+                              int64_t n, float *C, int32_t long_min, bool split, cudaStream_t st)
 {
     if (m <= 0 || n <= 0)
         return cudaSuccess;
@@ -849,12 +856,17 @@ cudaError_t launch_spdm_short(const Entry *packed, const int32_t *row_ptr, int64
     const unsigned grid = static_cast<unsigned>(blocks);
     const int32_t nt = static_cast<int32_t>(tiles);
     const int32_t tm = tiles > 1 && k * n * 4 > kShortTileMajorBytes ? 1 : 0;
+    const bool deep = split && warps <= kShortDeepWaves * device_sms() * 2 * short_ctas(4);
+#define GCOO_SHORT(V)                                                                                               \
+    (deep ? spdm_short_kernel<V, 8> : spdm_short_kernel<V, 4>)<<<grid, 64, 0, st>>>(packed, row_ptr, m, B, n, C, nt, \
+                                                                                    long_min, tm)
     if (v == 4)
-        spdm_short_kernel<4><<<grid, 64, 0, st>>>(packed, row_ptr, m, B, n, C, nt, long_min, tm);
+        GCOO_SHORT(4);
     else if (v == 2)
-        spdm_short_kernel<2><<<grid, 64, 0, st>>>(packed, row_ptr, m, B, n, C, nt, long_min, tm);
+        GCOO_SHORT(2);
     else
-        spdm_short_kernel<1><<<grid, 64, 0, st>>>(packed, row_ptr, m, B, n, C, nt, long_min, tm);
+        GCOO_SHORT(1);
+#undef GCOO_SHORT
     count_launches(1);
     return cudaGetLastError();
 }
