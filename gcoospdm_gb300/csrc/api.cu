@@ -353,7 +353,7 @@ gcoo_status choose_panels(gcoo_handle *h, cudaStream_t st)
     GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m, h->long_count.ptr, st));
     GCOO_CUDA(cudaMemcpyAsync(share, h->long_count.ptr, sizeof(share), cudaMemcpyDeviceToHost, st));
     GCOO_CUDA(cudaStreamSynchronize(st));
-    h->panels = share[0] >= 12 * share[1];
+    h->panels = share[1] > 0 && share[0] >= 12 * share[1];
     return GCOO_SUCCESS;
 }
 

@@ -387,8 +387,8 @@ spdm_panel_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
 }
 
 // How many rows of a panel share a column, on up to gridDim.x panels spread
-// over the matrix: out[0] += entries, out[1] += distinct columns (of the
-// first kShareCols columns).
+// over the matrix: out[0] += entries, out[1] += distinct columns, both of
+// kShareCols columns from each panel's first one with an entry on.
 constexpr int kShareCols = 1 << 17;
 constexpr int kSharePanels = 64;
 
@@ -397,14 +397,21 @@ panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__
                    unsigned long long *__restrict__ out)
 {
     __shared__ uint32_t s_seen[kShareCols / 32];
+    __shared__ int s_first;
     const int64_t r0 = (blockIdx.x * panels / gridDim.x) * kPanelRows;
     const int64_t r1 = r0 + kPanelRows < m ? r0 + kPanelRows : m;
     for (int i = threadIdx.x; i < kShareCols / 32; i += blockDim.x)
         s_seen[i] = 0;
+    if (threadIdx.x == 0)
+        s_first = 0x7fffffff;
+    __syncthreads();
+    const int64_t r = r0 + threadIdx.x;
+    if (r < r1 && row_ptr[r] < row_ptr[r + 1])
+        atomicMin(&s_first, packed[row_ptr[r]].col);
     __syncthreads();
     int entries = 0, distinct = 0;
     for (int64_t e = row_ptr[r0] + threadIdx.x; e < row_ptr[r1]; e += blockDim.x) {
-        const int c = packed[e].col;
+        const int c = packed[e].col - s_first;
         if (c < kShareCols) {
             ++entries;
             atomicOr(&s_seen[c >> 5], 1u << (c & 31));

@@ -1,0 +1,35 @@
+"""GPU: by what evidence a build chooses the walk of sixteen rows."""
+from __future__ import annotations
+
+import pytest
+
+from graph_kernels import captured_kernels
+
+pytestmark = pytest.mark.gpu
+
+
+def blocks(m, k, bs, density, first_col=0, seed=1):
+    """bs x bs blocks from first_col on, on the GPU."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    on = torch.rand(m // bs, (k - first_col) // bs, generator=gen, device="cuda") < density
+    A = torch.zeros(m, k, device="cuda")
+    A[:, first_col:] = on.repeat_interleave(bs, 0).repeat_interleave(bs, 1)
+    return A
+
+
+@pytest.mark.parametrize("bs,first_col,kernel", [(16, 0, "spdm_panel_kernel"), (4, 0, "spdm_group_kernel"),
+                                                 (16, 1 << 17, "spdm_panel_kernel"), (4, 1 << 17, "spdm_group_kernel")])
+def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
+    """Blocks as high as a panel take the panels, lower ones do not, wherever
+    in a wide matrix they lie; a rebuild chooses as the first build."""
+    import torch
+    A = blocks(64, 1 << 18, bs, 0.1, first_col)
+    h = native.GcooHandle(A).build()
+    B, C = torch.ones(1 << 18, 320, device="cuda"), torch.empty(64, 320, device="cuda")
+    s = torch.cuda.Stream()
+    for _ in range(2):
+        names = [name for name, _ in captured_kernels(s, lambda: h.spdm(B, C, stream=s))]
+        assert len(names) == 1 and kernel in names[0], names
+        h.build()
+        torch.cuda.synchronize()
