@@ -437,8 +437,8 @@ gcoo_status finish_build(gcoo_handle *h, cudaStream_t st)
 // against 54 with the wait, a second memset, a copy of the totals and one
 // launch more); mul->done says so. Only the row walk of a matrix that was not skewed by the
 // last build's totals goes ahead: any launch shape gives it the same chains,
-// and where the arrays turn out too small the placing kernel clears the row
-// pointers, so that it reads nothing and the host multiplies again.
+// and where the arrays turn out too small the placing kernel voids the row
+// pointers, so that it reads and writes nothing and the host multiplies again.
 struct NextMultiply {
     const float *dB;
     int64_t n;

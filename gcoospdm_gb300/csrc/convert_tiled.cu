@@ -511,7 +511,7 @@ place_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
              const int32_t *__restrict__ pref, const int32_t *__restrict__ group_index,
              const int32_t *__restrict__ row_ptr, float *__restrict__ vals, int32_t *__restrict__ rc,
              Entry *__restrict__ packed, const int64_t *__restrict__ d_total, int64_t cap, int64_t packed_cap,
-             int64_t staged_blocks, int32_t *__restrict__ clear_rows)
+             int64_t staged_blocks, int32_t *__restrict__ void_rows)
 {
     grid_wait_previous();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -522,10 +522,10 @@ place_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
     const int64_t total = d_total[0];
     if (d_total[3] != 0 || total < 0 || total > 0x7fffffffLL || total > cap || total + 2 > packed_cap) {
         // staging gave up or the arrays are too small: the host converts again on the two-pass path
-        if (clear_rows)
+        if (void_rows)
             for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i <= m;
                  i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-                clear_rows[i] = 0;
+                void_rows[i] = -1;
         return;
     }
     // from here every position is below total < 2^31: 32-bit offsets
@@ -720,7 +720,7 @@ cudaError_t launch_place(const float *A, int64_t m, int64_t k, int32_t cpg, int3
                          const int32_t *tile_tot, const int32_t *over_list, const unsigned long long *over_count,
                          const int32_t *pref, const int32_t *group_index, const int32_t *row_ptr, float *vals,
                          int32_t *rc, Entry *packed, const int64_t *d_total, int64_t cap, int64_t packed_cap,
-                         int32_t *clear_rows, cudaStream_t st)
+                         int32_t *void_rows, cudaStream_t st)
 {
     const int64_t tiles = conv_tiles(k), S = conv_segments(k);
     const int64_t units = ((m + cpg - 1) / cpg) * tiles;
@@ -737,7 +737,7 @@ cudaError_t launch_place(const float *A, int64_t m, int64_t k, int32_t cpg, int3
 #define GCOO_PLACE(C)                                                                                 \
     le = launch_after(al ? place_kernel<C, true> : place_kernel<C, false>, dim3(grid), dim3(kTileThreads), 0, st, \
         A, m, k, tiles, S, units, slot, stage, tile_tot, over_list, over_count, pref, group_index,    \
-        row_ptr, vals, rc, packed, d_total, cap, packed_cap, staged_blocks, clear_rows)
+        row_ptr, vals, rc, packed, d_total, cap, packed_cap, staged_blocks, void_rows)
     switch (cpg) {
     case 1: GCOO_PLACE(1); break;
     case 2: GCOO_PLACE(2); break;

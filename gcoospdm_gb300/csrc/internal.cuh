@@ -183,13 +183,14 @@ cudaError_t launch_stage(const float *A, int64_t m, int64_t k, int32_t cpg, int3
 // After launch_tile_prefix and launch_row_scan: the GCOO arrays (vals, rc =
 // rows | cols at rc + total) and the packed row order, total = d_total[0] read
 // on the device; writes nothing unless the stage status (d_total[3]) is 0,
-// total <= cap and total + 2 <= packed_cap; then, with clear_rows (m + 1 row
-// pointers, may be null), those are zeroed: no row has entries to read.
+// total <= cap and total + 2 <= packed_cap; then, with void_rows (m + 1 row
+// pointers, may be null), those are set to -1: no row has entries to read, and
+// a multiply enqueued behind (the row walk) leaves C as it is.
 cudaError_t launch_place(const float *A, int64_t m, int64_t k, int32_t cpg, int32_t slot, const uint2 *stage,
                          const int32_t *tile_tot, const int32_t *over_list, const unsigned long long *over_count,
                          const int32_t *pref, const int32_t *group_index, const int32_t *row_ptr, float *vals,
                          int32_t *rc, Entry *packed, const int64_t *d_total, int64_t cap, int64_t packed_cap,
-                         int32_t *clear_rows, cudaStream_t st);
+                         int32_t *void_rows, cudaStream_t st);
 
 // ---- FP32 multiply (spdm_fp32.cu) ------------------------------------------------------
 int device_sms(); // SMs of the current device (152 on a GB300)

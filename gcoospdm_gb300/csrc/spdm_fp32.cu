@@ -295,6 +295,8 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 
     const int64_t gs = row_ptr[r0];
     const int64_t ge = row_ptr[r_end];
+    if (gs < 0)
+        return; // enqueued behind a conversion that did not fit (launch_place): C stays as it is
     int64_t rs = 0, re = 0;
     if (has_row) {
         rs = row_ptr[row];
