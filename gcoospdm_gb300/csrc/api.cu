@@ -328,46 +328,53 @@ gcoo_status gcoo_create(gcoo_handle **out, const float *dA, int64_t m, int64_t k
 
 namespace {
 
+constexpr size_t kReadbackWords = 8; // of a handle's page-locked readback
+
 // Whether the FP32 multiply of a matrix whose groups share columns takes 16
 // rows per B load. Groups of four rows that share only part of their columns
 // (fewer than 3 of the 4 rows on average) share with their neighbours much
 // as among themselves: yes. Groups that share nearly all of them are blocks
 // of 4 rows or higher: only where the blocks reach across the 16 rows, which
-// a sample of panels tells (one more readback, for such matrices only). A
-// panel's staging costs about the same whatever its window holds: at 2 %
-// density (16 x 16 blocks, 4096^2) panels take 36 against the group walk's 53 us
-// at n = 256 and 54 against 60 at n = 1024, so below 1/64 the group walk stays.
-gcoo_status choose_panels(gcoo_handle *h, cudaStream_t st)
+// a sample of panels tells: share, when the build has read one back with its
+// totals (a steady loop's on such a matrix), else one more readback. A panel's
+// staging costs about the same whatever its window holds: at 2 % density (16 x
+// 16 blocks, 4096^2) panels take 36 against the group walk's 53 us at n = 256
+// and 54 against 60 at n = 1024, so below 1/64 the group walk stays.
+gcoo_status choose_panels(gcoo_handle *h, cudaStream_t st, const int64_t *share)
 {
-    h->panels = false;
+    h->panels = h->sampled = false;
     if (!h->seg_prefix || !group_order_chosen(h) || 64.0 * static_cast<double>(h->nnz) < static_cast<double>(h->m) * h->k)
         return GCOO_SUCCESS;
     if (h->nnz < 3 * h->distinct_cols) {
         h->panels = true;
         return GCOO_SUCCESS;
     }
-    if (!h->long_count.ensure(2))
-        return fail(GCOO_ERROR_ALLOC, "device allocation of the sharing counts failed");
-    unsigned long long share[2] = {0, 0};
-    GCOO_CUDA(cudaMemsetAsync(h->long_count.ptr, 0, sizeof(share), st));
-    GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m, h->long_count.ptr, st));
-    GCOO_CUDA(cudaMemcpyAsync(share, h->long_count.ptr, sizeof(share), cudaMemcpyDeviceToHost, st));
-    GCOO_CUDA(cudaStreamSynchronize(st));
+    h->sampled = true;
+    int64_t own[2] = {0, 0};
+    if (!share) {
+        if (!h->long_count.ensure(2))
+            return fail(GCOO_ERROR_ALLOC, "device allocation of the sharing counts failed");
+        GCOO_CUDA(cudaMemsetAsync(h->long_count.ptr, 0, sizeof(own), st));
+        GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m, h->long_count.ptr, st));
+        GCOO_CUDA(cudaMemcpyAsync(own, h->long_count.ptr, sizeof(own), cudaMemcpyDeviceToHost, st));
+        GCOO_CUDA(cudaStreamSynchronize(st));
+        share = own;
+    }
     h->panels = share[1] > 0 && share[0] >= 12 * share[1];
     return GCOO_SUCCESS;
 }
 
 // The end of every successful build: plans derived from the old arrays go,
 // and for a skewed matrix the list of its long rows (multiplied by their own
-// kernel) is collected, one readback of its length.
-gcoo_status finish_build(gcoo_handle *h, cudaStream_t st)
+// kernel) is collected, one readback of its length. share: see choose_panels.
+gcoo_status finish_build(gcoo_handle *h, cudaStream_t st, const int64_t *share = nullptr)
 {
     if (h->tc)
         destroy_tc_plan(h->tc);
     h->tc = nullptr;
     destroy_left_plan(h->left);
     h->left = nullptr;
-    const gcoo_status ps = choose_panels(h, st);
+    const gcoo_status ps = choose_panels(h, st, share);
     if (ps != GCOO_SUCCESS)
         return ps;
     h->n_long = 0;
@@ -390,7 +397,7 @@ gcoo_status finish_build(gcoo_handle *h, cudaStream_t st)
             GCOO_CUDA(launch_split_plan(h->row_ptr.ptr, h->long_rows.ptr, d_cnt, cap, h->piece_first.ptr,
                                         h->piece_row.ptr, pcap, h->piece_total.ptr, st));
         }
-        if (!h->readback && cudaMallocHost(&h->readback, 4 * sizeof(int64_t)) != cudaSuccess) {
+        if (!h->readback && cudaMallocHost(&h->readback, kReadbackWords * sizeof(int64_t)) != cudaSuccess) {
             h->readback = nullptr;
             return fail(GCOO_ERROR_ALLOC, "page-locked allocation of the readback words failed");
         }
@@ -465,7 +472,8 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
         (!one_scan && !h->scratch.ensure(scan_scratch_elems(h->m))) || !h->status.ensure(2 + 8 * 2))
         return fail(GCOO_ERROR_ALLOC, "device allocation of the GCOO index arrays failed");
     // [0] total nnz, [1] longest row, [2] distinct group columns, [3] staging status, [4] overflowed tiles,
-    // [5] ticket of the prefix-and-scan kernel; behind the status word: one memset clears all
+    // [5] ticket of the prefix-and-scan kernel, [6] entries and [7] distinct columns of the sampled panels;
+    // behind the status word: one memset clears all
     int64_t *d_total = reinterpret_cast<int64_t *>(h->status.ptr + 2);
     GCOO_CUDA(cudaMemsetAsync(h->status.ptr, 0, 8 + 8 * sizeof(int64_t), st));
     unsigned int *ticket = reinterpret_cast<unsigned int *>(d_total + 5);
@@ -480,7 +488,7 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
             !h->stage.ensure(static_cast<size_t>(tiles) * static_cast<size_t>(slot)) ||
             !h->tile_tot.ensure(static_cast<size_t>(tiles)) || !h->over_list.ensure(static_cast<size_t>(tiles)))
             return fail(GCOO_ERROR_ALLOC, "device allocation of the staged conversion state failed");
-        if (!h->readback && cudaMallocHost(&h->readback, 4 * sizeof(int64_t)) != cudaSuccess) {
+        if (!h->readback && cudaMallocHost(&h->readback, kReadbackWords * sizeof(int64_t)) != cudaSuccess) {
             h->readback = nullptr;
             return fail(GCOO_ERROR_ALLOC, "page-locked allocation of the readback words failed");
         }
@@ -502,14 +510,19 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
             GCOO_CUDA(launch_row_scan_max(h->row_ptr.ptr, h->m, cpg, h->group_index(), h->nnz_per_group(), d_total,
                                           h->scratch.ptr, h->status.ptr, st));
         }
+        // a matrix that needed the sample of its panels last time probably does again
+        const bool sample = h->sampled;
         // placed on the device before the one readback (the kernel checks the fit itself)
         const int64_t packed_cap = static_cast<int64_t>(h->packed.count);
         GCOO_CUDA(launch_place(h->dA, h->m, h->k, cpg, slot, h->stage.ptr, h->tile_tot.ptr, h->over_list.ptr,
                                over_count, h->tile_cnt.ptr, h->group_index(), h->row_ptr.ptr, h->vals.ptr, h->rc.ptr,
-                               h->packed.ptr, d_total, cap, packed_cap, ahead ? h->row_ptr.ptr : nullptr, st));
+                               h->packed.ptr, d_total, cap, packed_cap, ahead || sample ? h->row_ptr.ptr : nullptr, st));
+        if (sample)
+            GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m,
+                                         reinterpret_cast<unsigned long long *>(d_total + 6), st));
         const int64_t *t3 = h->readback;
-        if (!one_scan)
-            GCOO_CUDA(cudaMemcpyAsync(h->readback, d_total, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        if (!one_scan || sample)
+            GCOO_CUDA(cudaMemcpyAsync(h->readback, d_total, kReadbackWords * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         GCOO_CUDA(cudaEventRecord(h->ev_totals, st));
         if (ahead) {
             const gcoo_status s = spdm_fp32(h, mul->dB, mul->n, mul->dC, st, nullptr);
@@ -529,7 +542,7 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
             h->seg_prefix = true;
             if (mul)
                 mul->done = ahead;
-            return finish_build(h, st);
+            return finish_build(h, st, sample ? t3 + 6 : nullptr);
         }
         GCOO_CUDA(cudaMemsetAsync(d_total, 0, 8 * sizeof(int64_t), st));
     }

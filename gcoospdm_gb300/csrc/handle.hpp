@@ -41,6 +41,7 @@ struct gcoo_handle {
     gcoo::DevBuf<gcoo::Entry> packed; // row order, nnz + 2 (16-byte padded)
     gcoo::DevBuf<int32_t> tile_cnt;  // per-(row, column segment) counts of the tiled conversion, then their prefix
     bool panels = false;             // the FP32 multiply takes 16 rows per B load (api.cu: choose_panels)
+    bool sampled = false;            // ... which the last build learnt from a sample of panels
     bool seg_prefix = false;         // tile_cnt holds the built arrays' prefixes (built by the tiled conversion)
     gcoo::DevBuf<uint2> stage;       // staged rebuild: each tile's entries in a fixed slot
     gcoo::DevBuf<int32_t> tile_tot;  // staged rebuild: entries per tile, -1 when it overflowed

@@ -202,9 +202,11 @@ gcoo_status gcoo_prepare(gcoo_handle *h, int64_t n, gcoo_precision prec, void *s
 /* mutiplyBy() (src/ShGCOOSpDM.cu:131-180): conversion + multiply in one call
  * (FP32). Reuses the handle's arrays when they are large enough, so a steady
  * loop allocates nothing; it waits once for the nnz, as the reference does
- * (the multiply may still be running on `stream` when it returns). When the
- * conversion fails (more nonzeros than the format holds, no memory for them),
- * C keeps its contents. */
+ * (the multiply may still be running on `stream` when it returns). It waits a
+ * second time for the plan of a matrix whose rows are very uneven, and, on a
+ * handle's first call or when the matrix has turned to blocks since the call
+ * before, for a sample of those. When the conversion fails (more nonzeros
+ * than the format holds, no memory for them), C keeps its contents. */
 gcoo_status gcoo_multiply_by(gcoo_handle *h, const float *dB, int64_t n, float *dC, void *stream);
 
 gcoo_status gcoo_destroy(gcoo_handle *h);

@@ -1,4 +1,5 @@
-"""GPU: by what evidence a build chooses the walk of sixteen rows."""
+"""GPU: how a build learns whether sixteen rows share their columns: by what
+evidence, and without holding up a multiply that is already under way."""
 from __future__ import annotations
 
 import pytest
@@ -33,3 +34,22 @@ def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
         assert len(names) == 1 and kernel in names[0], names
         h.build()
         torch.cuda.synchronize()
+
+
+def test_multiply_by_returns_with_the_multiply_under_way(native):
+    """A steady loop on a block matrix whose width takes the row walk (here
+    milliseconds of it): the call waits for the conversion's totals only."""
+    import torch
+    A = blocks(65536, 8192, 16, 0.05)
+    B, C = torch.ones(8192, 128, device="cuda"), torch.empty(65536, 128, device="cuda")
+    h = native.GcooHandle(A)
+    h.multiply_by(B, C)
+    s = torch.cuda.current_stream()
+    running = []
+    for _ in range(4):
+        torch.cuda.synchronize()
+        h.multiply_by(B, C)
+        running.append(not s.query())
+    torch.cuda.synchronize()
+    assert sum(running) >= 3, running
+    assert torch.equal(C, A.sum(1, keepdim=True).expand(-1, 128))  # whole numbers: exact
