@@ -388,20 +388,24 @@ spdm_panel_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
 
 // How many rows of a panel share a column, on up to gridDim.x panels spread
 // over the matrix: out[0] += entries, out[1] += distinct columns, both of
-// kShareCols columns from each panel's first one with an entry on.
-constexpr int kShareCols = 1 << 17;
-constexpr int kSharePanels = 64;
+// kShareCols columns from each panel's first one with an entry on. A CTA has
+// one panel, and the build waits for it: many threads, eight entries' loads of
+// each in flight, a byte per column (8192^2 at 25 % in 16 x 16 blocks, 32768
+// entries a panel: 9.5 us; with 256 threads 42, 1024 threads that set bits
+// with atomics 17).
+constexpr int kShareCols = 1 << 15;
+constexpr int kSharePanels = 64, kShareThreads = 1024, kShareBatch = 8;
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kShareThreads)
 panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m, int64_t panels,
                    unsigned long long *__restrict__ out)
 {
-    __shared__ uint32_t s_seen[kShareCols / 32];
+    __shared__ __align__(16) uint8_t s_seen[kShareCols]; // 0 or 1: stores of 1 need no atomics
     __shared__ int s_first;
     const int64_t r0 = (blockIdx.x * panels / gridDim.x) * kPanelRows;
     const int64_t r1 = r0 + kPanelRows < m ? r0 + kPanelRows : m;
-    for (int i = threadIdx.x; i < kShareCols / 32; i += blockDim.x)
-        s_seen[i] = 0;
+    for (int i = threadIdx.x; i < kShareCols / 16; i += kShareThreads)
+        reinterpret_cast<uint4 *>(s_seen)[i] = make_uint4(0, 0, 0, 0);
     if (threadIdx.x == 0)
         s_first = 0x7fffffff;
     __syncthreads();
@@ -410,16 +414,24 @@ panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__
         atomicMin(&s_first, packed[row_ptr[r]].col);
     __syncthreads();
     int entries = 0, distinct = 0;
-    for (int64_t e = row_ptr[r0] + threadIdx.x; e < row_ptr[r1]; e += blockDim.x) {
-        const int c = packed[e].col - s_first;
-        if (c < kShareCols) {
-            ++entries;
-            atomicOr(&s_seen[c >> 5], 1u << (c & 31));
+    const int64_t end = row_ptr[r1];
+    for (int64_t e0 = row_ptr[r0] + threadIdx.x; e0 < end; e0 += kShareThreads * kShareBatch) {
+        int c[kShareBatch];
+#pragma unroll
+        for (int u = 0; u < kShareBatch; ++u) {
+            const int64_t e = e0 + u * kShareThreads;
+            c[u] = e < end ? packed[e].col - s_first : kShareCols;
         }
+#pragma unroll
+        for (int u = 0; u < kShareBatch; ++u)
+            if (c[u] < kShareCols) {
+                ++entries;
+                s_seen[c[u]] = 1;
+            }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kShareCols / 32; i += blockDim.x)
-        distinct += __popc(s_seen[i]);
+    for (int i = threadIdx.x; i < kShareCols / 4; i += kShareThreads)
+        distinct += __popc(reinterpret_cast<const uint32_t *>(s_seen)[i]);
     entries = __reduce_add_sync(0xffffffffu, entries);
     distinct = __reduce_add_sync(0xffffffffu, distinct);
     if ((threadIdx.x & 31) == 0) {
@@ -435,7 +447,7 @@ cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int6
 {
     const int64_t panels = (m + kPanelRows - 1) / kPanelRows;
     const unsigned grid = static_cast<unsigned>(panels < kSharePanels ? panels : kSharePanels);
-    panel_share_kernel<<<grid, 256, 0, st>>>(packed, row_ptr, m, panels, out);
+    panel_share_kernel<<<grid, kShareThreads, 0, st>>>(packed, row_ptr, m, panels, out);
     count_launches(1);
     return cudaGetLastError();
 }
