@@ -36,6 +36,27 @@ def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
         torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("m,k,rows,n,kernel", [
+    (2048, 2048, 2, 320, "spdm_panel_kernel"), (2048, 2048, 2, 1024, "spdm_fp32_kernel"),
+    (2048, 2048, 8, 1024, "spdm_panel_kernel"), (2048, 8192, 2, 1024, "spdm_group_kernel"),
+    (2048, 2048, 2, 1001, "spdm_panel_kernel"), (2048, 2048, 2, 128, "spdm_fp32_kernel")])
+def test_choice_by_the_gain(native, m, k, rows, n, kernel):
+    """Blocks of two rows at 15 %, half of the columns shared by a group's rows
+    and few more by a panel's: the panels where they gain enough on the
+    groups, the same bits by every walk."""
+    import torch
+    A = blocks(m, k, rows, 0.15)
+    if rows == 8:
+        A *= torch.rand(m, k, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda") < 0.6
+    h = native.GcooHandle(A).build()
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    B, C = torch.randn(k, n, generator=gen, device="cuda"), torch.empty(m, n, device="cuda")
+    s = torch.cuda.Stream()
+    names = [name for name, _ in captured_kernels(s, lambda: h.spdm(B, C, stream=s))]
+    assert len(names) == 1 and kernel in names[0], names
+    assert torch.equal(h.spdm(B, C), native.GcooHandle(A, fp32_order="rows").build().spdm(B))
+
+
 def test_multiply_by_returns_with_the_multiply_under_way(native):
     """A steady loop on a block matrix whose width takes the row walk (here
     milliseconds of it): the call waits for the conversion's totals only."""
