@@ -122,66 +122,42 @@ gcoo_status ensure_split_work(gcoo_handle *h, int64_t n)
     return GCOO_SUCCESS;
 }
 
-// What a panel has to gain on its groups (h->panel_gain: groups' columns per
-// panel column, so how many visits of a B row by a group one by a panel
-// replaces) to be faster, by the width of B and the panels' CTAs per SM.
-// Group walk over panels' time at gains of about 1.1, 1.3, 1.5, 1.75, 1.95,
-// 2.1, 3 (blocks of 2, 3, 4, 8 rows, aligned or not, with holes, unstructured):
-//   8192^2, n  512: .92 1.09 1.15 1.30 1.58 1.73 2.18   3.4 CTAs per SM
-//           n 1024: .66  .77  .81  .91 1.11 1.22 1.59   6.7
-//   4096^2, n 1024: .71  .83  .88  .94 1.19 1.31 1.67   3.4
-//   3000^2, n  512: .72  .80  .89 1.02 1.13 1.23 1.53   1.2
-//           n 1024: .59  .67  .74  .87  .95 1.05 1.32   2.5
-//   2048^2, n  512: .97 1.11 1.21 1.37 1.56 1.70 1.96   0.8
-//           n 1024: .58  .66  .74  .87  .92  .99 1.27   1.7
-//           n  256: .90 1.01 1.10 1.26 1.40 1.53 1.83   0.8
-// One to two CTAs per SM: the last SMs with two set the time.
-static double panel_gain_needed(const gcoo_handle *h, int64_t n, bool rows_instead)
-{
-    if (n <= 256)
-        return 1.35;
-    const double per_sm = static_cast<double>(panel_ctas(h->m, n)) / device_sms();
-    if (per_sm <= 1.0)
-        return rows_instead ? 1.3 : 1.2; // rows_instead: the alternative is the row walk, else the slower group walk
-    if (n <= 512)
-        return std::max(1.3, 1.1 * ceil(per_sm) / per_sm);
-    return per_sm <= 2.0 ? 2.1 : (per_sm <= 3.0 ? 2.0 : 1.8);
-}
-
-// Walk of a matrix whose groups share columns, by the width of B. Measured
-// at 4096^2 (us; row walk / group walk / panels):
-//   16 x 16 blocks, 25 %: n 64 199 / 366 / 139, n 128 215 / 380 / 147, n 256 331 / 397 / 106, n 1024 1030 / 561 / 230
-//   16 x 16 blocks,  5 %: n 64  36 /  91 /  59, n 128  42 /  93 /  57, n 256  60 /  97 /  46, n 1024  158 / 137 /  74
-//   4 x 4 blocks, 10 %:   n 128 59 / 154, n 256 103 / 162, n 300 - / 127, n 1024 333 / 235
-//   unstructured 30 %:    n 128 244 / 1178 / 345, n 256 375 / 1200 / 344, n 1024 1169 / 1548 / 937
-//   2 x 2 blocks, 10 %:   n 256 85 / 357 / 206, n 512 137 / 386 / 376, n 1024 267 / 451 / 542
-//   2 x 2 blocks,  2 %:   n 256 23 /  85 /  76, n 512  35 /  92 / 117, n 1024  61 / 107 / 172
-// Narrow B: one staging of a panel's or a group's entries serves few columns
-// and the row walk is faster, long rows in panels aside; the group walk is
-// slow there with 8 columns per lane (n % 8 == 0) only. Groups that share only
-// part of their columns and panels that gain too little on them: the row walk
-// as well, up to some hundred entries per row (8192^2 in 4 x 4 blocks with 40 %
-// holes, 819 a row: n 512 700 / 1092 / 990, n 1024 1380 / 1296 / 1656).
+// Walk of a matrix whose groups share columns. The row walk reads a B row once
+// per entry, the group walk once per column of a group (four rows), the panel
+// walk once per column of sixteen rows, but their lanes also wait for the
+// staging and the masks, and they have fewer CTAs. Measured on 4783 multiplies
+// (64^2 to 10000^2, blocks of 2 to 64 rows, aligned or not, with holes,
+// unstructured from 25 %, n 1 to 2048; rows / groups / panels, us):
+//   4096^2, 16 x 16 blocks, 25 %: n 128 215 / 380 / 147, n 256 331 / 397 / 106, n 1024 1030 / 561 / 230
+//           16 x 16 blocks,  5 %: n 128  42 /  93 /  57, n 256  60 /  97 /  46, n 1024  158 / 137 /  74
+//           the same, 40 % holes: n 256  48 / 186 /  70, n 512  77 / 197 /  93, n 1024  140 / 229 / 133
+//           4 x 4 blocks, 10 %:   n 128  59 / 154,       n 256 103 / 162,       n 1024  333 / 235
+//           unstructured 30 %:    n 128 244 /1178 / 345, n 512 504 /1347 / 637, n 1024 1066 /1550 / 928
+//           2 x 2 blocks, 10 %:   n 256  85 / 357 / 206, n 512 137 / 386 / 376, n 1024  267 / 451 / 542
+//   8192^2, 2 x 2 blocks, 25 %:   n 256 1557 /2425 / 927, n 1024 5791 /3156 /2856
+//   2048^2, 16 x 16, 40 % holes:  n 256  34 / 141 /  60, n 1024 78 / 154 / 84, n 2048 140 / 228 / 120
+// Panels win with many rows per panel column (share) and much work, so that
+// their CTAs fill the GPU: share^3 * nnz * n >= 2.9e11, the work counted
+// twice for long rows, which the row walk stages piecewise. Groups win for
+// blocks of four rows, wide and large. By this rule the multiplies take 1.3 %
+// longer than by the best walk of each (1 in 100 more than 1.3 times as long),
+// by the row walk alone 3 % and up to 6 times, by the group walk alone twice.
 enum SharedWalk { kWalkRows, kWalkGroups, kWalkPanels };
 
 static SharedWalk shared_walk(const gcoo_handle *h, int64_t n, uintptr_t b, uintptr_t c)
 {
+    if (h->p.vec != 0)
+        return kWalkGroups; // columns per lane chosen by the caller
+    const double share = h->panel_share; // 0: no panels
+    const double sharing4 = static_cast<double>(h->nnz) / static_cast<double>(h->distinct_cols);
+    if (h->p.fp32_order == 2)
+        return panel_ok(n) && share >= 1.75 * sharing4 ? kWalkPanels : kWalkGroups;
+    const double work = static_cast<double>(h->nnz) * static_cast<double>(n);
+    const bool long_rows = h->nnz >= 1600 * h->m;
+    if (panel_ok(n) && n >= 96 && share >= 4.0 && share * share * share * work * (long_rows ? 2 : 1) >= 2.9e11)
+        return kWalkPanels;
     const bool vec4 = n % 4 == 0 && !((b | c) & 15);
-    const bool forced = h->p.fp32_order == 2;
-    if (h->panels && h->p.vec == 0 && panel_ok(n)) {
-        const bool long_rows = h->nnz >= 1000 * h->m;
-        if (!vec4)
-            return forced || n >= 192 ? kWalkPanels : kWalkGroups;
-        if (n <= 128)
-            return forced || long_rows ? kWalkPanels : kWalkRows;
-        const bool rows_instead = !forced && h->nnz < (n <= 512 ? 1000 : 600) * h->m;
-        if (h->panel_gain >= panel_gain_needed(h, n, rows_instead) || (n <= 256 && long_rows))
-            return kWalkPanels;
-        return rows_instead ? kWalkRows : kWalkGroups;
-    }
-    if (!forced && vec4 && n % 8 == 0 && n <= 256 && h->p.vec == 0)
-        return kWalkRows;
-    return kWalkGroups;
+    return vec4 && n >= 640 && sharing4 >= 3.3 && work >= 3e8 ? kWalkGroups : kWalkRows;
 }
 
 static SharedWalk fp32_walk(const gcoo_handle *h, int64_t n, const float *dB, const float *dC)
@@ -367,20 +343,17 @@ namespace {
 
 constexpr size_t kReadbackWords = 8; // of a handle's page-locked readback
 
-// Whether the FP32 multiply of a matrix whose groups share columns may take
-// 16 rows per B load, and what that gains on the groups. Groups of four rows
-// that share only part of their columns (fewer than 3 of the 4 rows on
-// average) may, whatever their neighbours share: the gain tells. Groups that
-// share nearly all of them are blocks of 4 rows or higher: only where the
-// blocks reach across the 16 rows. A sample of panels tells both: share, when
+// How many rows of a panel (16 rows) share a column, for shared_walk; 0 where
+// the panels cannot run or never pay. A sample of panels tells: share, when
 // the build has read one back with its totals (a steady loop's on such a
 // matrix), else one more readback. A panel's staging costs about the same
 // whatever its window holds: at 2 % density (16 x 16 blocks, 4096^2) panels
 // take 36 against the group walk's 53 us at n = 256 and 54 against 60 at n =
-// 1024, so below 1/64 the group walk stays.
+// 1024, so below 1/64 they are left out.
 gcoo_status choose_panels(gcoo_handle *h, cudaStream_t st, const int64_t *share)
 {
-    h->panels = h->sampled = false;
+    h->panel_share = 0.0;
+    h->sampled = false;
     if (!h->seg_prefix || !group_order_chosen(h) || 64.0 * static_cast<double>(h->nnz) < static_cast<double>(h->m) * h->k)
         return GCOO_SUCCESS;
     h->sampled = true;
@@ -394,11 +367,8 @@ gcoo_status choose_panels(gcoo_handle *h, cudaStream_t st, const int64_t *share)
         GCOO_CUDA(cudaStreamSynchronize(st));
         share = own;
     }
-    if (share[1] <= 0)
-        return GCOO_SUCCESS;
-    const double per_column = static_cast<double>(share[0]) / static_cast<double>(share[1]);
-    h->panels = h->nnz < 3 * h->distinct_cols || per_column >= 12.0;
-    h->panel_gain = per_column * static_cast<double>(h->distinct_cols) / static_cast<double>(h->nnz);
+    if (share[1] > 0)
+        h->panel_share = static_cast<double>(share[0]) / static_cast<double>(share[1]);
     return GCOO_SUCCESS;
 }
 

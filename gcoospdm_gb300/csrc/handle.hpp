@@ -40,8 +40,7 @@ struct gcoo_handle {
     gcoo::DevBuf<int32_t> rc;        // rows[nnz] | cols[nnz]
     gcoo::DevBuf<gcoo::Entry> packed; // row order, nnz + 2 (16-byte padded)
     gcoo::DevBuf<int32_t> tile_cnt;  // per-(row, column segment) counts of the tiled conversion, then their prefix
-    bool panels = false;             // the FP32 multiply may take 16 rows per B load (api.cu: choose_panels)
-    double panel_gain = 0.0;         // ... and then visits a B row this many times less often than groups of 4
+    double panel_share = 0.0;        // entries per column of 16-row panels (api.cu: choose_panels), 0: no panels
     bool sampled = false;            // ... which the last build learnt from a sample of panels
     bool seg_prefix = false;         // tile_cnt holds the built arrays' prefixes (built by the tiled conversion)
     gcoo::DevBuf<uint2> stage;       // staged rebuild: each tile's entries in a fixed slot

@@ -258,7 +258,6 @@ cudaError_t launch_spdm_fp32_group(const float *vals, const int32_t *rows, const
 // row-ordered entries and the tiled conversion's segment prefixes
 // (pref[r * conv_segments(k) + s]).
 bool panel_ok(int64_t n);
-int64_t panel_ctas(int64_t m, int64_t n); // of the multiply's launch
 // Sampled sharing inside 16-row panels: out[0] += entries, out[1] += distinct
 // (panel, column) pairs (zeroed by the caller).
 cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, unsigned long long *out,

@@ -35,7 +35,6 @@
 // ms. Lanes of 8 rows x 8 columns 0.81 ms, 16 x 8 0.79 ms, four CTAs per SM at
 // 128 registers 0.80 ms, the next window's entries copied ahead 0.83 ms, a ring
 // of four 0.98 ms, of sixteen 0.93 ms.
-#include <algorithm>
 #include <type_traits>
 
 #include "internal.cuh"
@@ -456,22 +455,16 @@ cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int6
 // Wider B stays with the group walk, whose tile count decides what is possible
 bool panel_ok(int64_t n) { return n <= 1 << 20; }
 
-static int panel_warps(int64_t n) { return static_cast<int>(std::min<int64_t>((n + kCols - 1) / kCols, kMaxWarps)); }
-
-int64_t panel_ctas(int64_t m, int64_t n)
-{
-    const int64_t cols = panel_warps(n) * kCols;
-    return (m + kPanelRows - 1) / kPanelRows * ((n + cols - 1) / cols);
-}
-
 cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, const int32_t *pref, int64_t m,
                                    int64_t k, const float *B, int64_t n, float *C, cudaStream_t st)
 {
     if (m <= 0 || n <= 0)
         return cudaSuccess;
     const bool vec4 = n % 4 == 0 && !((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15);
-    const int warps = panel_warps(n);
-    const int64_t nx = (m + kPanelRows - 1) / kPanelRows, ny = panel_ctas(m, n) / nx;
+    const int64_t strips = (n + kCols - 1) / kCols;
+    const int warps = strips < kMaxWarps ? static_cast<int>(strips) : kMaxWarps;
+    const int64_t ny = (strips + warps - 1) / warps;
+    const int64_t nx = (m + kPanelRows - 1) / kPanelRows;
     if (!panel_ok(n) || nx > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
     const dim3 grid(static_cast<unsigned>(nx), static_cast<unsigned>(ny));

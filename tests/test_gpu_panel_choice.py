@@ -25,9 +25,9 @@ def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
     """Blocks as high as a panel take the panels, lower ones do not, wherever
     in a wide matrix they lie; a rebuild chooses as the first build."""
     import torch
-    A = blocks(64, 1 << 18, bs, 0.1, first_col)
+    A = blocks(64, 1 << 18, bs, 0.06, first_col)
     h = native.GcooHandle(A).build()
-    B, C = torch.ones(1 << 18, 320, device="cuda"), torch.empty(64, 320, device="cuda")
+    B, C = torch.ones(1 << 18, 1024, device="cuda"), torch.empty(64, 1024, device="cuda")
     s = torch.cuda.Stream()
     for _ in range(2):
         names = [name for name, _ in captured_kernels(s, lambda: h.spdm(B, C, stream=s))]
@@ -36,25 +36,27 @@ def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
         torch.cuda.synchronize()
 
 
-@pytest.mark.parametrize("m,k,rows,n,kernel", [
-    (2048, 2048, 2, 320, "spdm_panel_kernel"), (2048, 2048, 2, 1024, "spdm_fp32_kernel"),
-    (2048, 2048, 8, 1024, "spdm_panel_kernel"), (2048, 8192, 2, 1024, "spdm_group_kernel"),
-    (2048, 2048, 2, 1001, "spdm_panel_kernel"), (2048, 2048, 2, 128, "spdm_fp32_kernel")])
-def test_choice_by_the_gain(native, m, k, rows, n, kernel):
-    """Blocks of two rows at 15 %, half of the columns shared by a group's rows
-    and few more by a panel's: the panels where they gain enough on the
-    groups, the same bits by every walk."""
+@pytest.mark.parametrize("rows,holes,n,kernel", [
+    (2, 0.0, 1024, "spdm_fp32_kernel"), (2, 0.0, 1001, "spdm_fp32_kernel"), (2, 0.0, 128, "spdm_fp32_kernel"),
+    (4, 0.0, 1024, "spdm_group_kernel"), (4, 0.0, 1001, "spdm_fp32_kernel"), (4, 0.0, 512, "spdm_fp32_kernel"),
+    (16, 0.4, 1024, "spdm_panel_kernel"), (16, 0.4, 1001, "spdm_panel_kernel"), (16, 0.4, 256, "spdm_fp32_kernel")])
+@pytest.mark.parametrize("k", [2048, 2047])
+def test_choice_by_sharing_and_work(native, rows, holes, n, kernel, k):
+    """Blocks of several heights at 15 %: the walk by how many rows share a
+    column and by the work, whatever the rows' alignment; the same bits by
+    every walk."""
     import torch
-    A = blocks(m, k, rows, 0.15)
-    if rows == 8:
-        A *= torch.rand(m, k, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda") < 0.6
+    A = blocks(2048, 2048, rows, 0.15)[:, :k].contiguous()
+    A *= torch.rand(2048, k, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda") >= holes
     h = native.GcooHandle(A).build()
     gen = torch.Generator(device="cuda").manual_seed(3)
-    B, C = torch.randn(k, n, generator=gen, device="cuda"), torch.empty(m, n, device="cuda")
+    B, C = torch.randn(k, n, generator=gen, device="cuda"), torch.empty(2048, n, device="cuda")
     s = torch.cuda.Stream()
     names = [name for name, _ in captured_kernels(s, lambda: h.spdm(B, C, stream=s))]
     assert len(names) == 1 and kernel in names[0], names
-    assert torch.equal(h.spdm(B, C), native.GcooHandle(A, fp32_order="rows").build().spdm(B))
+    want = h.spdm(B, C).clone()
+    for order in ("rows", "groups"):
+        assert torch.equal(want, native.GcooHandle(A, fp32_order=order).build().spdm(B)), order
 
 
 def test_multiply_by_returns_with_the_multiply_under_way(native):
