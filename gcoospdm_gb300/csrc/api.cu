@@ -98,10 +98,9 @@ static gcoo_status check_n(int64_t n)
     return GCOO_SUCCESS;
 }
 
-// Whether the FP32 multiply (and the BF16 / FP8-B forms on the FMA engine)
-// walks groups in GCOO order (one B load per column shared by a group's rows)
-// instead of rows: forced by fp32_order, else when the conversion saw at
-// least 1.5 entries per distinct (group, column) pair.
+// Whether the groups share enough columns for the FP32 multiply to consider
+// the group and panel walks (shared_walk): forced by fp32_order, else when the
+// conversion saw at least 1.5 entries per distinct (group, column) pair.
 bool group_order_chosen(const gcoo_handle *h)
 {
     if (h->coo || !group_order_ok(h->p.rows_per_group) || h->p.fp32_order == 1)

@@ -75,10 +75,11 @@ typedef struct gcoo_params {
     int32_t engine;         /* gcoo_engine for non-FP32 forms               */
     int32_t depth;          /* B-load pipelining: 0 auto, 1 off, 2 on        */
     int32_t fp32_order;     /* walk of the FP32 multiply and of the BF16 /
-                               FP8-B forms on the FMA engine: 0 auto, 1 rows
-                               (packed row order), 2 groups (GCOO order, one
-                               B load per column shared by a group's rows;
-                               groups of 4 rows). Both give the same bits. */
+                               FP8-B forms on the FMA engine: 0 auto (by the
+                               matrix and n), 1 rows (packed row order), 2
+                               several rows per B load: groups of 4 rows (GCOO
+                               order) or, FP32 only, panels of 16 where their
+                               rows share more. All give the same bits. */
     int32_t fp32_sum;       /* gcoo_fp32_sum: summation of the FP32
                                multiply's long rows (at least 256 entries,
                                skewed matrices only)                      */
