@@ -404,8 +404,8 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
                      const int32_t *__restrict__ tile_panel,
                      const uint16_t *__restrict__ a_hi, const uint16_t *__restrict__ a_lo,
                      const uint16_t *__restrict__ b_hi, const uint16_t *__restrict__ b_lo, int64_t m, int64_t n,
-                     int64_t kb, int64_t tiles, const ShareCut cut, float *__restrict__ C, float *__restrict__ part,
-                     uint32_t *__restrict__ status)
+                     int64_t kb, int64_t panels, int64_t tiles, const ShareCut cut, bool shares,
+                     float *__restrict__ C, float *__restrict__ part, uint32_t *__restrict__ status)
 {
     constexpr int N = kSplitN, S = kSplitS;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -447,7 +447,8 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
     // products to bank 1, so each correction is rounded at its own (2^-8
     // smaller) magnitude, not at the running total's; the epilogue adds bank
     // 1 to bank 0.
-    ShareWalk sh(pf, tile_panel, kb, tiles, cut, blockIdx.x);
+    ShareWalk sh = shares ? ShareWalk(pf, tile_panel, kb, tiles, cut, blockIdx.x)
+                          : ShareWalk(pf, tile_panel, kb, tiles, panels, blockIdx.x);
 
     // Warps 4 and 5 walk together and one elected lane issues (a lane's own
     // branch costs the descriptors' moves to uniform registers at each MMA)
@@ -535,6 +536,13 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
     } else {
         // epilogue: warp w owns TMEM lanes 32w..32w+31 = panel rows
         uint32_t piece = 0;
+        if (!shares && sh.w == sh.end) {
+            // panel without entries: its C rows are zero, a warp's stores one row's 128 columns
+            const int64_t j = sh.jt * N + lane * 4;
+            for (int64_t row = sh.panel * kPanel + warp * 32, end = row + 32; row < end && row < m; ++row)
+                if (j < n)
+                    *reinterpret_cast<float4 *>(C + row * n + j) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         while (sh.next()) {
             const bool ok = mbar_wait(done, piece & 1);
             if (!__all_sync(0xffffffffu, ok ? 1 : 0) || *abort_flag) {
@@ -1092,23 +1100,37 @@ int64_t split_ctas(int64_t work)
     return by_work < 1 ? 1 : (by_work > most ? most : by_work);
 }
 
+// Shares, or (few tiles per panel) a CTA per (panel, strip): a share of several
+// panels walks them one after the other, some 4 us of drain each, and the
+// fix-up is a launch more. Measured on 960 multiplies (64^2 to 12000^2, blocks
+// and unstructured, n 16 to 2048), whole / shares, us: 5384 x 1267 at 0.2 %,
+// n = 64 14 / 42; 2322 x 386 at 3 %, n = 96 16 / 28; 1024^2 at 15 % in blocks (48
+// tiles a panel), n = 64 32 / 24. At 32 tiles the choice takes 0.6 % longer
+// than the better of the two (16 and 48: 1.8 and 1.2 %; shares alone 32 %).
+constexpr int64_t kSplitWholeTiles = 32;
+bool split_shares(const TcPlan &p) { return p.tiles > kSplitWholeTiles * p.panels; }
+
 cudaError_t launch_split(const TcPlan &p, int64_t m, int64_t n, float *C, uint32_t *status, cudaStream_t st)
 {
-    const int64_t njt = (n + kSplitN - 1) / kSplitN, work = p.tiles * njt, ctas = split_ctas(work);
+    const int64_t njt = (n + kSplitN - 1) / kSplitN, work = p.tiles * njt;
+    const bool shares = split_shares(p);
+    const int64_t ctas = shares ? split_ctas(work) : p.panels * njt;
     const ShareCut cut(work, ctas);
-    if (njt > 65535 || p.panels > 0x7fffffffLL)
+    if (njt > 65535 || p.panels > 0x7fffffffLL || ctas > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (work > 0) {
+    if (work > 0 || !shares) {
         cudaError_t e = cudaFuncSetAttribute(spdm_tc_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem);
         if (e != cudaSuccess)
             return e;
         e = launch_after(
-            spdm_tc_split_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kSplitThreads), kSplitSmem, st, p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n, p.kb, p.tiles,
-            cut, C, p.part.ptr, status);
+            spdm_tc_split_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kSplitThreads), kSplitSmem, st, p.pf.ptr, p.tile_cb.ptr, p.tile_panel.ptr, p.a_hi.ptr, p.a_lo.ptr, p.b_hi.ptr, p.b_lo.ptr, m, n, p.kb, p.panels,
+            p.tiles, cut, shares, C, p.part.ptr, status);
         if (e != cudaSuccess)
             return e;
         count_launches(1);
     }
+    if (!shares)
+        return cudaSuccess;
     const dim3 grid(static_cast<unsigned>(p.panels), static_cast<unsigned>(njt), kSplitN / 32);
     count_launches(1);
     return launch_after(tc_fixup_kernel, grid, dim3(kPanel), 0, st, p.pf.ptr, m, n, p.kb, p.tiles, cut, kSplitN,
@@ -1182,7 +1204,7 @@ gcoo_status tc_prepare_b(gcoo_handle *h, int64_t n, bool fp8)
     // the parts of the shares, whatever the width: two per CTA (split) or pair
     size_t parts = 0;
     if (p.split)
-        parts = 4 * static_cast<size_t>(device_sms()) * kPartFloats;
+        parts = split_shares(p) ? 4 * static_cast<size_t>(device_sms()) * kPartFloats : 0;
     else
         for (int64_t t = 1; t <= std::min<int64_t>(nt, kPairShareCols) && parts == 0; ++t)
             if (pair_cut(p.panels, p.tiles, t).shares)
