@@ -229,7 +229,7 @@ gcoo_status spdm_fp32(gcoo_handle *h, const float *dB, int64_t n, float *dC, cud
                   : launch_spdm_long(h->packed.ptr, h->row_ptr.ptr, h->long_rows.ptr, h->n_long, dB, n, dC, st);
         const cudaError_t es = el == cudaSuccess
                                    ? launch_spdm_short(h->packed.ptr, h->row_ptr.ptr, h->m, h->k, dB, n, dC,
-                                                       long_row_min(), split, h->side)
+                                                       long_row_min(), split ? 0 : h->max_row_nnz, h->side)
                                    : cudaSuccess;
         // joined whatever happened: nothing of this call runs past it on the side stream
         GCOO_CUDA(cudaEventRecord(h->ev_join, h->side));

@@ -213,10 +213,10 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
                              cudaStream_t st);
 // The rows shorter than long_min, one warp per (row, column tile), nothing
 // staged (skewed matrices, whose long rows go to launch_spdm_long); k is
-// B's row count, which sets the walk order; split: the long rows are summed in
-// pieces beside it, not as chains.
+// B's row count, which sets the walk order; chain: entries of the longest row
+// that is summed in one chain beside it.
 cudaError_t launch_spdm_short(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k, const float *B,
-                              int64_t n, float *C, int32_t long_min, bool split, cudaStream_t st);
+                              int64_t n, float *C, int32_t long_min, int64_t chain, cudaStream_t st);
 // ---- FP8-B scales (spdm_lowp.cu) -----------------------------------------------------------
 // scale[j] = the smallest power of two with absmax(B[:, j]) / scale[j] <= 448;
 // n % 4 == 0, B 16-byte aligned; amax: n words of scratch.

@@ -417,12 +417,16 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
 // (forty-eight with four: 137, sixty-four 147, forty with eight 145).
 // With the long rows in their copy-and-chain kernel: 118, forty-eight warps 118,
 // thirty-two with batches of eight 127, of six 130.
-// Thirty-two with batches of eight where the long rows are summed in pieces, so
-// that the short ones take longer, and all warps fit four waves: a row of some
-// hundred entries is then the time, and twice the loads in flight shorten it
-// (us, split sums, batches of four / eight: 8192 warps 23.3 / 20.3, 16384 26.6 /
-// 25.0, 24000 32.1 / 31.1, 30000 37.9 / 40.1, 65536 52 / 58; chains, 16346
-// warps 33.8 / 35.2, 24000 34.6 / 36.7).
+// Thirty-two with batches of eight where all warps fit four waves and the long
+// rows beside them take less time than the short ones (chains of up to 2500
+// entries, or sums in pieces): a row of some hundred entries is then the time,
+// and twice the loads in flight shorten it. Time with eight over time with four,
+// 1379 multiplies, by waves and longest row: up to one wave, up to 600 entries
+// .83, 1200 .86, 2500 .93, longer .99; two to four waves .89, .93, .96, .99;
+// eight to sixteen .97, .98, 1.01, 1.0; more 1.02. Zipf rows of up to 4096: 16346
+// warps 33.8 us with four, 35.2 with eight, 24000 34.6 / 36.7; the same with
+// sums in pieces 29.8 / 28.1, 32.1 / 31.1, and 65536 52 / 58.
+constexpr int64_t kShortDeepChain = 2500;
 constexpr int64_t kShortDeepWaves = 4;
 constexpr int short_ctas(int batch) { return batch == 4 ? 20 : 16; } // per SM
 
@@ -838,7 +842,7 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
 }
 
 cudaError_t launch_spdm_short(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k, const float *B,
-                              int64_t n, float *C, int32_t long_min, bool split, cudaStream_t st)
+                              int64_t n, float *C, int32_t long_min, int64_t chain, cudaStream_t st)
 {
     if (m <= 0 || n <= 0)
         return cudaSuccess;
@@ -858,7 +862,7 @@ cudaError_t launch_spdm_short(const Entry *packed, const int32_t *row_ptr, int64
     const unsigned grid = static_cast<unsigned>(blocks);
     const int32_t nt = static_cast<int32_t>(tiles);
     const int32_t tm = tiles > 1 && k * n * 4 > kShortTileMajorBytes ? 1 : 0;
-    const bool deep = split && warps <= kShortDeepWaves * device_sms() * 2 * short_ctas(4);
+    const bool deep = chain <= kShortDeepChain && warps <= kShortDeepWaves * device_sms() * 2 * short_ctas(4);
 #define GCOO_SHORT(V)                                                                                               \
     (deep ? spdm_short_kernel<V, 8> : spdm_short_kernel<V, 4>)<<<grid, 64, 0, st>>>(packed, row_ptr, m, B, n, C, nt, \
                                                                                     long_min, tm)
