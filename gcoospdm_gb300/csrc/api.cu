@@ -166,6 +166,25 @@ static SharedWalk fp32_walk(const gcoo_handle *h, int64_t n, const float *dB, co
                : kWalkRows;
 }
 
+// Whether a skewed matrix's long and short rows get kernels of their own. B
+// and C aligned for 16-byte accesses: yes. Else a lane of those kernels has
+// one column (two for even widths) where the row walk has four: only while the
+// longest row's chain is the time of the row walk and not the work. Measured on
+// 869 multiplies of such widths, own kernels / row walk, us: 40000 Zipf rows of
+// up to 4096 entries, n = 201 155 / 218; 65536, n = 255 340 / 376; 8609 x 2229
+// with 1.7 M entries, n = 1767 1764 / 760; 6135 x 6475, 3.7 M, n = 1207 4426 /
+// 1381. The lines below take 3 % longer than the better one (always own kernels
+// 7 %, up to 3.8 times; always the row walk 2 times on average).
+static bool long_rows_pay(const gcoo_handle *h, int64_t n, const float *dB, const float *dC)
+{
+    const uintptr_t at = reinterpret_cast<uintptr_t>(dB) | reinterpret_cast<uintptr_t>(dC);
+    if (n % 4 == 0 && !(at & 15))
+        return true;
+    const bool pairs = n % 2 == 0 && !(at & 7);
+    return static_cast<double>(h->nnz) * static_cast<double>(n) <=
+           (pairs ? 1.5e5 : 8e4) * static_cast<double>(h->max_row_nnz);
+}
+
 gcoo_status spdm_fp32(gcoo_handle *h, const float *dB, int64_t n, float *dC, cudaStream_t st,
                       const gcoo_params *override_params)
 {
@@ -206,7 +225,8 @@ gcoo_status spdm_fp32(gcoo_handle *h, const float *dB, int64_t n, float *dC, cud
     }
     // a skewed matrix (explicit launch-shape overrides aside): its long rows go
     // to their own kernel, the short rest to a kernel without staging
-    if (!override_params && h->n_long > 0 && h->side && h->ev_fork && h->ev_join && long_rows_ok(h->m, n)) {
+    if (!override_params && h->n_long > 0 && h->side && h->ev_fork && h->ev_join && long_rows_ok(h->m, n) &&
+        long_rows_pay(h, n, dB, dC)) {
         // the pieces' kernel copies 16 bytes at a time; other widths keep the chain
         const bool split = h->p.fp32_sum == GCOO_SUM_SPLIT && h->pieces_bound > 0 && n % 4 == 0 &&
                            (reinterpret_cast<uintptr_t>(dB) & 15) == 0;
