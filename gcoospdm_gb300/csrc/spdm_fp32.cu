@@ -772,11 +772,15 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
         // CTA's staging is the larger share, so one wave under 8 entries
         // (2048^2 at 0.1 % 8.1 us, 9.2 with two, 11.2 with four; 2880 x 1527
         // at 0.28 %, n = 1568 11.3, 11.4 and 14.0) and two under 16 (2048^2 at
-        // 0.5 % 16.0, 15.1 and 16.5)
+        // 0.5 % 16.0, 15.1 and 16.5), as long as no row is much longer: its CTA
+        // is then the time (6951 x 4723, 3 entries a row and up to 237, n = 728
+        // 80 us with one wave, 45 with two, 26 with four; lines at 1/2 to 1/5 of
+        // the longest row differ by less than 0.3 % over 2079 multiplies)
         int64_t ci = 768 / tile;
         const int64_t groups = (m + s.rows - 1) / s.rows;
         const int64_t resident = static_cast<int64_t>(device_sms()) * (s.warps <= 4 ? kRowCtas : 6);
-        const int64_t waves = nnz < 8 * m ? 1 : (nnz < 16 * m ? 2 : 4);
+        const double len = mean > max_row / 3.0 ? mean : max_row / 3.0;
+        const int64_t waves = len < 8.0 ? 1 : (len < 16.0 ? 2 : 4);
         const int64_t by_grid = groups * ny / (waves * resident);
         ci = ci > by_grid ? by_grid : ci;
         ci = ci < 1 ? 1 : (ci > ny ? ny : ci);

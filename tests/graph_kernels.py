@@ -1,5 +1,5 @@
 """The kernels that a call puts into a stream, from a capture of the call:
-names and priorities, through the CUDA driver API (nothing runs)."""
+names and grids, through the CUDA driver API (nothing runs)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -10,15 +10,13 @@ class KernelParams(C.Structure):  # CUDA_KERNEL_NODE_PARAMS_v2
                 ("params", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
 
 
-KERNEL_NODE = 0   # CU_GRAPH_NODE_TYPE_KERNEL
-PRIORITY = 8      # CU_LAUNCH_ATTRIBUTE_PRIORITY
-RELAXED = 2       # CU_STREAM_CAPTURE_MODE_RELAXED
+KERNEL_NODE = 0  # CU_GRAPH_NODE_TYPE_KERNEL
+RELAXED = 2      # CU_STREAM_CAPTURE_MODE_RELAXED
 
 
 def captured_kernels(stream, call):
-    """[(mangled name, priority)] of the kernels that call() launches on
-    `stream` (a torch stream, not the default one), in no particular order.
-    Lower numbers are higher priorities."""
+    """[(mangled name, (grid x, y, z))] of the kernels that call() launches on
+    `stream` (a torch stream, not the default one), in no particular order."""
     d = C.CDLL("libcuda.so.1")
 
     def ok(rc):
@@ -42,14 +40,13 @@ def captured_kernels(stream, call):
             ok(d.cuGraphNodeGetType(node, C.byref(kind)))
             if kind.value != KERNEL_NODE:
                 continue
-            p, name, value = KernelParams(), C.c_char_p(), (C.c_int * 16)()
+            p, name = KernelParams(), C.c_char_p()
             ok(d.cuGraphKernelNodeGetParams_v2(node, C.byref(p)))
             if p.func:
                 ok(d.cuFuncGetName(C.byref(name), C.c_void_p(p.func)))
             else:
                 ok(d.cuKernelGetName(C.byref(name), C.c_void_p(p.kern)))
-            ok(d.cuGraphKernelNodeGetAttribute(node, C.c_int(PRIORITY), value))
-            found.append((name.value.decode(), value[0]))
+            found.append((name.value.decode(), tuple(p.grid)))
         return found
     finally:
         d.cuGraphDestroy(graph)
