@@ -153,10 +153,16 @@ static SharedWalk shared_walk(const gcoo_handle *h, int64_t n, uintptr_t b, uint
         return panel_ok(n) && share >= 1.75 * sharing4 ? kWalkPanels : kWalkGroups;
     const double work = static_cast<double>(h->nnz) * static_cast<double>(n);
     const bool long_rows = h->nnz >= 1600 * h->m;
+    // a skewed matrix (its long rows have kernels of their own in the row walk):
+    // panels once the work outweighs the one panel that walks the longest row's
+    // columns (4308 x 667 in 16 x 16 blocks at 2 %, one full row, n = 1700: rows 36,
+    // groups 111, panels 66 us)
+    if (h->n_long > 0 && work < 5e5 * static_cast<double>(h->max_row_nnz))
+        return kWalkRows;
     if (panel_ok(n) && n >= 96 && share >= 4.0 && share * share * share * work * (long_rows ? 2 : 1) >= 2.9e11)
         return kWalkPanels;
     const bool vec4 = n % 4 == 0 && !((b | c) & 15);
-    return vec4 && n >= 640 && sharing4 >= 3.3 && work >= 3e8 ? kWalkGroups : kWalkRows;
+    return vec4 && n >= 640 && sharing4 >= 3.3 && work >= 3e8 && h->n_long == 0 ? kWalkGroups : kWalkRows;
 }
 
 static SharedWalk fp32_walk(const gcoo_handle *h, int64_t n, const float *dB, const float *dC)
@@ -167,22 +173,31 @@ static SharedWalk fp32_walk(const gcoo_handle *h, int64_t n, const float *dB, co
 }
 
 // Whether a skewed matrix's long and short rows get kernels of their own. B
-// and C aligned for 16-byte accesses: yes. Else a lane of those kernels has
-// one column (two for even widths) where the row walk has four: only while the
-// longest row's chain is the time of the row walk and not the work. Measured on
-// 869 multiplies of such widths, own kernels / row walk, us: 40000 Zipf rows of
-// up to 4096 entries, n = 201 155 / 218; 65536, n = 255 340 / 376; 8609 x 2229
+// and C aligned for 16-byte accesses: yes, but where nearly all entries are in
+// long rows and the work outweighs the longest one (8192^2, 410 entries a row
+// and one full row, n = 1024: 1275 us, the row walk 716; 13622 x 5573, 286 a row,
+// n = 976 1554 / 872). At other alignments a lane of those kernels has one column
+// (two for even widths) where the row walk has four: only while the longest
+// row's chain is the time of the row walk and not the work, sooner if more than
+// half of the entries are in long rows. Measured on 869 multiplies of such
+// widths, own kernels / row walk, us: 40000 Zipf rows of up to 4096 entries (38 %
+// of all in long rows), n = 201 155 / 218; 65536, n = 255 340 / 376; 8609 x 2229
 // with 1.7 M entries, n = 1767 1764 / 760; 6135 x 6475, 3.7 M, n = 1207 4426 /
-// 1381. The lines below take 3 % longer than the better one (always own kernels
-// 7 %, up to 3.8 times; always the row walk 2 times on average).
+// 1381; 6850^2, 504 a row, n = 33 411 / 232. The lines below take 3 % longer than
+// the better one (always own kernels 7 %, up to 3.8 times; always the row walk
+// 2 times on average).
 static bool long_rows_pay(const gcoo_handle *h, int64_t n, const float *dB, const float *dC)
 {
     const uintptr_t at = reinterpret_cast<uintptr_t>(dB) | reinterpret_cast<uintptr_t>(dC);
-    if (n % 4 == 0 && !(at & 15))
-        return true;
-    const bool pairs = n % 2 == 0 && !(at & 7);
-    return static_cast<double>(h->nnz) * static_cast<double>(n) <=
-           (pairs ? 1.5e5 : 8e4) * static_cast<double>(h->max_row_nnz);
+    const bool quads = n % 4 == 0 && !(at & 15), pairs = n % 2 == 0 && !(at & 7);
+    if (quads && h->p.fp32_sum == GCOO_SUM_SPLIT)
+        return true; // sums in pieces stay where they are asked for
+    const int64_t tile = quads ? 128 : (pairs ? 64 : 32);
+    const double cols = static_cast<double>(quads ? n : (n + tile - 1) / tile * tile); // walked
+    const double work = static_cast<double>(h->nnz) * cols / static_cast<double>(h->max_row_nnz);
+    if (quads)
+        return work <= 2e5 || 20 * h->long_entries <= 17 * h->nnz;
+    return work <= (pairs ? 1.5e5 : (2 * h->long_entries <= h->nnz ? 8e4 : 3e4));
 }
 
 gcoo_status spdm_fp32(gcoo_handle *h, const float *dB, int64_t n, float *dC, cudaStream_t st,
