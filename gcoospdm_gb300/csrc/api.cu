@@ -376,6 +376,7 @@ gcoo_status gcoo_create(gcoo_handle **out, const float *dA, int64_t m, int64_t k
 namespace {
 
 constexpr size_t kReadbackWords = 8; // of a handle's page-locked readback
+constexpr int64_t kSampleEntries = 34500; // 16^3 * entries * 2048 columns < 2.9e11 below (shared_walk)
 
 // How many rows of a panel (16 rows) share a column, for shared_walk; 0 where
 // the panels cannot run or never pay. A sample of panels tells: share, when
@@ -383,21 +384,23 @@ constexpr size_t kReadbackWords = 8; // of a handle's page-locked readback
 // matrix), else one more readback. A panel's staging costs about the same
 // whatever its window holds: at 2 % density (16 x 16 blocks, 4096^2) panels
 // take 36 against the group walk's 53 us at n = 256 and 54 against 60 at n =
-// 1024, so below 1/64 they are left out.
+// 1024, so below 1/64 they are left out; and matrices so small that only B
+// wider than 2048 columns would take them are not sampled, which is a tenth of
+// a small matrix's rebuild (255 x 794 at 36 % 37 us with it, 32 without).
 gcoo_status choose_panels(gcoo_handle *h, cudaStream_t st, const int64_t *share)
 {
     h->panel_share = 0.0;
     h->sampled = false;
-    if (!h->seg_prefix || !group_order_chosen(h) || 64.0 * static_cast<double>(h->nnz) < static_cast<double>(h->m) * h->k)
+    if (!h->seg_prefix || !group_order_chosen(h) || h->nnz < kSampleEntries ||
+        64.0 * static_cast<double>(h->nnz) < static_cast<double>(h->m) * h->k)
         return GCOO_SUCCESS;
     h->sampled = true;
     int64_t own[2] = {0, 0};
     if (!share) {
-        if (!h->long_count.ensure(2))
-            return fail(GCOO_ERROR_ALLOC, "device allocation of the sharing counts failed");
-        GCOO_CUDA(cudaMemsetAsync(h->long_count.ptr, 0, sizeof(own), st));
-        GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m, h->long_count.ptr, st));
-        GCOO_CUDA(cudaMemcpyAsync(own, h->long_count.ptr, sizeof(own), cudaMemcpyDeviceToHost, st));
+        // the build's words [6] and [7], zero as it left them
+        unsigned long long *words = reinterpret_cast<unsigned long long *>(h->status.ptr + 2) + 6;
+        GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m, h->k, words, nullptr, nullptr, st));
+        GCOO_CUDA(cudaMemcpyAsync(own, words, sizeof(own), cudaMemcpyDeviceToHost, st));
         GCOO_CUDA(cudaStreamSynchronize(st));
         share = own;
     }
@@ -514,7 +517,7 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
         (!one_scan && !h->scratch.ensure(scan_scratch_elems(h->m))) || !h->status.ensure(2 + 8 * 2))
         return fail(GCOO_ERROR_ALLOC, "device allocation of the GCOO index arrays failed");
     // [0] total nnz, [1] longest row, [2] distinct group columns, [3] staging status, [4] overflowed tiles,
-    // [5] ticket of the prefix-and-scan kernel, [6] entries and [7] distinct columns of the sampled panels;
+    // [5] tickets of the prefix-and-scan and the sampling kernel, [6] entries and [7] distinct columns of the sample;
     // behind the status word: one memset clears all
     int64_t *d_total = reinterpret_cast<int64_t *>(h->status.ptr + 2);
     GCOO_CUDA(cudaMemsetAsync(h->status.ptr, 0, 8 + 8 * sizeof(int64_t), st));
@@ -559,11 +562,12 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
         GCOO_CUDA(launch_place(h->dA, h->m, h->k, cpg, slot, h->stage.ptr, h->tile_tot.ptr, h->over_list.ptr,
                                over_count, h->tile_cnt.ptr, h->group_index(), h->row_ptr.ptr, h->vals.ptr, h->rc.ptr,
                                h->packed.ptr, d_total, cap, packed_cap, ahead || sample ? h->row_ptr.ptr : nullptr, st));
-        if (sample)
-            GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m,
-                                         reinterpret_cast<unsigned long long *>(d_total + 6), st));
+        if (sample) // its totals with the others'
+            GCOO_CUDA(launch_panel_share(h->packed.ptr, h->row_ptr.ptr, h->m, h->k,
+                                         reinterpret_cast<unsigned long long *>(d_total + 6), ticket + 1,
+                                         one_scan ? h->readback + 6 : nullptr, st));
         const int64_t *t3 = h->readback;
-        if (!one_scan || sample)
+        if (!one_scan)
             GCOO_CUDA(cudaMemcpyAsync(h->readback, d_total, kReadbackWords * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         GCOO_CUDA(cudaEventRecord(h->ev_totals, st));
         if (ahead) {

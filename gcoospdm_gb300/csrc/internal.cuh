@@ -259,9 +259,10 @@ cudaError_t launch_spdm_fp32_group(const float *vals, const int32_t *rows, const
 // (pref[r * conv_segments(k) + s]).
 bool panel_ok(int64_t n);
 // Sampled sharing inside 16-row panels: out[0] += entries, out[1] += distinct
-// (panel, column) pairs (zeroed by the caller).
-cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, unsigned long long *out,
-                               cudaStream_t st);
+// (panel, column) pairs (zeroed by the caller). host (may be null): page-locked
+// memory that receives both; *ticket, then, is zeroed by the caller.
+cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k,
+                               unsigned long long *out, unsigned int *ticket, int64_t *host, cudaStream_t st);
 cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, const int32_t *pref, int64_t m,
                                    int64_t k, const float *B, int64_t n, float *C, cudaStream_t st);
 // The same walk for the BF16 / FP8-B forms on the FMA engine, from B already

@@ -388,34 +388,42 @@ spdm_panel_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
 
 // How many rows of a panel share a column, on up to gridDim.x panels spread
 // over the matrix: out[0] += entries, out[1] += distinct columns, both of
-// kShareCols columns from each panel's first one with an entry on. A CTA has
-// one panel, and the build waits for it: many threads, eight entries' loads of
-// each in flight, a byte per column (8192^2 at 25 % in 16 x 16 blocks, 32768
-// entries a panel: 9.5 us; with 256 threads 42, 1024 threads that set bits
-// with atomics 17).
+// kShareCols columns from each panel's first one with an entry on. host (may be
+// null; page-locked): out as the CTA that finishes last (*ticket, zeroed
+// before) finds it. A CTA has one panel, and the build waits for it: many
+// threads, eight entries' loads of each in flight, a byte per column (8192^2
+// at 25 % in 16 x 16 blocks, 32768 entries a panel: 9.5 us; with 256 threads
+// 42, 1024 threads that set bits with atomics 17).
 constexpr int kShareCols = 1 << 15;
 constexpr int kSharePanels = 64, kShareThreads = 1024, kShareBatch = 8;
 
 __global__ void __launch_bounds__(kShareThreads)
-panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m, int64_t panels,
-                   unsigned long long *__restrict__ out)
+panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m, int64_t k,
+                   int64_t panels, unsigned long long *__restrict__ out, unsigned int *__restrict__ ticket,
+                   int64_t *__restrict__ host)
 {
     __shared__ __align__(16) uint8_t s_seen[kShareCols]; // 0 or 1: stores of 1 need no atomics
-    __shared__ int s_first;
+    __shared__ int s_first, s_sum[2];
     const int64_t r0 = (blockIdx.x * panels / gridDim.x) * kPanelRows;
     const int64_t r1 = r0 + kPanelRows < m ? r0 + kPanelRows : m;
-    for (int i = threadIdx.x; i < kShareCols / 16; i += kShareThreads)
+    const int used = static_cast<int>(k < kShareCols ? (k + 15) / 16 : kShareCols / 16);
+    for (int i = threadIdx.x; i < used; i += kShareThreads)
         reinterpret_cast<uint4 *>(s_seen)[i] = make_uint4(0, 0, 0, 0);
-    if (threadIdx.x == 0)
-        s_first = 0x7fffffff;
+    if (threadIdx.x == 0) {
+        s_first = k > kShareCols ? 0x7fffffff : 0;
+        s_sum[0] = s_sum[1] = 0;
+    }
+    grid_wait_previous();
     __syncthreads();
-    const int64_t r = r0 + threadIdx.x;
-    if (r < r1 && row_ptr[r] < row_ptr[r + 1])
-        atomicMin(&s_first, packed[row_ptr[r]].col);
-    __syncthreads();
+    const int64_t begin = row_ptr[r0], end = row_ptr[r1];
+    if (k > kShareCols) {
+        const int64_t r = r0 + threadIdx.x;
+        if (r < r1 && row_ptr[r] < row_ptr[r + 1])
+            atomicMin(&s_first, packed[row_ptr[r]].col);
+        __syncthreads();
+    }
     int entries = 0, distinct = 0;
-    const int64_t end = row_ptr[r1];
-    for (int64_t e0 = row_ptr[r0] + threadIdx.x; e0 < end; e0 += kShareThreads * kShareBatch) {
+    for (int64_t e0 = begin + threadIdx.x; e0 < end; e0 += kShareThreads * kShareBatch) {
         int c[kShareBatch];
 #pragma unroll
         for (int u = 0; u < kShareBatch; ++u) {
@@ -430,26 +438,39 @@ panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__
             }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kShareCols / 4; i += kShareThreads)
+    for (int i = threadIdx.x; i < 4 * used; i += kShareThreads)
         distinct += __popc(reinterpret_cast<const uint32_t *>(s_seen)[i]);
     entries = __reduce_add_sync(0xffffffffu, entries);
     distinct = __reduce_add_sync(0xffffffffu, distinct);
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(out, static_cast<unsigned long long>(entries));
-        atomicAdd(out + 1, static_cast<unsigned long long>(distinct));
+        atomicAdd(&s_sum[0], entries);
+        atomicAdd(&s_sum[1], distinct);
+    }
+    __syncthreads();
+    if (threadIdx.x != 0)
+        return;
+    atomicAdd(out, static_cast<unsigned long long>(s_sum[0]));
+    atomicAdd(out + 1, static_cast<unsigned long long>(s_sum[1]));
+    if (!host)
+        return;
+    __threadfence(); // the sums before the ticket
+    if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+        __threadfence();
+        host[0] = static_cast<int64_t>(__ldcg(out));
+        host[1] = static_cast<int64_t>(__ldcg(out + 1));
     }
 }
 
 } // namespace
 
-cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, unsigned long long *out,
-                               cudaStream_t st)
+cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k,
+                               unsigned long long *out, unsigned int *ticket, int64_t *host, cudaStream_t st)
 {
     const int64_t panels = (m + kPanelRows - 1) / kPanelRows;
     const unsigned grid = static_cast<unsigned>(panels < kSharePanels ? panels : kSharePanels);
-    panel_share_kernel<<<grid, kShareThreads, 0, st>>>(packed, row_ptr, m, panels, out);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_after(panel_share_kernel, dim3(grid), dim3(kShareThreads), 0, st, packed, row_ptr, m, k, panels, out,
+                        ticket, host);
 }
 
 // Wider B stays with the group walk, whose tile count decides what is possible
