@@ -1,0 +1,35 @@
+"""GPU: the row walk's launch shapes by rows per group and by how many CTAs
+there are for the GPU's SMs, bit for bit against the oracle on some rows."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from graph_kernels import captured_kernels
+
+pytestmark = pytest.mark.gpu
+
+
+def check(native, oracle_mod, m, k, n, per_row, rows_per_group=4):
+    import torch
+    rng = np.random.default_rng(m + n)
+    A = np.where(rng.random((m, k)) < per_row / k, rng.standard_normal((m, k)), 0.0).astype(np.float32)
+    B = rng.standard_normal((k, n)).astype(np.float32)
+    h = native.GcooHandle(torch.from_numpy(A).cuda(), rows_per_group=rows_per_group, fp32_order="rows").build()
+    C = torch.full((m + 1, n), 7.0, device="cuda")
+    dB, s = torch.from_numpy(B).cuda(), torch.cuda.Stream()
+    for _ in range(3):  # one behind another
+        h.spdm(dB, C[:m])
+    some = np.r_[0:9, m // 2, m - 5:m]
+    want = oracle_mod.spdm(oracle_mod.convert(A[some]), B)
+    assert np.array_equal(C.cpu().numpy()[some].view(np.uint32), want.view(np.uint32))
+    assert bool((C[m] == 7.0).all()) and bool((C[:m] != 7.0).any(1).all())
+    (name, grid), = captured_kernels(s, lambda: h.spdm(dB, C[:m], stream=s))
+    return name, grid[0] * grid[1]
+
+
+@pytest.mark.parametrize("rows_per_group", [8, 16, 32])
+@pytest.mark.parametrize("per_row", [7, 130])
+@pytest.mark.parametrize("n", [100, 133, 518])
+def test_many_rows_per_group(native, oracle_mod, rows_per_group, per_row, n):
+    check(native, oracle_mod, 1003, 400, n, per_row, rows_per_group)
