@@ -792,6 +792,17 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
         // (measured 2-6 % faster at 0.1-1 % density)
         s.chunk = static_cast<int>(max_row * s.rows);
     }
+    // Rows of some hundred entries and little more than one wave of CTAs: their
+    // spread over the SMs is the time. Not started while the predecessor drains,
+    // where they would take whichever slots come free first (1924 x 249, 154
+    // entries a row, n = 236: 22.3 us behind another multiply, 18.9 so; shorter
+    // rows gain by it, 6 % on average over 1504 multiplies).
+    if (mean >= 100.0) {
+        const int64_t tile = static_cast<int64_t>(s.col_warps) * 32 * s.vec * s.col_iters;
+        const int64_t ctas = (m + s.rows - 1) / s.rows * ((n + tile - 1) / tile), sms = device_sms();
+        const int64_t per_sm = s.warps <= 4 ? kRowCtas : 48 / s.warps;
+        s.after = 10 * ctas > 13 * per_sm * sms;
+    }
     return s;
 }
 
@@ -812,14 +823,19 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
     // kernel stages any larger group in several passes)
     const int chunk = s.chunk > 0 && s.chunk < kChunk ? s.chunk : kChunk;
     const int smem = 128 + (chunk + 2) * static_cast<int>(sizeof(Entry));
+    const auto go = [&](auto kernel, int32_t col_iters) {
+        if (s.after)
+            return launch_after(kernel, grid, dim3(threads), smem, st, packed, row_ptr, m, cpg, B, n, C, s.col_warps,
+                                col_iters, chunk, status);
+        kernel<<<grid, threads, smem, st>>>(packed, row_ptr, m, cpg, B, n, C, s.col_warps, col_iters, chunk, status);
+        return cudaGetLastError();
+    };
 #define GCOO_FP32_LAUNCH(V, W, T, P)                                                                       \
     do {                                                                                                \
         if (s.col_iters > 1)                                                                            \
-            le = launch_after(spdm_fp32_kernel<V, W, T, P, true>, grid, dim3(threads), smem, st,          \
-                packed, row_ptr, m, cpg, B, n, C, s.col_warps, s.col_iters, chunk, status);             \
+            le = go(spdm_fp32_kernel<V, W, T, P, true>, s.col_iters);                                    \
         else                                                                                            \
-            le = launch_after(spdm_fp32_kernel<V, W, T, P, false>, grid, dim3(threads), smem, st,         \
-                packed, row_ptr, m, cpg, B, n, C, s.col_warps, 1, chunk, status);                       \
+            le = go(spdm_fp32_kernel<V, W, T, P, false>, 1);                                             \
     } while (0)
 #define GCOO_FP32_VEC(T, P)                                                                             \
     do {                                                                                                \
