@@ -204,6 +204,7 @@ struct LaunchShape {
     int width = 1;     // columns per load (1, 2, 4; at most vec)
     int chunk = 0;     // entries staged per pass (shared memory), 0: the full 2048
     bool after = true;  // started while its predecessor in the stream drains (launch_after)
+    bool tight = false; // registers for twelve 4-warp CTAs per SM
 };
 // Heavy-tailed row lengths: the longest row at least 256 entries and above 8x the mean.
 bool row_lengths_skewed(int64_t m, int64_t nnz, int64_t max_row);

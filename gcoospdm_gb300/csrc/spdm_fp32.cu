@@ -796,12 +796,15 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
     // spread over the SMs is the time. Not started while the predecessor drains,
     // where they would take whichever slots come free first (1924 x 249, 154
     // entries a row, n = 236: 22.3 us behind another multiply, 18.9 so; shorter
-    // rows gain by it, 6 % on average over 1504 multiplies).
+    // rows gain by it, 6 % on average over 1504 multiplies); and with twelve
+    // 4-warp CTAs per SM where that is one wave and kRowCtas are not (1199 x
+    // 4114, 170 a row, n = 728: 42.5 us with ten, 34.3 with twelve).
     if (mean >= 100.0) {
         const int64_t tile = static_cast<int64_t>(s.col_warps) * 32 * s.vec * s.col_iters;
         const int64_t ctas = (m + s.rows - 1) / s.rows * ((n + tile - 1) / tile), sms = device_sms();
         const int64_t per_sm = s.warps <= 4 ? kRowCtas : 48 / s.warps;
         s.after = 10 * ctas > 13 * per_sm * sms;
+        s.tight = s.warps <= 4 && ctas > per_sm * sms && ctas <= 12 * sms;
     }
     return s;
 }
@@ -848,7 +851,7 @@ cudaError_t launch_spdm_fp32(const Entry *packed, const int32_t *row_ptr, int64_
     } while (0)
     const bool pipe = s.depth >= 2;
     cudaError_t le = cudaSuccess;
-    if (threads <= 128 && !pipe) {
+    if (threads <= 128 && !pipe && !s.tight) {
         GCOO_FP32_VEC(128, false);
     } else if (threads <= 512) {
         if (pipe) GCOO_FP32_VEC(512, true);

@@ -33,3 +33,16 @@ def check(native, oracle_mod, m, k, n, per_row, rows_per_group=4):
 @pytest.mark.parametrize("n", [100, 133, 518])
 def test_many_rows_per_group(native, oracle_mod, rows_per_group, per_row, n):
     check(native, oracle_mod, 1003, 400, n, per_row, rows_per_group)
+
+
+@pytest.mark.parametrize("n", [128, 131, 258, 512])
+def test_one_wave_of_ten_and_of_twelve_ctas(native, oracle_mod, n):
+    """Around 10 and 12 CTAs per SM: twelve are resident only in the kernel of fewer registers."""
+    import torch
+    sms, names = torch.cuda.get_device_properties(0).multi_processor_count, []
+    tiles = -(-n // 128)
+    for per_sm in (9.9, 10.1, 11.9, 12.1):
+        name, ctas = check(native, oracle_mod, 4 * int(per_sm * sms / tiles), 300, n, 140)
+        assert abs(ctas - per_sm * sms) <= tiles
+        names.append(name)
+    assert names[0] == names[3] != names[1] == names[2], names
