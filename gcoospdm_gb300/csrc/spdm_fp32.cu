@@ -802,9 +802,10 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
     if (mean >= 100.0) {
         const int64_t tile = static_cast<int64_t>(s.col_warps) * 32 * s.vec * s.col_iters;
         const int64_t ctas = (m + s.rows - 1) / s.rows * ((n + tile - 1) / tile), sms = device_sms();
-        const int64_t per_sm = s.warps <= 4 ? kRowCtas : 48 / s.warps;
+        const int64_t twelve = 48 / s.warps < 32 ? 48 / s.warps : 32; // of CTAs that wide as many as 48 warps
+        const int64_t per_sm = s.warps <= 4 && 4 * kRowCtas / s.warps < twelve ? 4 * kRowCtas / s.warps : twelve;
         s.after = 10 * ctas > 13 * per_sm * sms;
-        s.tight = s.warps <= 4 && ctas > per_sm * sms && ctas <= 12 * sms;
+        s.tight = s.warps <= 4 && ctas > per_sm * sms && ctas <= twelve * sms;
     }
     return s;
 }
