@@ -28,7 +28,9 @@ constexpr int kChunk = 2048; // most entries staged per pass (16 KB)
 // 12 1024 / 1092 / 194, against 1085 / 1104 / 183 with neither this bound nor
 // batched row tails (44 registers). CTAs of 5 to 16 warps: 40 registers, as
 // many as hold 48 warps on an SM (16 rows per group, 5396 x 1859, 18 entries a
-// row, n = 1148 42 us; 80 registers, what they take without a bound, 62).
+// row, n = 1148 42 us; 80 registers, what they take without a bound, 62), but 64
+// where a lane's columns come by narrow loads, which spill with 40 (8671 x 10332,
+// 6 a row, n = 981 59.7 us with 40, 49 with 64).
 constexpr int kRowCtas = 10;
 // rows shorter than this walk two column tiles at once: twice the loads in
 // flight (16384^2 at 0.1 %, rows of ~16: 1011 us below 16 entries, 959 below
@@ -272,7 +274,7 @@ __device__ __forceinline__ void row_chain_pair(const Entry *__restrict__ s, int 
 // warp walks col_iters column tiles, col_warps tiles apart, reusing the
 // staged entries, so short rows do not pay one staging per tile.
 template <int V, int W, int MAXT, bool PIPE, bool MULTI>
-__global__ void __launch_bounds__(MAXT, MAXT == 128 ? kRowCtas : (MAXT == 512 && !PIPE ? 3 : 1))
+__global__ void __launch_bounds__(MAXT, MAXT == 128 ? kRowCtas : (MAXT == 512 && !PIPE ? (W == V ? 3 : 2) : 1))
 spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr, int64_t m,
                  int32_t cpg, const float *__restrict__ B, int64_t n, float *__restrict__ C,
                  int32_t col_warps, int32_t col_iters, int32_t chunk_cap, uint32_t *__restrict__ status)
