@@ -30,7 +30,7 @@ constexpr int kChunk = 2048; // most entries staged per pass (16 KB)
 // many as hold 48 warps on an SM (16 rows per group, 5396 x 1859, 18 entries a
 // row, n = 1148 42 us; 80 registers, what they take without a bound, 62), but 64
 // where a lane's columns come by narrow loads, which spill with 40 (8671 x 10332,
-// 6 a row, n = 981 59.7 us with 40, 49 with 64).
+// 6 a row, n = 981 60 us with 40, 30 with 64).
 constexpr int kRowCtas = 10;
 // rows shorter than this walk two column tiles at once: twice the loads in
 // flight (16384^2 at 0.1 %, rows of ~16: 1011 us below 16 entries, 959 below
