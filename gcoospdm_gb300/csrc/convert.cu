@@ -793,8 +793,13 @@ cudaError_t launch_scatter(const float *A, int64_t m, int64_t k, int32_t cpg, co
     if (ng <= 0)
         return cudaSuccess;
     const unsigned grid = static_cast<unsigned>(ng);
-    if ((reinterpret_cast<uintptr_t>(A) & 3) == 0 && cpg <= 8) {
-        const bool al = k % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    // Rows that do not start on 16 bytes: the vector kernel up to 4 rows per group
+    // (4000 x 4001 at 2 %: 1 row 43 us against 79 of 4-byte loads, 2 42 / 57, 4 44 /
+    // 58); with 8 its shifted rows take too many registers (84 / 61; 5653 x 5910 at
+    // 16 % 235 / 108).
+    const bool al = k % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    // 16 % 235 / 108).
+    if (al ? cpg <= 8 : (reinterpret_cast<uintptr_t>(A) & 3) == 0 && cpg <= 4) {
 #define GCOO_SCATTER_VEC(C)                                                                                         \
     (al ? scatter_vec_kernel<C, true> : scatter_vec_kernel<C, false>)<<<grid, kScatterThreads, 0, st>>>(            \
         A, m, k, group_index, row_ptr, vals, rows, cols, packed)
@@ -802,7 +807,10 @@ cudaError_t launch_scatter(const float *A, int64_t m, int64_t k, int32_t cpg, co
         case 1: GCOO_SCATTER_VEC(1); break;
         case 2: GCOO_SCATTER_VEC(2); break;
         case 4: GCOO_SCATTER_VEC(4); break;
-        case 8: GCOO_SCATTER_VEC(8); break;
+        case 8:
+            scatter_vec_kernel<8, true><<<grid, kScatterThreads, 0, st>>>(A, m, k, group_index, row_ptr, vals, rows,
+                                                                          cols, packed);
+            break;
         default: return cudaErrorInvalidValue;
         }
 #undef GCOO_SCATTER_VEC
