@@ -787,7 +787,7 @@ cudaError_t launch_prefix_scan(int32_t *cnt, int64_t segments, int32_t *row_ptr,
 
 cudaError_t launch_scatter(const float *A, int64_t m, int64_t k, int32_t cpg, const int32_t *group_index,
                            const int32_t *row_ptr, float *vals, int32_t *rows, int32_t *cols, Entry *packed,
-                           cudaStream_t st)
+                           cudaStream_t st, bool dense)
 {
     const int64_t ng = (m + cpg - 1) / cpg;
     if (ng <= 0)
@@ -796,10 +796,10 @@ cudaError_t launch_scatter(const float *A, int64_t m, int64_t k, int32_t cpg, co
     // Rows that do not start on 16 bytes: the vector kernel up to 4 rows per group
     // (4000 x 4001 at 2 %: 1 row 43 us against 79 of 4-byte loads, 2 42 / 57, 4 44 /
     // 58); with 8 its shifted rows take too many registers (84 / 61; 5653 x 5910 at
-    // 16 % 235 / 108).
+    // 16 % 235 / 108). Known to be dense: one row per group only (4000 x 4001 at
+    // 40 % 51 / 88, 2 69 / 67, 4 96 / 80).
     const bool al = k % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
-    // 16 % 235 / 108).
-    if (al ? cpg <= 8 : (reinterpret_cast<uintptr_t>(A) & 3) == 0 && cpg <= 4) {
+    if (al ? cpg <= 8 : (reinterpret_cast<uintptr_t>(A) & 3) == 0 && cpg <= (dense ? 1 : 4)) {
 #define GCOO_SCATTER_VEC(C)                                                                                         \
     (al ? scatter_vec_kernel<C, true> : scatter_vec_kernel<C, false>)<<<grid, kScatterThreads, 0, st>>>(            \
         A, m, k, group_index, row_ptr, vals, rows, cols, packed)

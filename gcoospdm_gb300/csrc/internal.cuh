@@ -143,7 +143,7 @@ cudaError_t launch_row_scan_max(int32_t *row_counts_then_ptr, int64_t m, int32_t
 // Group arrays only (count entry point without row pointers): from row counts.
 cudaError_t launch_scatter(const float *A, int64_t m, int64_t k, int32_t rows_per_group,
                            const int32_t *group_index, const int32_t *row_ptr, float *vals,
-                           int32_t *rows, int32_t *cols, Entry *packed, cudaStream_t st);
+                           int32_t *rows, int32_t *cols, Entry *packed, cudaStream_t st, bool dense = false);
 
 // ---- tiled conversion (convert_tiled.cu): a warp per (group, 128-column segment)
 int64_t conv_segments(int64_t k); // segments per row: the count array is m x conv_segments(k)
