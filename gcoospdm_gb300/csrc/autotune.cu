@@ -113,7 +113,7 @@ gcoo_status gcoo_autotune(gcoo_handle *h, const float *dB, int64_t n, float *dC,
         const LaunchShape s = pick_shape(p, h->m, n, h->nnz, h->max_row_nnz, reinterpret_cast<uintptr_t>(dB),
                                          reinterpret_cast<uintptr_t>(dC));
         if (s.vec != p.vec)
-            continue; // not valid for this width / alignment
+            continue; // narrowed for this width and alignment: a narrower candidate's shape
         gcoo_status r = spdm_fp32(h, dB, n, dC, st, &p); // warm-up
         if (r != GCOO_SUCCESS)
             continue;

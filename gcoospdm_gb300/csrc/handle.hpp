@@ -14,7 +14,7 @@ void destroy_left_plan(LeftPlan *p);
 
 struct gcoo_handle;
 namespace gcoo {
-// Whether multiplies walk groups in GCOO order (api.cu): forced by
+// Whether multiplies may walk a group's rows together (api.cu): forced by
 // fp32_order, else when the rows of a group share columns.
 bool group_order_chosen(const gcoo_handle *h);
 } // namespace gcoo

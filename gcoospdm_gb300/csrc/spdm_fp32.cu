@@ -1,14 +1,15 @@
 // spdm_fp32.cu -- the plain FP32 GCOO x dense multiply on sm_103a.
 //
 // Replaces sparse_dense_groupcoo_mat_mul_kernel (src/gcoo_spdm_kernels.cu:
-// 92-158). One CTA per (GCOO group, column tile):
-//   * one elected thread stages the group's nonzeros (the contiguous range
+// 92-158). One CTA per (GCOO group, or part of one, and span of column tiles):
+//   * one elected thread stages the CTA's nonzeros (the contiguous range
 //     [row_ptr[g*cpg], row_ptr[(g+1)*cpg]) of the packed row-ordered layout)
 //     into shared memory with cp.async.bulk, completing on an mbarrier;
-//   * each warp owns one row of the group and 32*V output columns; for every
-//     entry of its row (a shared-memory broadcast) each lane loads V
-//     consecutive B values with one 128-bit (V=4) coalesced load and updates
-//     V register accumulators with fmaf;
+//   * each warp owns one row and walks the span's tiles of 32*V output columns
+//     from that one staging; for every entry of its row (a shared-memory
+//     broadcast) each lane loads V B values, consecutive in one 128-bit load
+//     (V = 4) or in pieces of W where n or B is not 16-byte aligned, and
+//     updates V register accumulators with fmaf;
 //   * rows of the group run side by side, so B rows shared by several rows of
 //     a group are served from L1.
 // Every C element is a sequential fmaf chain over its row's entries in

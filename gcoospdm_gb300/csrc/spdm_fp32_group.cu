@@ -22,7 +22,10 @@
 // converted by spdm_lowp.cu: bf16, or E4M3 with per-column scales applied to
 // the finished sums): a B segment is decoded once per column run instead of
 // once per row. Per element the entries are the same and in the same order as
-// in the row walk of those forms, so the results are identical to it.
+// in the row walk of those forms, so the results are identical to it. Those
+// forms come here only where the caller asks for the order (their row walk is
+// the faster one); FP32 does for blocks of about four rows, wide and large
+// (shared_walk, api.cu).
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 

@@ -473,7 +473,8 @@ cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int6
                         ticket, host);
 }
 
-// Wider B stays with the group walk, whose tile count decides what is possible
+// Column tiles along the grid's y: wider B takes another walk (shared_walk,
+// api.cu), whose tile count decides what is possible
 bool panel_ok(int64_t n) { return n <= 1 << 20; }
 
 cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, const int32_t *pref, int64_t m,

@@ -102,32 +102,23 @@ __device__ __forceinline__ void fma_pair(unsigned long long &acc, unsigned long 
 
 // V columns of shared memory in registers, and their chains
 template <int V>
-struct Chain {
-    unsigned long long acc[V / 2];
-    __device__ __forceinline__ void zero()
-    {
-#pragma unroll
-        for (int v = 0; v < V / 2; ++v)
-            acc[v] = 0ull;
-    }
+struct Chain;
+template <>
+struct Chain<4> {
+    unsigned long long lo, hi; // two columns each
+    __device__ __forceinline__ void zero() { lo = hi = 0ull; }
     __device__ __forceinline__ void add(float val, const float *b)
     {
-        unsigned long long vv, x[V / 2];
+        unsigned long long vv;
         asm("mov.b64 %0, {%1, %1};" : "=l"(vv) : "f"(val));
-        if (V == 4) {
-            const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(b);
-            x[0] = t.x;
-            x[V / 2 - 1] = t.y;
-        } else {
-            x[0] = *reinterpret_cast<const unsigned long long *>(b);
-        }
-#pragma unroll
-        for (int v = 0; v < V / 2; ++v)
-            fma_pair(acc[v], vv, x[v]);
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(b);
+        fma_pair(lo, vv, t.x);
+        fma_pair(hi, vv, t.y);
     }
     __device__ __forceinline__ float at(int v) const
     {
-        return __uint_as_float(static_cast<unsigned>(v & 1 ? acc[v / 2] >> 32 : acc[v / 2]));
+        const unsigned long long two = v < 2 ? lo : hi;
+        return __uint_as_float(static_cast<unsigned>(v & 1 ? two >> 32 : two));
     }
 };
 template <>
@@ -154,7 +145,6 @@ __device__ __forceinline__ void cp_async_w(void *dst, const void *src)
 // their instructions are (half as many per column; 65536 rows, n = 256 119 us,
 // V = 1 136, V = 2 123-126). Two copy warps instead of four: 1-10 % more;
 // eight at V = 4: 7 % more.
-template <int V>
 constexpr int kCopyWarps = 4;
 template <int V>
 constexpr int kBatch = V == 1 ? 128 : 32; // entries per step
@@ -183,12 +173,12 @@ struct Spread {
 
 // V: columns per lane of the chain warp; W: floats per copy (B's alignment)
 template <int V, int W>
-__global__ void __launch_bounds__(32 * (1 + kCopyWarps<V>))
+__global__ void __launch_bounds__(32 * (1 + kCopyWarps))
 spdm_long_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ row_ptr,
                  const int32_t *__restrict__ list, unsigned tiles, const Spread spread, const float *__restrict__ B,
                  int64_t n, float *__restrict__ C)
 {
-    constexpr int kCols = 32 * V, kChunks = kCols / W, kWarps = kCopyWarps<V>;
+    constexpr int kCols = 32 * V, kChunks = kCols / W, kWarps = kCopyWarps;
     constexpr int BATCH = kBatch<V>, DEPTH = kDepth<V>, EDEPTH = 2 * DEPTH; // entries land before their pieces are requested
     extern __shared__ __align__(16) float s_b[]; // [DEPTH][BATCH][kCols]
     Entry *s_e = reinterpret_cast<Entry *>(s_b + DEPTH * BATCH * kCols); // [EDEPTH][BATCH]
@@ -297,7 +287,7 @@ cudaError_t launch_long(const Entry *packed, const int32_t *row_ptr, const int32
     const cudaError_t e = cudaFuncSetAttribute(spdm_long_kernel<V, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
     if (e != cudaSuccess)
         return e;
-    spdm_long_kernel<V, W><<<static_cast<unsigned>(ctas), 32 * (1 + kCopyWarps<V>), smem, st>>>(
+    spdm_long_kernel<V, W><<<static_cast<unsigned>(ctas), 32 * (1 + kCopyWarps), smem, st>>>(
         packed, row_ptr, list, static_cast<unsigned>(tiles), spread, B, n, C);
     count_launches(1);
     return cudaGetLastError();
@@ -307,8 +297,9 @@ cudaError_t launch_long(const Entry *packed, const int32_t *row_ptr, const int32
 
 int32_t long_row_min() { return 256; }
 
-// Any width and alignment of B (copies of 16, 8 or 4 bytes) within the grids
-// of this kernel and the short rows'.
+// What this kernel and the short rows' can run: any alignment of B (copies of
+// 16, 8 or 4 bytes), widths within their grids. Where they gain is another
+// question (long_rows_pay, api.cu).
 bool long_rows_ok(int64_t m, int64_t n)
 {
     const int64_t tiles = (n + 31) / 32;

@@ -25,7 +25,7 @@ namespace gcoo {
 struct LowpWork {
     DevBuf<uint16_t> bf;     // k*n bf16 (FP8: E4M3 values as bf16)
     DevBuf<uint32_t> split;  // k*n (hi | lo << 16) bf16 pairs
-    DevBuf<uint8_t> f8;      // k*n e4m3 (the group walk's)
+    DevBuf<uint8_t> f8;      // k*n e4m3 (wide B and the group walk)
     DevBuf<float> scale;     // n column scales
     DevBuf<unsigned> amax;   // n column absmax (float bits)
 };

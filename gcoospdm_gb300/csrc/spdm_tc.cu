@@ -20,9 +20,10 @@
 // half of four tiles and its 128-column halves of their B tiles per stage
 // with tensor-map bulk copies (cta_group::2, completing on the first CTA's
 // barrier), and the first CTA issues tcgen05.mma.cta_group::2 (M=256, N=256,
-// K=16) into both CTAs' tensor memory, one accumulator per 256 columns. Split-BF16 kernel (spdm_tc_split_kernel): equal shares of the
-// (tile, 128 columns) products, two CTAs per SM, one stage per tile, six MMAs
-// per tile. Every wait is bounded.
+// K=16) into both CTAs' tensor memory, one accumulator per 256 columns.
+// Split-BF16 kernel (spdm_tc_split_kernel): equal shares of the (tile, 128
+// columns) products, or (panel, 128 columns) where panels have few tiles, two
+// CTAs per SM, one stage per tile, six MMAs per tile. Every wait is bounded.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -323,13 +324,13 @@ b_tiles_kernel(const float *__restrict__ B, int64_t k, int64_t n, int64_t kb, __
     }
 }
 
-// ---- split-BF16: one CTA per equal share of the tiles ---------------------------------
+// ---- split-BF16: one CTA per equal share of the tiles, or per panel and strip ----------
 // The tile products (tile t of the plan x 128 output columns jt) are ordered
 // w = jt * tiles + t and cut into equal consecutive shares, one per CTA, two
 // CTAs per SM: no wave of CTAs is nearly empty and a few panels fill the GPU.
 // Measured with 16 x 16 blocks at 25 % (us; a CTA per panel and 128 columns
-// before): 8192^2, n = 1024 458 -> 393 (the kernel 424 -> 352, 2.1 PFLOP/s of
-// MMAs, and 13 of fix-up), n = 128 216 -> 84; 2048 x 8192, n = 256 222 -> 57;
+// before): 8192^2, n = 1024 472-478 -> 436-453 by GPU and run (the MMAs 387 at
+// their measured peak rate, 13 of fix-up), n = 128 216 -> 84; 2048 x 8192, n = 256 222 -> 57;
 // 2048^2, n = 1024 67 -> 49; 1024^2 at 15 %, n = 64 32 -> 24. A share is
 // walked panel by panel; a (panel, jt) that lies in one share is written to
 // C, the others' sums go to a workspace and tc_fixup_kernel adds them in
@@ -580,7 +581,7 @@ spdm_tc_split_kernel(const int32_t *__restrict__ pf, const int32_t *__restrict__
             ++piece;
         }
     }
-    __syncwarp(); // warps 4 and 5: their one working lane is back
+    __syncwarp(); // warps 4 and 5: their elected lanes are back
     __syncthreads();
     // after a wait gave up, copies already issued may still be landing in
     // this CTA's shared memory: give them a bounded time before it is released
@@ -958,7 +959,7 @@ spdm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             ++piece;
         }
     }
-    __syncwarp(); // warps 4 and 5: their one working lane is back
+    __syncwarp(); // warps 4 and 5: their elected lanes are back
     // after a wait gave up (in either CTA: the status word), copies already
     // issued may still be landing in this CTA or signalling the first CTA's
     // barriers: give them a bounded time before the pair leaves
