@@ -77,9 +77,13 @@ seg_count_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tile
     float4 v[CPG];
 #pragma unroll
     for (int r = 0; r < CPG; ++r)
-        v[r] = (u.live && r < u.nrows) // warp-uniform
-                   ? seg_load<AL, false>(A + (u.r0 + r) * k + u.s * kSegCols, lane, k - u.s * kSegCols, A, A + m * k)
-                   : make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (AL)
+            v[r] = r < u.nrows && u.c < k ? __ldg(reinterpret_cast<const float4 *>(A + (u.r0 + r) * k + u.c))
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        else
+            v[r] = (u.live && r < u.nrows) // warp-uniform
+                       ? seg_load<AL, false>(A + (u.r0 + r) * k + u.s * kSegCols, lane, k - u.s * kSegCols, A, A + m * k)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t any = 0;
 #pragma unroll
     for (int r = 0; r < CPG; ++r) {
@@ -155,9 +159,13 @@ __device__ __forceinline__ void scatter_segment(const float *__restrict__ A, int
     float4 v[CPG];
 #pragma unroll
     for (int r = 0; r < CPG; ++r)
-        v[r] = r < u.nrows // warp-uniform
-                   ? seg_load<AL, true>(A + (u.r0 + r) * k + u.s * kSegCols, lane, k - u.s * kSegCols, A, A + m * k)
-                   : make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (AL)
+            v[r] = r < u.nrows && u.c < k ? __ldcs(reinterpret_cast<const float4 *>(A + (u.r0 + r) * k + u.c))
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        else
+            v[r] = r < u.nrows // warp-uniform
+                       ? seg_load<AL, true>(A + (u.r0 + r) * k + u.s * kSegCols, lane, k - u.s * kSegCols, A, A + m * k)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t bits[CPG];
     uint32_t word[NP];
     uint32_t any = 0;
