@@ -55,3 +55,23 @@ def test_view_skips_rows_of_other_groups(native, oracle_mod):
     C = native.spdm_view(24, 90, 4, t(ref.groupIndex), t(ref.nnzPerGroup), t(ref.vals), t(rows), t(ref.cols), t(B))
     want = oracle_mod.spdm(oracle_mod.convert(A2, 4), B)
     assert np.array_equal(C.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("cpg", [1, 2, 4])
+@pytest.mark.parametrize("n", [1, 55, 130, 256])
+def test_groups_around_a_chunk(native, oracle_mod, n, cpg):
+    """Groups of one entry less and more than one, two and three staged chunks (256 entries per row of a group)."""
+    import torch
+    rng = np.random.default_rng(n + cpg)
+    totals = [c * 256 * cpg + d for c in (1, 2, 3) for d in (-1, 0, 1)] + [0, 1]
+    k = 800
+    A = np.zeros((len(totals) * cpg, k), np.float32)
+    for i, total in enumerate(totals):
+        at = rng.choice(cpg * k, total, replace=False)
+        A[i * cpg + at // k, at % k] = rng.standard_normal(total)
+    B = rng.standard_normal((k, n)).astype(np.float32)
+    ref = oracle_mod.convert(A, cpg)
+    t = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    C = native.spdm_view(A.shape[0], k, cpg, t(ref.groupIndex), t(ref.nnzPerGroup), t(ref.vals), t(ref.rows),
+                         t(ref.cols), t(B))
+    assert np.array_equal(C.cpu().numpy().view(np.uint32), oracle_mod.spdm(ref, B).view(np.uint32))
