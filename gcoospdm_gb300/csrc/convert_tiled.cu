@@ -62,6 +62,52 @@ __device__ __forceinline__ SegUnit seg_unit(int64_t m, int64_t k, int64_t tiles,
     return u;
 }
 
+// The nonzero bits of a warp's segment, four columns per lane and row, of rows
+// that need not start on 16 bytes. A row's segment is shifted by 0..3 floats
+// against the granules; each lane loads one granule, lane r also the 33rd of
+// row r, and the lanes shift their bits, not their floats (one shuffle a row
+// where seg_load has three, and one 33rd load a warp; counting 4001 x 3999, 4 rows
+// per group 24.9 -> 16.4 us, 1 row 27.1 -> 25.8). Granules that may reach outside A
+// (the first and the last groups'): seg_load.
+template <int CPG>
+__device__ __forceinline__ void seg_bits(const float *__restrict__ A, int64_t m, int64_t k, const SegUnit &u, int lane,
+                                         uint32_t (&bits)[CPG])
+{
+    const int64_t first = u.r0 * k + u.s * kSegCols; // of row 0's segment
+    const int64_t valid = k - u.s * kSegCols;        // columns from the segment's start on
+    // loads reach at most 3 floats before a row's segment and 6 past its valid columns
+    const bool inside = first >= 4 && (m - u.r0 - u.nrows) * k >= 8;
+    if (!u.live || !inside) { // warp-uniform
+#pragma unroll
+        for (int r = 0; r < CPG; ++r)
+            bits[r] = u.live && r < u.nrows
+                          ? nz_bits(seg_load<false, false>(A + first + r * k, lane, valid, A, A + m * k))
+                          : 0u;
+        return;
+    }
+    const uint32_t at = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(A) >> 2) + static_cast<uint32_t>(first);
+    const auto shift = [&](int r) { return (at + static_cast<uint32_t>(r) * static_cast<uint32_t>(k)) & 3u; };
+    const bool on = 4 * lane < valid + 3;
+    float4 v[CPG];
+#pragma unroll
+    for (int r = 0; r < CPG; ++r)
+        v[r] = on && r < u.nrows
+                   ? __ldg(reinterpret_cast<const float4 *>(A + first + r * k - shift(r) + 4 * lane))
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < u.nrows && shift(lane) != 0 && valid > kSegCols - 3)
+        e = __ldg(reinterpret_cast<const float4 *>(A + first + lane * k - shift(lane) + kSegCols));
+    const uint32_t beyond = nz_bits(e);
+    const int64_t left = valid - 4 * lane;
+    const uint32_t mask = left >= 4 ? 15u : (left > 0 ? (1u << left) - 1u : 0u);
+#pragma unroll
+    for (int r = 0; r < CPG; ++r) {
+        const uint32_t own = nz_bits(v[r]);
+        const uint32_t down = __shfl_down_sync(0xffffffffu, own, 1), last = __shfl_sync(0xffffffffu, beyond, r);
+        bits[r] = ((own | (lane == 31 ? last : down) << 4) >> shift(r)) & mask;
+    }
+}
+
 // distinct (when not null) accumulates the number of distinct (group,
 // column) pairs, i.e. columns with a nonzero in at least one row of the
 // group; nnz / distinct tells how many rows of a group share a B row.
@@ -74,22 +120,24 @@ seg_count_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tile
     __shared__ int s_dist[kSegsPerCta];
     const SegUnit u = seg_unit<CPG>(m, k, tiles, blockIdx.x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float4 v[CPG];
+    uint32_t bits[CPG]; // the lane's four columns of each row
+    if constexpr (AL) {
+        float4 v[CPG];
 #pragma unroll
-    for (int r = 0; r < CPG; ++r)
-        if constexpr (AL)
+        for (int r = 0; r < CPG; ++r)
             v[r] = r < u.nrows && u.c < k ? __ldg(reinterpret_cast<const float4 *>(A + (u.r0 + r) * k + u.c))
                                           : make_float4(0.f, 0.f, 0.f, 0.f);
-        else
-            v[r] = (u.live && r < u.nrows) // warp-uniform
-                       ? seg_load<AL, false>(A + (u.r0 + r) * k + u.s * kSegCols, lane, k - u.s * kSegCols, A, A + m * k)
-                       : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < CPG; ++r)
+            bits[r] = nz_bits(v[r]);
+    } else {
+        seg_bits<CPG>(A, m, k, u, lane, bits);
+    }
     uint32_t any = 0;
 #pragma unroll
     for (int r = 0; r < CPG; ++r) {
-        const uint32_t b = nz_bits(v[r]);
-        any |= b;
-        const int x = __reduce_add_sync(0xffffffffu, __popc(b));
+        any |= bits[r];
+        const int x = __reduce_add_sync(0xffffffffu, __popc(bits[r]));
         if (u.live && lane == r && r < u.nrows)
             cnt[(u.r0 + r) * S + u.s] = x;
     }
