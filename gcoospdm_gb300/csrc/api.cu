@@ -136,11 +136,14 @@ gcoo_status ensure_split_work(gcoo_handle *h, int64_t n)
 //   8192^2, 2 x 2 blocks, 25 %:   n 256 1557 /2425 / 927, n 1024 5791 /3156 /2856
 //   2048^2, 16 x 16, 40 % holes:  n 256  34 / 141 /  60, n 1024 78 / 154 / 84, n 2048 140 / 228 / 120
 // Panels win with many rows per panel column (share) and much work, so that
-// their CTAs fill the GPU: share^3 * nnz * n >= 2.9e11, the work counted
-// twice for long rows, which the row walk stages piecewise. Groups win for
-// blocks of four rows, wide and large. By this rule the multiplies take 1.3 %
-// longer than by the best walk of each (1 in 100 more than 1.3 times as long),
-// by the row walk alone 3 % and up to 6 times, by the group walk alone twice.
+// their CTAs fill the GPU: share^3 * nnz * n >= 6e10 * (5 + windows), a window
+// of 512 columns taking some 4 us to stage whatever it holds (16 x 16 blocks at
+// 1.7 %, rows / panels: 2747 x 7474, n = 272 30 / 61; 1758 x 9967, n = 280 34 / 71);
+// >= 1.5e11 for long rows, which the row walk stages piecewise (182 x 98796, 9217
+// entries a row, n = 496 5682 / 1345). Groups win for blocks of four
+// rows, wide and large. By this rule 4255 multiplies (wide matrices among them) take 1.1 % longer than by the best walk of each (1 in 100 more
+// than 1.25 times as long), by the row walk alone 3 % and up to 6 times, by the
+// group walk alone twice.
 enum SharedWalk { kWalkRows, kWalkGroups, kWalkPanels };
 
 static SharedWalk shared_walk(const gcoo_handle *h, int64_t n, uintptr_t b, uintptr_t c)
@@ -159,10 +162,15 @@ static SharedWalk shared_walk(const gcoo_handle *h, int64_t n, uintptr_t b, uint
     // groups 111, panels 66 us)
     if (h->n_long > 0 && work < 5e5 * static_cast<double>(h->max_row_nnz))
         return kWalkRows;
-    if (panel_ok(n) && n >= 96 && share >= 4.0 && share * share * share * work * (long_rows ? 2 : 1) >= 2.9e11)
+    const int64_t windows = (h->k + 511) / 512;
+    const double enough = long_rows ? 1.5e11 : 6e10 * static_cast<double>(5 + windows);
+    if (panel_ok(n) && n >= 96 && share >= 4.0 && share * share * share * work >= enough)
         return kWalkPanels;
     const bool vec4 = n % 4 == 0 && !((b | c) & 15);
-    return vec4 && n >= 640 && sharing4 >= 3.3 && work >= 3e8 && h->n_long == 0 ? kWalkGroups : kWalkRows;
+    // a CTA per group and 1024 columns: with few of them the row walk (263 x 2693 at
+    // 49 %, n = 940 107 / 420)
+    const bool many = long_rows || h->m * ((n + 1023) / 1024) >= 2000;
+    return vec4 && n >= 640 && sharing4 >= 3.3 && work >= 3e8 && many && h->n_long == 0 ? kWalkGroups : kWalkRows;
 }
 
 static SharedWalk fp32_walk(const gcoo_handle *h, int64_t n, const float *dB, const float *dC)

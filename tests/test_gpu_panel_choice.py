@@ -39,7 +39,7 @@ def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
 @pytest.mark.parametrize("rows,holes,n,kernel", [
     (2, 0.0, 1024, "spdm_fp32_kernel"), (2, 0.0, 1001, "spdm_fp32_kernel"), (2, 0.0, 128, "spdm_fp32_kernel"),
     (4, 0.0, 1024, "spdm_group_kernel"), (4, 0.0, 1001, "spdm_fp32_kernel"), (4, 0.0, 512, "spdm_fp32_kernel"),
-    (16, 0.4, 1024, "spdm_panel_kernel"), (16, 0.4, 1001, "spdm_panel_kernel"), (16, 0.4, 256, "spdm_fp32_kernel")])
+    (16, 0.4, 2048, "spdm_panel_kernel"), (16, 0.4, 2001, "spdm_panel_kernel"), (16, 0.4, 1024, "spdm_fp32_kernel")])
 @pytest.mark.parametrize("k", [2048, 2047])
 def test_choice_by_sharing_and_work(native, rows, holes, n, kernel, k):
     """Blocks of several heights at 15 %: the walk by how many rows share a
@@ -57,6 +57,23 @@ def test_choice_by_sharing_and_work(native, rows, holes, n, kernel, k):
     want = h.spdm(B, C).clone()
     for order in ("rows", "groups"):
         assert torch.equal(want, native.GcooHandle(A, fp32_order=order).build().spdm(B)), order
+
+
+@pytest.mark.parametrize("m,k,density,n,kernel", [
+    (2048, 2048, 0.25, 256, "spdm_panel_kernel"),  # four windows of 512 columns
+    (2048, 16384, 0.03125, 256, "spdm_fp32_kernel"),  # as many entries in 32
+    (2048, 16384, 0.25, 256, "spdm_panel_kernel")])  # long rows
+def test_choice_by_the_windows(native, m, k, density, n, kernel):
+    """Few entries in each of many windows of columns: not the panels."""
+    import torch
+    A = blocks(m, k, 16, density)
+    h = native.GcooHandle(A).build()
+    B, C = torch.ones(k, n, device="cuda"), torch.empty(m, n, device="cuda")
+    s = torch.cuda.Stream()
+    names = [name for name, _ in captured_kernels(s, lambda: h.spdm(B, C, stream=s))]
+    assert len(names) == 1 and kernel in names[0], names
+    torch.cuda.synchronize()
+    assert torch.equal(h.spdm(B), A.sum(1, keepdim=True).expand(-1, n))  # whole numbers: exact
 
 
 def test_multiply_by_returns_with_the_multiply_under_way(native):
