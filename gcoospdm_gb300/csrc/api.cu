@@ -506,6 +506,9 @@ struct NextMultiply {
     bool done;
 };
 
+// last density up to which one read of A takes any matrix (build_handle)
+constexpr double kStagedDensity = 0.26;
+
 static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *mul)
 {
     const bool ahead = mul && h->built && !h->coo && h->n_long == 0 && h->p.fp32_sum == GCOO_SUM_CHAIN &&
@@ -534,18 +537,20 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
     // steady loop of mutiplyBy / build); otherwise, or if they turn out too
     // small, the two-pass path below converts and sizes them exactly.
     const int64_t cap = std::min<int64_t>(static_cast<int64_t>(h->vals.count), static_cast<int64_t>(h->rc.count / 2));
-    // Not where much lies above 28 % (the slots hold 25 %): nearly every tile
+    // Not where much lies above 26 % (the slots hold 25 %): nearly every tile
     // overflows and is read again (8192^2, 4 rows: at 40 % 635 us, two passes 521, at
     // 30 % 477 / 386, at 25 % 323 / 333; 4000 x 4001 at 40 % 184 / 139), sooner off
     // 16-byte boundaries, where the second pass is another kernel (3000 x 3001: at
-    // 60 % 161 / 97, at 90 % 240 / 121; 2000 x 2001 at 90 % 97 / 74). With few entries
-    // the wait between the passes costs more (multiply_by, n = 8, of 7062 x 1257 at
-    // 40 % 167 / 166, 2000 x 2001 at 40 % 88 / 92, 1000 x 1001 52 / 58; aligned: 2000^2 at
-    // 90 % 154 / 158, 3000^2 at 60 % 318 / 291).
+    // 60 % 161 / 97, at 90 % 240 / 121; 2000 x 2001 at 90 % 97 / 74; aligned: 3000^2 at
+    // 60 % 146 / 121, 2000^2 92 / 85 at 90 %). With few entries, and more of them where
+    // a multiply is enqueued ahead, the wait between the passes costs more
+    // (multiply_by, n = 8, of 7062 x 1257 at 40 % 167 / 166, 2000 x 2001 at 40 % 88 /
+    // 92, 1000 x 1001 52 / 58; 2000^2 at 90 % 154 / 158, 3000^2 at 60 % 318 / 291).
     const double size = static_cast<double>(h->m) * static_cast<double>(h->k);
     const bool shifted = h->k % 4 != 0 || (reinterpret_cast<uintptr_t>(h->dA) & 15) != 0; // rows off 16 bytes
-    const double above = static_cast<double>(h->nnz) - 0.28 * size;
-    const bool one_read = above <= 0 || (size < 1.5e7 && above <= (shifted ? 8e5 : 2.5e6));
+    const double above = static_cast<double>(h->nnz) - kStagedDensity * size;
+    const double most = ahead ? (shifted ? 8e5 : 2.5e6) : (shifted ? 3e5 : 6e5);
+    const bool one_read = above <= 0 || (size < 1.5e7 && above <= most);
     if (tiled && h->vals.ptr && h->rc.ptr && cap > 0 && one_read && staged_convert_ok(h->dA, h->m, h->k, cpg)) {
         const int64_t tiles = staged_tiles(h->m, h->k, cpg);
         const int32_t slot = staged_slot(h->nnz, tiles, cpg);
@@ -647,7 +652,7 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
     int32_t *cols = h->rc.ptr + nnz;
     // dense rows off 16-byte boundaries: a CTA per group with 4-byte loads (4000 x
     // 4001 at 40 %, 4 rows: two passes 139 us, with shifted rows 161)
-    const bool dense = static_cast<double>(total) > 0.28 * size && shifted && cpg > 1;
+    const bool dense = static_cast<double>(total) > kStagedDensity * size && shifted && cpg > 1;
     if (tiled && !dense)
         GCOO_CUDA(launch_tile_scatter(h->dA, h->m, h->k, cpg, h->tile_cnt.ptr, h->group_index(), h->row_ptr.ptr,
                                       h->vals.ptr, rows, cols, h->packed.ptr, st));
