@@ -913,7 +913,13 @@ cudaError_t launch_spdm_view(const gcoo_view &a, const float *B, int64_t n, floa
     if ((n + 127) / 128 > 65535) // the widest B this entry point takes
         return cudaErrorInvalidConfiguration;
     const int cpg = a.rows_per_group;
-    const int warps = cpg < kViewMaxWarps ? cpg : kViewMaxWarps;
+    // Short rows: a CTA's staging is most of it, and two warps of a few rows
+    // each let more groups be resident (60000 x 1000, 1 entry a row, n = 1: 4 rows
+    // per group 23.6 us, 19.6 so, 8 rows 23.7 / 17.2; 32 rows 18.5 / 18.9, n = 130
+    // 27.9 / 40.0)
+    const double len = a.m > 0 ? static_cast<double>(a.nnz) / static_cast<double>(a.m) : 0.0;
+    const int most = len < 8.0 && cpg <= 8 ? 2 : kViewMaxWarps;
+    const int warps = cpg < most ? cpg : most;
     gcoo_params p{};
     p.rows_per_group = cpg;
     p.warps = p.col_warps = 1;
@@ -926,10 +932,14 @@ cudaError_t launch_spdm_view(const gcoo_view &a, const float *B, int64_t n, floa
     int chunk = 256;
     while (chunk < warps * 256 && chunk < 2 * mean + 64)
         chunk *= 2;
-    // as the row walk: about 768 columns per CTA, but four waves of CTAs
+    // as the row walk: about 768 columns per CTA, but four waves of CTAs, two
+    // of rows under 16 entries, one at most under 8 (1 entry a row, four waves /
+    // as now, us: 5606 x 336, n = 218, 4 rows per group 13.1 / 9.8, n = 801 18.5 /
+    // 12.2; 8000 x 300, n = 130 13.3 / 9.9)
     const int64_t tile = 32 * s.vec, tiles = (n + tile - 1) / tile;
     const int64_t resident = static_cast<int64_t>(device_sms()) * kRowCtas * 4 / warps;
-    int64_t ci = a.n_group * tiles / (4 * resident);
+    const int64_t waves = len < 8.0 ? 1 : (len < 16.0 ? 2 : 4);
+    int64_t ci = (a.n_group * tiles + (len < 8.0 ? resident - 1 : 0)) / (waves * resident);
     ci = ci > 768 / tile ? 768 / tile : ci;
     ci = ci < 1 ? 1 : ci;
     while ((tiles + ci - 1) / ci > 65535)

@@ -75,3 +75,23 @@ def test_groups_around_a_chunk(native, oracle_mod, n, cpg):
     C = native.spdm_view(A.shape[0], k, cpg, t(ref.groupIndex), t(ref.nnzPerGroup), t(ref.vals), t(ref.rows),
                          t(ref.cols), t(B))
     assert np.array_equal(C.cpu().numpy().view(np.uint32), oracle_mod.spdm(ref, B).view(np.uint32))
+
+
+@pytest.mark.parametrize("cpg", [1, 4, 8, 16])
+@pytest.mark.parametrize("m,entries", [(3000, 1), (40000, 1), (40000, 7), (3000, 9), (700, 17)])
+def test_short_rows(native, cpg, m, entries):
+    """Rows of few entries, few and many waves of groups: one strip of columns per group or several."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(m + entries)
+    k = 300
+    A = torch.randint(1, 5, (m, k), generator=gen, device="cuda").float()
+    A.masked_fill_(torch.rand(m, k, generator=gen, device="cuda") >= entries / k, 0.0)
+    gi, npg, nnz = native.convert_count(A, cpg)
+    vals, rows, cols = native.convert_scatter(A, gi, nnz, cpg)
+    for n in (1, 130, 801):
+        B = torch.randint(-8, 9, (k, n), generator=gen, device="cuda").float()
+        C = torch.full((m + 1, n), 7.0, device="cuda")
+        native.spdm_view(m, k, cpg, gi, npg, vals, rows, cols, B, C[:m])
+        want = native.GcooHandle(A, fp32_order="rows").build().spdm(B)
+        assert torch.equal(C[:m], want) and bool((C[m] == 7.0).all())
+        assert torch.equal(want.double(), A.double() @ B.double())  # whole numbers: exact
