@@ -46,3 +46,12 @@ def test_one_wave_of_ten_and_of_twelve_ctas(native, oracle_mod, n):
         assert abs(ctas - per_sm * sms) <= tiles
         names.append(name)
     assert names[0] == names[3] != names[1] == names[2], names
+
+
+@pytest.mark.parametrize("rows_per_group", [1, 4, 8, 32])
+@pytest.mark.parametrize("n", [1, 100, 133])
+def test_rows_longer_than_a_chunk(native, oracle_mod, rows_per_group, n):
+    """Rows of more entries than a CTA stages at once: one row per CTA."""
+    m = 301
+    _, ctas = check(native, oracle_mod, m, 2700, n, 2400, rows_per_group)
+    assert ctas % m == 0, ctas
