@@ -739,7 +739,7 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
     // at 50 %, n = 1: 32 rows 1667 us, 4 rows 212, one 155; 300 x 8192, n = 16 7206 /
     // 840 / 216).
     const auto fits = [&](int rows) { return max_row > 0 && max_row * static_cast<int64_t>(rows) + 2 <= kChunk; };
-    if (!skewed && p.warps <= 0 && p.col_warps <= 0)
+    if (!skewed && p.warps <= 0 && p.col_warps <= 0 && max_row > 0) // 0: not known
         while (s.rows > 1 && !fits(s.rows))
             s.rows = s.rows / 2 > 0 ? s.rows / 2 : 1;
     const int cpg = s.rows;
