@@ -299,8 +299,8 @@ seg_scatter_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t ti
                    int32_t *__restrict__ cols, Entry *__restrict__ packed)
 {
     grid_wait_previous();
-    scatter_segment<CPG, AL>(A, m, k, S, seg_unit<CPG>(m, k, tiles, blockIdx.x), pref, group_index, row_ptr, vals, rows,
-                         cols, packed);
+    scatter_segment<CPG, AL>(A, m, k, S, seg_unit<CPG>(m, k, tiles, blockIdx.x), written(pref), written(group_index),
+                             written(row_ptr), vals, rows, cols, packed);
 }
 
 // ---- staged rebuild: A read once --------------------------------------------------
@@ -570,6 +570,14 @@ place_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t tiles, i
              int64_t staged_blocks, int32_t *__restrict__ void_rows)
 {
     grid_wait_previous();
+    stage = written(stage);
+    tile_tot = written(tile_tot);
+    over_list = written(over_list);
+    over_count = written(over_count);
+    pref = written(pref);
+    group_index = written(group_index);
+    row_ptr = written(row_ptr);
+    d_total = written(d_total);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool staged_block = static_cast<int64_t>(blockIdx.x) < staged_blocks;
     const int64_t b = static_cast<int64_t>(blockIdx.x) * kSegsPerCta + warp;

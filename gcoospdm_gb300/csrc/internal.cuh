@@ -101,6 +101,17 @@ struct __align__(8) Entry {
 // call grid_launch_next: with it (and the staging kernel's) the row walk after
 // them took 4-8 % longer (8192^2 at 1 % 1083 -> 1138 us).
 __device__ __forceinline__ void grid_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A pointer to what a predecessor wrote, taken after grid_wait_previous. Loads
+// through a const __restrict__ parameter are invariant to the compiler, which
+// moves those whose address it has above the wait (a kernel that read totals
+// so always saw the zeros of the memset before); through this one they stay
+// below it. Loads at addresses that such a load returned follow it.
+template <typename T>
+__device__ __forceinline__ const T *written(const T *p)
+{
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
 __device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... P, typename... A>

@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(256)
 transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t R, int64_t Cc, bool early)
 {
     grid_wait_previous();
+    in = written(in);
     if (early)
         grid_launch_next();
     __shared__ float tile[kTr][kTr + 1];

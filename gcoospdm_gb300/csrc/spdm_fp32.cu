@@ -281,6 +281,7 @@ spdm_fp32_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
                  int32_t col_warps, int32_t col_iters, int32_t chunk_cap, uint32_t *__restrict__ status)
 {
     grid_wait_previous();
+    row_ptr = written(row_ptr);
     grid_launch_next();
     if (!MULTI)
         col_iters = 1;

@@ -131,6 +131,8 @@ spdm_panel_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ 
                   float *__restrict__ C)
 {
     grid_wait_previous();
+    row_ptr = written(row_ptr);
+    pref = written(pref);
     grid_launch_next();
     extern __shared__ __align__(16) unsigned char smem[];
     float *s_a = reinterpret_cast<float *>(smem);                             // [listed column][kPanelRows]
@@ -414,6 +416,7 @@ panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__
         s_sum[0] = s_sum[1] = 0;
     }
     grid_wait_previous();
+    row_ptr = written(row_ptr);
     __syncthreads();
     const int64_t begin = row_ptr[r0], end = row_ptr[r1];
     if (k > kShareCols) {

@@ -243,6 +243,8 @@ spdm_lowp_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__ r
                  float *__restrict__ C, int32_t col_iters, int32_t chunk, uint32_t *__restrict__ status)
 {
     grid_wait_previous();
+    row_ptr = written(row_ptr);
+    col_scale = written(col_scale);
     constexpr int V = FormTraits<F>::V;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
@@ -414,6 +416,7 @@ prep_fp8_kernel(const float *__restrict__ B, const unsigned *__restrict__ amax, 
                 void *__restrict__ out, int64_t k, int64_t n)
 {
     grid_wait_previous();
+    amax = written(amax);
     grid_launch_next();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t j = static_cast<int64_t>(blockIdx.x) * kStripCols + lane * 4;

@@ -606,6 +606,7 @@ tc_fixup_kernel(const int32_t *__restrict__ pf, int64_t m, int64_t n, int64_t kb
                 int cols, const float *__restrict__ part, float *__restrict__ C)
 {
     grid_wait_previous();
+    part = written(part);
     __shared__ __align__(16) float staging[2 * kPanel * kStageRow];
     const int R = blockDim.x;
     const int64_t panel = blockIdx.x, jt = blockIdx.y;
