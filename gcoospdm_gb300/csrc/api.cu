@@ -136,14 +136,16 @@ gcoo_status ensure_split_work(gcoo_handle *h, int64_t n)
 //   8192^2, 2 x 2 blocks, 25 %:   n 256 1557 /2425 / 927, n 1024 5791 /3156 /2856
 //   2048^2, 16 x 16, 40 % holes:  n 256  34 / 141 /  60, n 1024 78 / 154 / 84, n 2048 140 / 228 / 120
 // Panels win with many rows per panel column (share) and much work, so that
-// their CTAs fill the GPU: share^3 * nnz * n >= 6e10 * (5 + windows), a window
+// their CTAs fill the GPU: share^3 * nnz * n >= 5e10 * (5 + windows), a window
 // of 512 columns taking some 4 us to stage whatever it holds (16 x 16 blocks at
-// 1.7 %, rows / panels: 2747 x 7474, n = 272 30 / 61; 1758 x 9967, n = 280 34 / 71);
-// >= 1.5e11 for long rows, which the row walk stages piecewise (182 x 98796, 9217
-// entries a row, n = 496 5682 / 1345). Groups win for blocks of four
-// rows, wide and large. By this rule 4255 multiplies (wide matrices among them) take 1.1 % longer than by the best walk of each (1 in 100 more
-// than 1.25 times as long), by the row walk alone 3 % and up to 6 times, by the
-// group walk alone twice.
+// 1.7 %, rows / panels: 2747 x 7474, n = 272 30 / 61; 1758 x 9967, n = 280 34 / 71).
+// Less counts of the work where the last strip of 128 columns is not full and
+// where lanes copy B in 4-byte pieces, and rows of 1600 entries need twice as
+// much (1139 x 5876, 3379 a row in 16 x 16 blocks with holes, n = 190 227 / 458).
+// Groups win for blocks of four rows, wide and large. By this rule 5275
+// multiplies (wide matrices and long rows among them) take 1.1 % longer than by
+// the best walk of each (1 in 100 more than 1.27 times as long), by the row walk
+// alone 5 % and up to 4 times; by the group walk alone twice.
 enum SharedWalk { kWalkRows, kWalkGroups, kWalkPanels };
 
 static SharedWalk shared_walk(const gcoo_handle *h, int64_t n, uintptr_t b, uintptr_t c)
@@ -155,21 +157,21 @@ static SharedWalk shared_walk(const gcoo_handle *h, int64_t n, uintptr_t b, uint
     if (h->p.fp32_order == 2)
         return panel_ok(n) && share >= 1.75 * sharing4 ? kWalkPanels : kWalkGroups;
     const double work = static_cast<double>(h->nnz) * static_cast<double>(n);
-    const bool long_rows = h->nnz >= 1600 * h->m;
+    const bool vec4 = n % 4 == 0 && !((b | c) & 15);
     // a skewed matrix (its long rows have kernels of their own in the row walk):
     // panels once the work outweighs the one panel that walks the longest row's
     // columns (4308 x 667 in 16 x 16 blocks at 2 %, one full row, n = 1700: rows 36,
     // groups 111, panels 66 us)
     if (h->n_long > 0 && work < 5e5 * static_cast<double>(h->max_row_nnz))
         return kWalkRows;
-    const int64_t windows = (h->k + 511) / 512;
-    const double enough = long_rows ? 1.5e11 : 6e10 * static_cast<double>(5 + windows);
-    if (panel_ok(n) && n >= 96 && share >= 4.0 && share * share * share * work >= enough)
+    const double strips = static_cast<double>((n + 127) / 128 * 128), windows = static_cast<double>((h->k + 511) / 512);
+    const double counts = work * (static_cast<double>(n) / strips) * (vec4 ? 1.0 : 0.6);
+    const double enough = 5e10 * (5.0 + windows) * (h->nnz >= 1600 * h->m ? 2.0 : 1.0);
+    if (panel_ok(n) && n >= 96 && share >= 4.0 && share * share * share * counts >= enough)
         return kWalkPanels;
-    const bool vec4 = n % 4 == 0 && !((b | c) & 15);
     // a CTA per group and 1024 columns: with few of them the row walk (263 x 2693 at
     // 49 %, n = 940 107 / 420)
-    const bool many = long_rows || h->m * ((n + 1023) / 1024) >= 2000;
+    const bool many = h->m * ((n + 1023) / 1024) >= 2000;
     return vec4 && n >= 640 && sharing4 >= 3.3 && work >= 3e8 && many && h->n_long == 0 ? kWalkGroups : kWalkRows;
 }
 
@@ -384,7 +386,7 @@ gcoo_status gcoo_create(gcoo_handle **out, const float *dA, int64_t m, int64_t k
 namespace {
 
 constexpr size_t kReadbackWords = 8; // of a handle's page-locked readback
-constexpr int64_t kSampleEntries = 34500; // 16^3 * entries * 2048 columns < 2.9e11 below (shared_walk)
+constexpr int64_t kSampleEntries = 34500; // 16^3 * entries * 2048 columns < 3e11 (shared_walk)
 
 // How many rows of a panel (16 rows) share a column, for shared_walk; 0 where
 // the panels cannot run or never pay. A sample of panels tells: share, when

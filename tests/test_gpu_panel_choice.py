@@ -23,10 +23,11 @@ def blocks(m, k, bs, density, first_col=0, seed=1):
                                                  (16, 1 << 17, "spdm_panel_kernel"), (4, 1 << 17, "spdm_group_kernel")])
 def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
     """Blocks as high as a panel take the panels, lower ones do not, wherever
-    in a wide matrix they lie; a rebuild chooses as the first build."""
+    in a wide matrix they lie; a rebuild chooses as the first build. (Asked
+    for either: by themselves so few rows take the row walk.)"""
     import torch
     A = blocks(64, 1 << 18, bs, 0.06, first_col)
-    h = native.GcooHandle(A).build()
+    h = native.GcooHandle(A, fp32_order="groups").build()
     B, C = torch.ones(1 << 18, 1024, device="cuda"), torch.empty(64, 1024, device="cuda")
     s = torch.cuda.Stream()
     for _ in range(2):
@@ -39,7 +40,8 @@ def test_choice_by_the_blocks_height(native, bs, first_col, kernel):
 @pytest.mark.parametrize("rows,holes,n,kernel", [
     (2, 0.0, 1024, "spdm_fp32_kernel"), (2, 0.0, 1001, "spdm_fp32_kernel"), (2, 0.0, 128, "spdm_fp32_kernel"),
     (4, 0.0, 1024, "spdm_group_kernel"), (4, 0.0, 1001, "spdm_fp32_kernel"), (4, 0.0, 512, "spdm_fp32_kernel"),
-    (16, 0.4, 2048, "spdm_panel_kernel"), (16, 0.4, 2001, "spdm_panel_kernel"), (16, 0.4, 1024, "spdm_fp32_kernel")])
+    (16, 0.4, 2048, "spdm_panel_kernel"), (16, 0.4, 2001, "spdm_fp32_kernel"), (16, 0.4, 1024, "spdm_fp32_kernel"),
+    (16, 0.0, 1001, "spdm_panel_kernel")])
 @pytest.mark.parametrize("k", [2048, 2047])
 def test_choice_by_sharing_and_work(native, rows, holes, n, kernel, k):
     """Blocks of several heights at 15 %: the walk by how many rows share a
