@@ -636,7 +636,12 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
         GCOO_CUDA(launch_row_scan_max(h->row_ptr.ptr, h->m, h->p.rows_per_group, h->group_index(), h->nnz_per_group(),
                                       d_total, h->scratch.ptr, h->status.ptr, st));
     }
-    int64_t tot2[3] = {0, 0, 0};
+    // a matrix that needed the sample of its panels last time probably does again
+    const bool sample2 = tiled && h->sampled && dense_share_ok(h->k);
+    if (sample2)
+        GCOO_CUDA(launch_dense_share(h->dA, h->m, h->k, kSampleEntries, h->p.fp32_order == 2, d_total,
+                                     reinterpret_cast<unsigned long long *>(d_total + 6), st));
+    int64_t tot2[kReadbackWords] = {};
     GCOO_CUDA(cudaMemcpyAsync(tot2, d_total, sizeof(tot2), cudaMemcpyDeviceToHost, st));
     GCOO_CUDA(cudaStreamSynchronize(st));
     const int64_t total = tot2[0];
@@ -663,7 +668,7 @@ static gcoo_status build_handle(gcoo_handle *h, cudaStream_t st, NextMultiply *m
                                  cols, h->packed.ptr, st, dense));
     h->nnz = total;
     h->seg_prefix = tiled;
-    return finish_build(h, st);
+    return finish_build(h, st, sample2 ? tot2 + 6 : nullptr);
 }
 
 gcoo_status gcoo_build(gcoo_handle *h, void *stream)

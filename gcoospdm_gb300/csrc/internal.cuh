@@ -276,6 +276,10 @@ bool panel_ok(int64_t n);
 // memory that receives both; *ticket, then, is zeroed by the caller.
 cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k,
                                unsigned long long *out, unsigned int *ticket, int64_t *host, cudaStream_t st);
+// The same from A itself, no host words; see dense_share_kernel.
+bool dense_share_ok(int64_t k);
+cudaError_t launch_dense_share(const float *A, int64_t m, int64_t k, int64_t least, bool any, const int64_t *totals,
+                               unsigned long long *out, cudaStream_t st);
 cudaError_t launch_spdm_fp32_panel(const Entry *packed, const int32_t *row_ptr, const int32_t *pref, int64_t m,
                                    int64_t k, const float *B, int64_t n, float *C, cudaStream_t st);
 // The same walk for the BF16 / FP8-B forms on the FMA engine, from B already

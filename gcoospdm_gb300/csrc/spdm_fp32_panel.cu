@@ -464,7 +464,68 @@ panel_share_kernel(const Entry *__restrict__ packed, const int32_t *__restrict__
     }
 }
 
+// The same sample of A itself (k <= kShareCols), before the entries are placed:
+// a conversion in two passes reads it with its totals, where the sample of the
+// entries needs a wait of its own (builds, us: 2153 x 1929 at 36 % 75 -> 57,
+// 6645 x 4381 227 -> 200, 8192^2 at 40 % 554 -> 522).
+// totals: [0] entries, [2] distinct group columns; with fewer than `least` entries
+// or, unless `any`, too little sharing to consider panels nothing is read. A CTA
+// has 1024 columns of a panel.
+constexpr int kDenseShareThreads = 256, kDenseShareCols = 1024;
+
+__global__ void __launch_bounds__(kDenseShareThreads)
+dense_share_kernel(const float *__restrict__ A, int64_t m, int64_t k, int64_t panels, int64_t least,
+                   bool any, const int64_t *__restrict__ totals, unsigned long long *__restrict__ out)
+{
+    __shared__ int s_sum[2];
+    if (threadIdx.x == 0)
+        s_sum[0] = s_sum[1] = 0;
+    grid_wait_previous();
+    totals = written(totals);
+    const int64_t nnz = totals[0], groups = totals[2];
+    if (nnz < least || (!any && 2 * nnz < 3 * groups))
+        return; // the same for all
+    __syncthreads();
+    const int64_t r0 = (blockIdx.x * panels / gridDim.x) * kPanelRows;
+    const int rows = static_cast<int>(r0 + kPanelRows < m ? kPanelRows : m - r0);
+    int entries = 0, distinct = 0;
+#pragma unroll 1
+    for (int q = 0; q < kDenseShareCols; q += kDenseShareThreads) {
+        const int64_t c = static_cast<int64_t>(blockIdx.y) * kDenseShareCols + q + threadIdx.x;
+        int x = 0;
+#pragma unroll
+        for (int r = 0; r < kPanelRows; ++r)
+            x += c < k && r < rows && A[(r0 + r) * k + c] != 0.0f;
+        entries += x;
+        distinct += x != 0;
+    }
+    entries = __reduce_add_sync(0xffffffffu, entries);
+    distinct = __reduce_add_sync(0xffffffffu, distinct);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_sum[0], entries);
+        atomicAdd(&s_sum[1], distinct);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(out, static_cast<unsigned long long>(s_sum[0]));
+        atomicAdd(out + 1, static_cast<unsigned long long>(s_sum[1]));
+    }
+}
+
 } // namespace
+
+bool dense_share_ok(int64_t k) { return k <= kShareCols; }
+
+cudaError_t launch_dense_share(const float *A, int64_t m, int64_t k, int64_t least, bool any,
+                               const int64_t *totals, unsigned long long *out, cudaStream_t st)
+{
+    const int64_t panels = (m + kPanelRows - 1) / kPanelRows;
+    const dim3 grid(static_cast<unsigned>(panels < kSharePanels ? panels : kSharePanels),
+                    static_cast<unsigned>((k + kDenseShareCols - 1) / kDenseShareCols));
+    count_launches(1);
+    return launch_after(dense_share_kernel, grid, dim3(kDenseShareThreads), 0, st, A, m, k, panels, least, any,
+                        totals, out);
+}
 
 cudaError_t launch_panel_share(const Entry *packed, const int32_t *row_ptr, int64_t m, int64_t k,
                                unsigned long long *out, unsigned int *ticket, int64_t *host, cudaStream_t st)

@@ -78,6 +78,30 @@ def test_choice_by_the_windows(native, m, k, density, n, kernel):
     assert torch.equal(h.spdm(B), A.sum(1, keepdim=True).expand(-1, n))  # whole numbers: exact
 
 
+@pytest.mark.parametrize("bs,kernel", [(16, "spdm_panel_kernel"), (2, "spdm_fp32_kernel")])
+@pytest.mark.parametrize("m,k", [(2048, 2047), (2047, 2050), (4096, 4096)])
+def test_choice_of_dense_rebuilds(native, m, k, bs, kernel):
+    """Matrices so dense that a rebuild reads A twice: the sample of A itself
+    tells what that of the first build's entries told, also when the matrix
+    has turned to other blocks in between."""
+    import torch
+    blk = lambda bs: blocks(2048 if m < 4000 else m, 4096, bs, 0.5)[:m, :k].contiguous()  # noqa: E731
+    A = blk(bs)
+    h = native.GcooHandle(A).build()
+    B, C = torch.ones(k, 256, device="cuda"), torch.empty(m, 256, device="cuda")
+    s = torch.cuda.Stream()
+    for turn in range(3):
+        names = [name for name, _ in captured_kernels(s, lambda: h.spdm(B, C, stream=s))]
+        assert len(names) == 1 and kernel in names[0], (turn, names)
+        torch.cuda.synchronize()
+        assert torch.equal(h.spdm(B), A.sum(1, keepdim=True).expand(-1, 256))  # whole numbers: exact
+        if turn == 0:
+            A.copy_(blk(18 - bs))
+            h.build()
+            A.copy_(blk(bs))
+        h.build()
+
+
 def test_multiply_by_returns_with_the_multiply_under_way(native):
     """A steady loop on a block matrix whose width takes the row walk (here
     milliseconds of it): the call waits for the conversion's totals only."""
