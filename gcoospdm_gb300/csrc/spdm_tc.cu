@@ -1025,8 +1025,12 @@ bool encode_map(CUtensorMap *map, const void *base, cuuint32_t rank, const cuuin
 // the grid within one wave). Shares: equal parts of the products with one
 // accumulator, one per pair, where their estimate is shorter, in MMA times of
 // one tile: a product of a share costs kPairShareRate (its A half feeds one
-// MMA), and the exposed last drain with the fix-up kPairShareCost. Measured,
-// 16 x 16 blocks, whole / shares: 8192^2 at 25 %, n = 128 68 / 50 us, n = 512
+// MMA), the exposed last drain with the fix-up kPairShareCost, and each share
+// that a panel's strip is cut into kPairSharePart (the fix-up adds them one
+// after another: 206 x 4980, n = 192, 312 tiles in one panel 41 / 73). The choice
+// takes 0.6 % longer than the better one over 768 multiplies of 64 x 400 to 10000
+// x 14000 (2.9 % without the parts, up to 1.8 times). Measured, 16 x 16 blocks,
+// whole / shares: 8192^2 at 25 %, n = 128 68 / 50 us, n = 512
 // 72 / 80, n = 1024 94 / 125; 10240 x 8192 at 25 %, n = 1024 (80 units on 76
 // pairs) 172 / 147; 2048 x 8192 at 25 %, n = 256 63 / 35; 1024 x 16384 at 10 %,
 // n = 1024 110 / 61; 4096^2, n = 256 38 / 32; 2048^2, n = 1024 28 / 33;
@@ -1036,7 +1040,7 @@ struct PairCut {
     int nt;
     bool shares;
 };
-constexpr double kPairShareRate = 1.45, kPairShareCost = 150.0;
+constexpr double kPairShareRate = 1.45, kPairShareCost = 80.0, kPairSharePart = 7.0;
 constexpr int64_t kPairShareCols = 128; // column tiles at most: beyond, whole units fill the waves
 
 PairCut pair_cut(int64_t panels, int64_t tiles, int64_t ntn)
@@ -1047,7 +1051,8 @@ PairCut pair_cut(int64_t panels, int64_t tiles, int64_t ntn)
     const int64_t work = tiles * ntn;
     // in tiles of one accumulator
     const double whole = static_cast<double>((units + slots - 1) / slots) * nt_whole * tiles / (panels > 0 ? panels : 1);
-    const double share = kPairShareRate * static_cast<double>(work) / slots + kPairShareCost;
+    const double parts = static_cast<double>(slots) / static_cast<double>(panels * ntn > 0 ? panels * ntn : 1);
+    const double share = kPairShareRate * static_cast<double>(work) / slots + kPairShareCost + kPairSharePart * parts;
     if (share < whole && work >= slots * kPairK && ntn <= kPairShareCols)
         return PairCut{slots, 1, true};
     return PairCut{units, nt_whole, false};

@@ -40,3 +40,19 @@ def test_shares_over_strips_and_panels(native, m, k, n, density, prec):
         assert torch.equal(out[:m], want)
         assert bool((out[m] == 7.0).all())
     assert h.device_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n", [(206, 4980, 192), (112, 2807, 480), (439, 2934, 112)])
+def test_few_panels_of_few_tiles_stay_whole(native, m, k, n):
+    """A share of four tiles each, seventy to be added per panel: not cut."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    A = torch.randint(-3, 4, (m, k), generator=gen, device="cuda").float()
+    B = torch.randint(-3, 4, (k, n), generator=gen, device="cuda").float()
+    h = native.GcooHandle(A, engine="tensor").build()
+    h.prepare(n, "bf16")
+    L = native.lib()
+    before = L.gcoo_kernel_launches()
+    C = h.spdm(B, prec="bf16")
+    assert L.gcoo_kernel_launches() - before == 2  # B's tiles and the multiply
+    assert torch.equal(C, (A.double() @ B.double()).float())
