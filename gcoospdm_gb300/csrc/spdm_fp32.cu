@@ -803,15 +803,17 @@ LaunchShape pick_shape(const gcoo_params &p, int64_t m, int64_t n, int64_t nnz, 
     // spread over the SMs is the time. Not started while the predecessor drains,
     // where they would take whichever slots come free first (1924 x 249, 154
     // entries a row, n = 236: 22.3 us behind another multiply, 18.9 so; shorter
-    // rows gain by it, 6 % on average over 1504 multiplies); and with twelve
-    // 4-warp CTAs per SM where that is one wave and kRowCtas are not (1199 x
-    // 4114, 170 a row, n = 728: 42.5 us with ten, 34.3 with twelve).
+    // rows gain by it, 6 % on average over 1504 multiplies, and so does less than
+    // half a wave, which finds slots whoever drains: 355 x 11466, 122 a row, 16 rows
+    // per group, n = 184 11.0 against 16.6); and with twelve 4-warp CTAs per SM
+    // where that is one wave and kRowCtas are not (1199 x 4114, 170 a row, n = 728:
+    // 42.5 us with ten, 34.3 with twelve).
     if (mean >= 100.0) {
         const int64_t tile = static_cast<int64_t>(s.col_warps) * 32 * s.vec * s.col_iters;
         const int64_t ctas = (m + s.rows - 1) / s.rows * ((n + tile - 1) / tile), sms = device_sms();
         const int64_t twelve = 48 / s.warps < 32 ? 48 / s.warps : 32; // of CTAs that wide as many as 48 warps
         const int64_t per_sm = s.warps <= 4 && 4 * kRowCtas / s.warps < twelve ? 4 * kRowCtas / s.warps : twelve;
-        s.after = 10 * ctas > 13 * per_sm * sms;
+        s.after = 10 * ctas > 13 * per_sm * sms || 10 * ctas < (mean < 500.0 ? 5 : 3) * per_sm * sms;
         s.tight = s.warps <= 4 && ctas > per_sm * sms && ctas <= twelve * sms;
     }
     return s;
